@@ -155,7 +155,9 @@ struct b2r_engine {
   uint64_t bytes_per_slot{0}, bytes{0};
   b2r::dev::state st{};
   cudaStream_t stream{nullptr};
-  cudaGraphExec_t graph{nullptr};
+  cudaGraphExec_t graph[2]{nullptr, nullptr};  // the super-step, without and with journeys rebuilt beside it
+  cudaStream_t stream_recon{nullptr};           // the latter's branch
+  cudaEvent_t ev_fork{nullptr}, ev_join{nullptr};
   cudaStream_t stream2{nullptr};  // exports overlapping the super-steps
   b2r_launch_shape shape{8, 256, 8, 4, 4, 0};  // launch shape of the super-step
   cudaGraphExec_t lb_graph{nullptr};  // 4 x 2 Bellman-Ford iterations
@@ -552,10 +554,14 @@ __global__ void k_set_journeys(dev::state st, uint32_t s, dev::journey_rec const
 b2r_engine::~b2r_engine() {
   for (auto ev : prof_ev) cudaEventDestroy(ev);
   for (auto ev : prof_rc_ev) cudaEventDestroy(ev);
-  if (graph != nullptr) cudaGraphExecDestroy(graph);
+  for (auto* g : graph)
+    if (g != nullptr) cudaGraphExecDestroy(g);
   if (lb_graph != nullptr) cudaGraphExecDestroy(lb_graph);
   if (stream != nullptr) cudaStreamDestroy(stream);
   if (stream2 != nullptr) cudaStreamDestroy(stream2);
+  if (stream_recon != nullptr) cudaStreamDestroy(stream_recon);
+  if (ev_fork != nullptr) cudaEventDestroy(ev_fork);
+  if (ev_join != nullptr) cudaEventDestroy(ev_join);
   if (ev0 != nullptr) cudaEventDestroy(ev0);
   if (ev1 != nullptr) cudaEventDestroy(ev1);
   if (ev_base != nullptr) cudaEventDestroy(ev_base);
@@ -589,23 +595,44 @@ cudaError_t record_in_graph(cudaEvent_t ev, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------- super-step
-void enqueue_superstep(b2r_engine& e, cudaStream_t s) {
+// grid of a kernel whose threads stride over n items, `per` a block
+unsigned blocks_for(uint64_t n, uint64_t per, uint64_t most) {
+  return static_cast<unsigned>(std::min<uint64_t>(most, std::max<uint64_t>(1U, (n + per - 1U) / per)));
+}
+
+// One round of every running slot.  recon: some resident query runs several
+// start-time groups, so journeys are rebuilt between them; that kernel runs
+// on stream2 beside the round's, from the swap of the mark arrays (k_routes)
+// to the end of the step.
+void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
   auto const& st = e.st;
-  auto const slot_blocks = (e.S + 127) / 128;
-  auto const list_blocks = e.sms * 8;
-  dev::k_ctl_begin<<<list_blocks, 256, 0, s>>>(st);
-  // a warp per 32-location chunk of the sweep: one pass over the locations
-  auto const sweep_chunks = (st.tt.n_loc + 31U) / 32U;
-  dev::k_sweep<<<std::min<uint32_t>(e.sms * 16U, std::max<uint32_t>(1U, (sweep_chunks + 7U) / 8U)), 256, 0, s>>>(st);
-  dev::k_ctl_dest<<<slot_blocks, 128, 0, s>>>(st);
-  auto const pair_blocks = e.sms * e.shape.pair_blocks_per_sm;
-  dev::k_mark_routes<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_list_routes<<<e.sms * 8, 256, 0, s>>>(st);
-  if (st.tt.n_rt != 0U) {  // a real-time overlay is bound: its runs are marked too
-    dev::k_mark_rt<<<list_blocks, 256, 0, s>>>(st);
-    dev::k_list_rt<<<e.sms * 8, 256, 0, s>>>(st);
+  auto const words = static_cast<uint64_t>(st.tt.n_loc) * e.G;
+  auto const pair_blocks = static_cast<uint64_t>(e.sms) * e.shape.pair_blocks_per_sm;
+  auto const slot_blocks = static_cast<uint64_t>((e.S + 7U) / 8U);  // a warp per slot
+  auto const list_blocks = static_cast<uint64_t>(e.sms) * 8U;
+  dev::k_mark<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
+  dev::k_routes<<<std::max(blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks),
+                           blocks_for(slot_blocks, 1U, list_blocks)),
+                  256, 0, s>>>(st);
+  cudaEvent_t rc_a = nullptr, rc_b = nullptr;
+  if (recon) {
+    auto* s2 = e.stream_recon;
+    B2R_CUDA(cudaEventRecord(e.ev_fork, s));
+    B2R_CUDA(cudaStreamWaitEvent(s2, e.ev_fork, 0));
+    if (e.cfg.profile == 1U) {
+      while (e.prof_rc_used + 2 > e.prof_rc_ev.size()) {
+        cudaEvent_t x;
+        B2R_CUDA(cudaEventCreate(&x));
+        e.prof_rc_ev.push_back(x);
+      }
+      rc_a = e.prof_rc_ev[e.prof_rc_used++];
+      rc_b = e.prof_rc_ev[e.prof_rc_used++];
+      B2R_CUDA(cudaEventRecord(rc_a, s2));
+    }
+    dev::k_reconstruct<<<blocks_for(e.S, 1U, static_cast<uint64_t>(e.sms) * e.shape.recon_blocks_per_sm), 128, 0, s2>>>(st);
+    if (e.cfg.profile == 1U) B2R_CUDA(cudaEventRecord(rc_b, s2));
+    B2R_CUDA(cudaEventRecord(e.ev_join, s2));
   }
-  dev::k_ctl_marked<<<slot_blocks, 128, 0, s>>>(st);
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   if (e.cfg.profile == 2U) {  // timing build: one event pair, captured in the super-step graph
     B2R_CUDA(record_in_graph(e.ev_scan_a, s));
@@ -640,30 +667,34 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s) {
     if (idx < b2r_engine::kProfRows) k_prof_row<<<1, 1, 0, s>>>(st, e.d_prof_rows, idx);
   }
   if (st.tt.n_rt != 0U) dev::k_rt_scan<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_list_reached<<<e.sms * 8, 256, 0, s>>>(st);
-  dev::k_clear_x<<<list_blocks, 256, 0, s>>>(st);
-  dev::k_transfers_pre<<<slot_blocks, 128, 0, s>>>(st);
-  dev::k_transfers<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_intermodal_fp_pre<<<slot_blocks, 128, 0, s>>>(st);
-  dev::k_footpaths<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_end_collect<<<slot_blocks, 128, 0, s>>>(st);
-  cudaEvent_t rc_a = nullptr, rc_b = nullptr;
-  if (e.cfg.profile == 1U) {
-    while (e.prof_rc_used + 2 > e.prof_rc_ev.size()) {
-      cudaEvent_t x;
-      B2R_CUDA(cudaEventCreate(&x));
-      e.prof_rc_ev.push_back(x);
-    }
-    rc_a = e.prof_rc_ev[e.prof_rc_used++];
-    rc_b = e.prof_rc_ev[e.prof_rc_used++];
-    B2R_CUDA(cudaEventRecord(rc_a, s));
-  }
-  dev::k_reconstruct<<<e.sms * e.shape.recon_blocks_per_sm, 128, 0, s>>>(st);
-  if (e.cfg.profile == 1U) B2R_CUDA(cudaEventRecord(rc_b, s));
-  dev::k_next_summary<<<slot_blocks, 128, 0, s>>>(st);
-  dev::k_list_marked<<<e.sms * 8, 256, 0, s>>>(st);
+  dev::k_reached<<<std::max(blocks_for(words, 1024U, list_blocks), blocks_for(slot_blocks, 1U, list_blocks)), 256, 0,
+                   s>>>(st);
+  dev::k_relax<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
+  if (recon) B2R_CUDA(cudaStreamWaitEvent(s, e.ev_join, 0));
+  dev::k_end<<<e.G, 1024, 0, s>>>(st, false);
 }
-uint64_t launches_per_step(b2r_engine const& e) { return e.st.tt.n_rt != 0U ? 21U : 18U; }
+uint64_t launches_per_step(b2r_engine const& e, bool recon) {
+  return 7U + (recon ? 1U : 0U) + (e.st.tt.n_rt != 0U ? 1U : 0U);
+}
+
+// a super-step as its graph (recon: the one with the reconstruction branch)
+// or as single launches
+void run_superstep(b2r_engine& e, cudaStream_t s, bool graph, bool recon) {
+  if (graph) {
+    B2R_CUDA(cudaGraphLaunch(e.graph[recon ? 1 : 0], s));
+  } else {
+    enqueue_superstep(e, s, recon);
+    B2R_CUDA(cudaGetLastError());
+  }
+}
+
+// admitted slots get their first start labels (and every slot its views) for
+// the next super-step
+void seed(b2r_engine& e, cudaStream_t s) {
+  ++e.aux_launches;
+  dev::k_end<<<e.G, 1024, 0, s>>>(e.st, true);
+  B2R_CUDA(cudaGetLastError());
+}
 
 // --------------------------------------------------------- admission
 size_t admission_bytes(b2r_engine const& e, prepped_query const& p) {
@@ -963,6 +994,7 @@ void admit(b2r_engine& e, std::vector<adm_req> const& adm, cudaStream_t s) {
       e.max_starts, e.max_dest, e.max_off);
   B2R_CUDA(cudaGetLastError());
   if (any_device_lb) solve_lower_bounds(e, s);
+  seed(e, s);
 }
 
 void retire(b2r_engine& e, std::vector<uint32_t> const& slots, cudaStream_t s) {
@@ -1586,6 +1618,10 @@ bool sweeps(prepped_query const& p) { return !p.ontrip && !p.one_to_all; }
 // when it is done (the queries whose reconstruction waits for that)
 bool single_group(prepped_query const& p) { return p.ontrip && !p.one_to_all && p.recon_mode == 0 && !p.pong; }
 
+// whether journeys of the query are rebuilt between its start-time groups
+// (range queries; pong queries, whose phases share the slot)
+bool rebuilds_between_groups(prepped_query const& p) { return !single_group(p) && !p.one_to_all; }
+
 // a new interval-extension phase for the query in slot s (search.h:283-316)
 void rearm(b2r_engine& e, uint32_t s, query_run& q, cudaStream_t st) {
   // new phase: upload the new starts (and journeys kept), keep the rt
@@ -1622,6 +1658,7 @@ void rearm(b2r_engine& e, uint32_t s, query_run& q, cudaStream_t st) {
   ++e.aux_launches;
   k_set_journeys<<<1, 32, 0, st>>>(e.st, s, dj, static_cast<uint32_t>(q.keep.size()));
   B2R_CUDA(cudaMemcpyAsync(e.st.slots + s, &cur, sizeof(slot_t), cudaMemcpyHostToDevice, st));
+  seed(e, st);
   B2R_CUDA(cudaStreamSynchronize(st));
   e.h2d_bytes += starts.size() * sizeof(dev::start_rec) + q.keep.size() * sizeof(dev::journey_rec) +
                  sizeof(slot_t);
@@ -1739,14 +1776,11 @@ struct batch_runner {
     auto const busy = [&]() { return next < runs.size() || running(); };
     auto const launch_chunk = [&](uint32_t n_steps) {
       B2R_CUDA(cudaEventRecord(e.ev0, st));
+      auto recon = false;
+      for (auto const x : slot_q) recon = recon || (x >= 0 && rebuilds_between_groups(runs[static_cast<size_t>(x)].p));
       for (uint32_t c = 0; c != n_steps; ++c) {
-        if (use_graph) {
-          B2R_CUDA(cudaGraphLaunch(e.graph, st));
-        } else {
-          enqueue_superstep(e, st);
-          B2R_CUDA(cudaGetLastError());
-        }
-        launches += launches_per_step(e);
+        run_superstep(e, st, use_graph, recon);
+        launches += launches_per_step(e, recon);
         ++steps;
       }
       B2R_CUDA(cudaEventRecord(e.ev1, st));
@@ -1888,13 +1922,23 @@ struct batch_runner {
   }
 };
 
+void drop_graphs(b2r_engine& e) {
+  for (auto*& g : e.graph) {
+    if (g != nullptr) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 void capture_graph(b2r_engine& e) {
-  cudaGraph_t g = nullptr;
-  B2R_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_superstep(e, e.stream);
-  B2R_CUDA(cudaStreamEndCapture(e.stream, &g));
-  B2R_CUDA(cudaGraphInstantiate(&e.graph, g, 0));
-  cudaGraphDestroy(g);
+  drop_graphs(e);
+  for (auto recon = 0; recon != 2; ++recon) {
+    cudaGraph_t g = nullptr;
+    B2R_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
+    enqueue_superstep(e, e.stream, recon != 0);
+    B2R_CUDA(cudaStreamEndCapture(e.stream, &g));
+    B2R_CUDA(cudaGraphInstantiate(&e.graph[recon], g, 0));
+    cudaGraphDestroy(g);
+  }
 }
 
 // Host preparation on worker threads, in query order, overlapping the
@@ -2101,7 +2145,7 @@ struct serve_state {
   void driver_loop() {
     auto* st = e.stream;
     auto const chunk = e.cfg.steps_per_sync != 0 ? e.cfg.steps_per_sync : std::min(2U, e.shape.steps_per_sync);
-    auto const use_graph = e.cfg.use_graphs != 0 && e.graph != nullptr;
+    auto const use_graph = e.cfg.use_graphs != 0 && e.graph[0] != nullptr;
     try {
       B2R_CUDA(cudaSetDevice(e.tt->device));
       std::vector<uint8_t> retiring(e.S, 0), stale(e.S, 0), waiting(e.S, 0);
@@ -2112,16 +2156,11 @@ struct serve_state {
       // is throughput-bound then)
       auto const launch_chunk = [&]() {
         auto const n_steps = backlog ? std::max(chunk, e.shape.steps_per_sync) : chunk;
+        auto recon = false;
+        for (auto const* x : slot_item) recon = recon || (x != nullptr && rebuilds_between_groups(x->run.p));
         this->n_steps += n_steps;
-        n_launches += n_steps * launches_per_step(e);
-        for (uint32_t c = 0; c != n_steps; ++c) {
-          if (use_graph) {
-            B2R_CUDA(cudaGraphLaunch(e.graph, st));
-          } else {
-            enqueue_superstep(e, st);
-            B2R_CUDA(cudaGetLastError());
-          }
-        }
+        n_launches += n_steps * launches_per_step(e, recon);
+        for (uint32_t c = 0; c != n_steps; ++c) run_superstep(e, st, use_graph, recon);
         B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, e.S * sizeof(b2r_engine::summary_t),
                                  cudaMemcpyDeviceToHost, st));
         in_flight = true;
@@ -2559,7 +2598,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
                               (sizeof(b2r::dev::journey_rec) + b2r::dev::kMaxLegs * sizeof(b2r_leg)) +
                           e->max_starts * sizeof(b2r::dev::start_rec) +
                           e->max_dest * sizeof(b2r::dev::dest_rec) + e->max_off * sizeof(b2r_offset) +
-                          b2r::dev::kMaxTimeline * sizeof(b2r::dev::tl_entry) +
+                          2U * b2r::dev::kMaxTimeline * sizeof(b2r::dev::tl_entry) +
                           (static_cast<uint64_t>(nl) * (4 + b2r::dev::kK) + tt->d.n_routes) / 8 + 256;
       auto by_budget = cfg.hbm_budget / std::max<uint64_t>(1, e->bytes_per_slot);
       auto slots = std::min<uint64_t>(std::max(32U, cfg.max_slots), by_budget);
@@ -2589,11 +2628,11 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.best, static_cast<size_t>(nl) * S);
       al(st.tmp, static_cast<size_t>(nl) * S);
       al(st.lb, static_cast<size_t>(nl) * S);
-      al(st.X, static_cast<size_t>(nl) * G);
+      al(st.X[0], static_cast<size_t>(nl) * G);
+      al(st.X[1], static_cast<size_t>(nl) * G);
       al(st.Y, static_cast<size_t>(nl) * G);
       al(st.R, static_cast<size_t>(tt->d.n_routes) * G);
       al(st.D, static_cast<size_t>(nl) * G);
-      al(st.xlist, static_cast<size_t>(nl) * G);
       al(st.ylist, static_cast<size_t>(nl) * G);
       al(st.rlist, static_cast<size_t>(tt->d.n_routes) * G);
       al(st.counters, 16);
@@ -2607,9 +2646,9 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.legs, S * e->max_j * b2r::dev::kMaxLegs);
       al(st.blocks_used, S * ((e->max_j + 31) / 32));
       al(st.recon_list, S * e->max_j);
-      al(st.timeline, S * b2r::dev::kMaxTimeline);
-      al(st.timeline_n, S);
-      al(st.tad_phase, S);
+      al(st.timeline, 2U * S * b2r::dev::kMaxTimeline);
+      al(st.timeline_n, 2U * S);
+      al(st.tad_phase, 2U * S);
       al(st.status_word, 4);
       al(e->d_summary, S);
       st.summary = e->d_summary;
@@ -2637,7 +2676,12 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       B2R_CUDA(cudaMemset(st.touched, 0, static_cast<size_t>(b2r::dev::kK) * G * nl * 4));
       B2R_CUDA(cudaMemset(st.best, 0xFF, static_cast<size_t>(nl) * S * 4));
       B2R_CUDA(cudaMemset(st.tmp, 0xFF, static_cast<size_t>(nl) * S * 4));
-      B2R_CUDA(cudaMemset(st.X, 0, static_cast<size_t>(nl) * G * 4));
+      B2R_CUDA(cudaMemset(st.X[0], 0, static_cast<size_t>(nl) * G * 4));
+      B2R_CUDA(cudaMemset(st.X[1], 0, static_cast<size_t>(nl) * G * 4));
+      B2R_CUDA(cudaMemset(st.lanes, 0, S * sizeof(b2r::dev::lane_t)));
+      B2R_CUDA(cudaMemset(st.run_mask, 0, G * 4));
+      B2R_CUDA(cudaMemset(st.sweep_mask, 0, G * 4));
+      B2R_CUDA(cudaMemset(st.any_mask, 0, G * 4));
       B2R_CUDA(cudaMemset(st.Y, 0, static_cast<size_t>(nl) * G * 4));
       B2R_CUDA(cudaMemset(st.R, 0, static_cast<size_t>(tt->d.n_routes) * G * 4));
       B2R_CUDA(cudaMemset(st.D, 0, static_cast<size_t>(nl) * G * 4));
@@ -2648,6 +2692,9 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       B2R_CUDA(cudaMallocHost(&e->h_lbcount, sizeof(uint32_t)));
       B2R_CUDA(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
       B2R_CUDA(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
+      B2R_CUDA(cudaStreamCreateWithFlags(&e->stream_recon, cudaStreamNonBlocking));
+      B2R_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
+      B2R_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
       B2R_CUDA(cudaEventCreate(&e->ev0));
       B2R_CUDA(cudaEventCreate(&e->ev1));
       B2R_CUDA(cudaEventCreate(&e->ev_base));
@@ -2706,7 +2753,7 @@ int b2r_search_batch(b2r_engine* e, const b2r_query* qs, uint32_t n, b2r_result*
       e->admit_ms = e->export_ms = e->idle_ms = 0;
       b2r::preparer prep;
       prep.start(*e, qs, n, runs, false);
-      b2r::batch_runner br{*e, runs, e->cfg.use_graphs != 0 && e->graph != nullptr};
+      b2r::batch_runner br{*e, runs, e->cfg.use_graphs != 0 && e->graph[0] != nullptr};
       if (e->cfg.profile) B2R_CUDA(cudaMemsetAsync(e->st.prof, 0, 8 * sizeof(unsigned long long), e->stream));
       e->scan_ms = 0;
       e->scan_launches = 0;
@@ -2827,10 +2874,8 @@ int b2r_engine_set_shape(b2r_engine* e, const b2r_launch_shape* sh) {
     try {
       B2R_CUDA(cudaSetDevice(e->tt->device));
       e->shape = *sh;
-      if (e->graph != nullptr) {  // the graph holds the old launch configuration
+      if (e->graph[0] != nullptr) {  // the graphs hold the old launch configuration
         B2R_CUDA(cudaStreamSynchronize(e->stream));
-        cudaGraphExecDestroy(e->graph);
-        e->graph = nullptr;
         b2r::capture_graph(*e);
       }
       return B2R_OK;
@@ -3128,12 +3173,7 @@ dev::slot_summary run_slot0(b2r_engine& e) {
   auto* st = e.stream;
   for (uint64_t step = 0;; ++step) {
     if (step > 100000) throw std::runtime_error("super-step cap exceeded");
-    if (e.cfg.use_graphs != 0 && e.graph != nullptr) {
-      B2R_CUDA(cudaGraphLaunch(e.graph, st));
-    } else {
-      enqueue_superstep(e, st);
-      B2R_CUDA(cudaGetLastError());
-    }
+    run_superstep(e, st, e.cfg.use_graphs != 0 && e.graph[0] != nullptr, false);
     B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, sizeof(b2r_engine::summary_t), cudaMemcpyDeviceToHost, st));
     B2R_CUDA(cudaStreamSynchronize(st));
     auto const state = e.h_summary[0].state;
@@ -3528,9 +3568,7 @@ int b2r_engine_set_rt(b2r_engine* e, const b2r_rt* rt) {
       e->st.tt = rt != nullptr ? rt->d : e->tt->d;
       e->view = e->tt->view;
       e->view.rt = rt != nullptr ? &rt->host : nullptr;
-      if (e->graph != nullptr) {  // the graph holds the old image and kernels
-        cudaGraphExecDestroy(e->graph);
-        e->graph = nullptr;
+      if (e->graph[0] != nullptr) {  // the graphs hold the old image and kernels
         b2r::capture_graph(*e);
       }
       return B2R_OK;

@@ -33,7 +33,8 @@ enum : uint8_t {
   S_RUN = 2,       // running rounds
   S_COLLECT = 3,   // rounds of the current group finished
   S_DONE = 4,      // phase finished, host reads results
-  S_ERROR = 5
+  S_ERROR = 5,
+  S_RECON = 6      // journeys of the finished group being rebuilt, next group follows
 };
 
 // ------------------------------------------------------- timetable image
@@ -234,16 +235,15 @@ struct state {
   uint32_t* best;   // [n_loc][S]
   uint32_t* tmp;    // [n_loc][S]
   uint16_t* lb;     // [n_loc][S]
-  uint32_t* X;      // station marks  [n_loc][G]
+  uint32_t* X[2];   // station marks  [n_loc][G]: the round's and the next round's (C_PAR)
   uint32_t* Y;      // route-reached marks [n_loc][G]
   uint32_t* R;      // route marks [n_routes][G]
   uint32_t* RT_R;   // rt transport marks [n_rt][G] (an overlay is bound)
   uint32_t* rtlist; // frontier list of (rt transport * G + g)
   uint32_t* D;      // is-destination bits [n_loc][G]
-  uint32_t* xlist;  // frontier lists of (loc * G + g)
-  uint32_t* ylist;
+  uint32_t* ylist;  // frontier lists of (loc * G + g)
   uint32_t* rlist;
-  uint32_t* counters;  // [0] xlist, [1] ylist, [2] rlist, [3] recon count, [4] x2 ...
+  uint32_t* counters;  // C_*: list lengths, mark parity, error bits
   uint32_t* run_mask;  // [G]
   uint32_t* sweep_mask;  // [G]
   uint32_t* any_mask;  // [G]
@@ -254,9 +254,9 @@ struct state {
   b2r_leg* legs;          // [S][max_j][kMaxLegs]
   uint32_t* blocks_used;  // [S][max_j / 32]
   uint32_t* recon_list;   // (slot << 16 | journey index)
-  tl_entry* timeline;     // [S][kMaxTimeline]
-  uint32_t* timeline_n;   // [S]
-  int16_t* tad_phase;     // [S] tad[k] at the start of the phase
+  tl_entry* timeline;     // [2][S][kMaxTimeline]: transfers, footpaths
+  uint32_t* timeline_n;   // [2][S]
+  int16_t* tad_phase;     // [2][S] tad[k] at the start of the phase
   uint32_t* status_word;  // [0] device error flags
   unsigned long long* prof;  // route-scan work counters (profiling engines)
   uint32_t profile;

@@ -11,7 +11,13 @@
 
 namespace b2r::dev {
 
-enum : uint32_t { C_X = 0, C_Y = 1, C_R = 2, C_RECON = 3, C_ERR = 4, C_F0 = 5, C_F1 = 6, C_RT = 7 };
+// C_PAR: which of the two station-mark arrays the next marks go to (k_routes
+// flips it between a step's reads and its writes); C_RECON0 + parity: the
+// journeys listed for reconstruction
+enum : uint32_t {
+  C_PAR = 0, C_Y = 1, C_R = 2, C_RECON0 = 3, C_ERR = 4, C_F0 = 5, C_F1 = 6, C_RT = 7, C_RECON1 = 8
+};
+constexpr uint32_t recon_counter(uint32_t par) { return par == 0u ? C_RECON0 : C_RECON1; }
 
 __device__ __forceinline__ size_t li(state const& st, uint32_t l, uint32_t s) {
   return static_cast<size_t>(l) * st.S + s;
@@ -103,51 +109,25 @@ __device__ __forceinline__ void update_tad(slot_t& sl, uint32_t k, int key) {  /
   }
 }
 
-// ----------------------------------------------------------- control
-// Start of a super-step: the route-reached marks of the last one cleared
-// (all threads), and per slot (threads < S, a warp per slot group) the lane
-// view and the group's run / sweep masks, written whole from ballots.  The
-// reached-list counter is reset by k_ctl_dest, after every thread here has
-// read it.
-__global__ void k_ctl_begin(state st) {
-  auto const tid = blockIdx.x * blockDim.x + threadIdx.x;
-  auto const ny = st.counters[C_Y];
-  for (auto i = tid; i < ny; i += gridDim.x * blockDim.x) st.Y[st.ylist[i]] = 0u;
-  if (tid == 0) {
-    st.counters[C_R] = 0u;
-    st.counters[C_RECON] = 0u;
-    st.counters[C_RT] = 0u;
-  }
-  if ((tid & ~31u) >= st.S) return;  // whole warps: S is a multiple of 32
-  auto const s = tid;
-  auto& sl = st.slots[s];
+// The compact view of a slot that every lane of the round kernels reads.
+__device__ __forceinline__ lane_t lane_of(slot_t const& sl) {
   lane_t ln{};
-  auto const run = sl.state == S_RUN;
-  auto const run_bits = __ballot_sync(kFull, run);
-  auto const sweep_bits = __ballot_sync(kFull, run && sl.need_sweep);
-  if ((s & 31u) == 0u) {
-    st.run_mask[s >> 5] = run_bits;
-    st.sweep_mask[s >> 5] = sweep_bits;
-    st.any_mask[s >> 5] = 0u;
-  }
-  if (run) {
-    ln.run = 1;
-    ln.fwd = sl.fwd;
-    ln.k = sl.k;
-    ln.base = sl.base;
-    ln.gtag = tagcode(sl.gen_group);
-    ln.qtag = tagcode(sl.gen_query);
-    ln.mode = (sl.intermodal_dest ? 1u : 0u) |
-              ((!sl.intermodal_dest && !sl.one_to_all && sl.n_dest != 0) ? 2u : 0u) |
-              (sl.tts.is_default ? 4u : 0u) | (sl.no_lb ? 8u : 0u) | (static_cast<uint32_t>(sl.prf) << 4) |
-              (keeps_round_times(sl) ? 128u : 0u);
-    ln.tad_k = sl.tad[sl.k];
-    ln.claszes = sl.allowed_claszes;
-    ln.req = sl.req_flags;
-    ln.blast = sl.blast;
-    ++sl.n_rounds;
-  }
-  st.lanes[s] = ln;
+  if (sl.state != S_RUN) return ln;
+  ln.run = 1;
+  ln.fwd = sl.fwd;
+  ln.k = sl.k;
+  ln.base = sl.base;
+  ln.gtag = tagcode(sl.gen_group);
+  ln.qtag = tagcode(sl.gen_query);
+  ln.mode = (sl.intermodal_dest ? 1u : 0u) |
+            ((!sl.intermodal_dest && !sl.one_to_all && sl.n_dest != 0) ? 2u : 0u) |
+            (sl.tts.is_default ? 4u : 0u) | (sl.no_lb ? 8u : 0u) | (static_cast<uint32_t>(sl.prf) << 4) |
+            (keeps_round_times(sl) ? 128u : 0u);
+  ln.tad_k = sl.tad[sl.k];
+  ln.claszes = sl.allowed_claszes;
+  ln.req = sl.req_flags;
+  ln.blast = sl.blast;
+  return ln;
 }
 
 // best <- min(best, round_times[k]) over all locations (raptor.h:219-223)
@@ -160,10 +140,7 @@ __global__ void k_ctl_begin(state st) {
 // to an earlier query of the slot (its tag no longer matches) are cleared
 // here; any later write sets them again.  Slots of one group at different
 // rounds are taken one round at a time.
-__global__ void k_sweep(state st) {
-  auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void sweep(state const& st, uint32_t lane, uint32_t warp, uint32_t n_warps) {
   auto const n_loc = st.tt.n_loc;
   auto const n_chunks = (n_loc + 31u) / 32u;
   for (auto g = 0u; g != st.G; ++g) {
@@ -221,48 +198,56 @@ __global__ void k_sweep(state st) {
   }
 }
 
-// destination times into time_at_dest (raptor.h:224-226)
-__global__ void k_ctl_dest(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) st.counters[C_Y] = 0u;  // k_ctl_begin has cleared the listed words
-  if (s >= st.S) return;
-  auto& sl = st.slots[s];
-  if (sl.state != S_RUN || sl.one_to_all) return;
-  auto const gtag = tagcode(sl.gen_group);
-  if (sl.intermodal_dest) {
-    update_tad(sl, sl.k, dec(st.best[li(st, B2R_SPECIAL_END, s)], gtag));
-  } else {
-    for (auto i = 0u; i != sl.n_dest; ++i) {
-      update_tad(sl, sl.k, dec(st.best[li(st, st.dest_pool[sl.dest_off + i].loc, s)], gtag));
-    }
-  }
-  st.lanes[s].tad_k = sl.tad[sl.k];
-}
-
-// station marks -> route marks (raptor.h:228-241)
-// A warp takes 32 marked (location, group) words and spreads their
-// (word, route) pairs over its lanes, so that hub stations with many routes
-// do not hold one lane.  The per-group "any route marked" word is read
-// before its atomicOr: it only gains bits during the kernel, so a read that
-// shows the bits set makes the atomic redundant, and same-address atomics
-// would queue in L2.
-__global__ void k_mark_routes(state st) {
-  auto const nx = st.counters[C_X];
+// station marks -> route marks (raptor.h:228-241), then the sweep.
+//
+// A warp takes 32 words of the station marks ((location, group) pairs; most
+// are zero, and 32 zero words cost one load and one ballot), and spreads the
+// (word, route) pairs of the marked ones over its lanes, so that hub
+// stations with many routes do not hold one lane.  Reading the marks where
+// they lie saves a frontier list and its launch: the words of a step are
+// read in full once here and once where they are cleared (k_reached).
+// The per-group "any route marked" word is read before its atomicOr: it only
+// gains bits during the kernel, so a read that shows the bits set makes the
+// atomic redundant, and same-address atomics would queue in L2.  A marked
+// real-time run (n_rt != 0) also keeps its queries in the round.
+__global__ void k_mark(state st) {
   auto const lane = threadIdx.x & 31u;
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
-  for (auto w0 = warp * 32u; w0 < nx; w0 += n_warps * 32u) {
-    auto const i = w0 + lane;
-    uint32_t g = 0, w = 0, rb = 0, cnt = 0;
-    if (i < nx) {
-      auto const e = st.xlist[i];
+  auto const par = st.counters[C_PAR];
+  auto const* X = st.X[par];
+  auto const& T = st.tt;
+  if (blockIdx.x == 0u && threadIdx.x == 0u) {  // this step's lists
+    st.counters[C_Y] = 0u;
+    st.counters[C_R] = 0u;
+    st.counters[C_RT] = 0u;
+    st.counters[recon_counter(par ^ 1u)] = 0u;
+  }
+  auto const n = T.n_loc * st.G;
+  auto const step = n_warps * 32u;
+  auto i = warp * 32u + lane;
+  auto x = i < n ? X[i] : 0u;
+  for (auto w0 = warp * 32u; w0 < n; w0 += step) {
+    auto const e = i;
+    auto w = x;
+    i += step;
+    x = i < n ? X[i] : 0u;  // the next pass's word, in flight during this one
+    if (__ballot_sync(kFull, w != 0u) == 0u) continue;
+    uint32_t g = 0, rb = 0, cnt = 0;
+    if (w != 0u) {
       g = e % st.G;
       auto const l = e / st.G;
-      w = st.X[e] & st.run_mask[g];
+      w &= st.run_mask[g];
       if (w != 0u) {
-        rb = __ldg(st.tt.loc_routes_idx + l);
-        cnt = __ldg(st.tt.loc_routes_idx + l + 1) - rb;
-        if (cnt != 0u && (st.any_mask[g] & w) != w) atomicOr(&st.any_mask[g], w);
+        rb = __ldg(T.loc_routes_idx + l);
+        cnt = __ldg(T.loc_routes_idx + l + 1) - rb;
+        auto any = cnt;
+        if (T.n_rt != 0u) {
+          auto const b = T.loc_rt_idx[l], m = T.loc_rt_idx[l + 1] - b;
+          any += m;
+          for (auto j = 0u; j != m; ++j) atomicOr(&st.RT_R[T.loc_rt[b + j] * st.G + g], w);
+        }
+        if (any != 0u && (st.any_mask[g] & w) != w) atomicOr(&st.any_mask[g], w);
       }
     }
     auto end = cnt;  // inclusive prefix sum of the route counts
@@ -283,11 +268,12 @@ __global__ void k_mark_routes(state st) {
       auto const o_g = __shfl_sync(kFull, g, static_cast<int>(owner));
       auto const o_w = __shfl_sync(kFull, w, static_cast<int>(owner));
       if (p < total) {
-        auto const r = __ldg(st.tt.loc_routes + o_rb + (p - o_first));
-        atomicOr(&st.R[r * st.G + o_g], o_w);  // listed by k_list_routes
+        auto const r = __ldg(T.loc_routes + o_rb + (p - o_first));
+        atomicOr(&st.R[r * st.G + o_g], o_w);  // listed by k_routes
       }
     }
   }
+  sweep(st, lane, warp, n_warps);
 }
 
 // The indices of the non-zero words of W[0, n) appended to `list` (in no
@@ -340,40 +326,48 @@ __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W,
   }
 }
 
-// marked (route, group) entries of this round
-__global__ void k_list_routes(state st) { list_nonzero(st, st.R, st.tt.n_routes * st.G, st.rlist, C_R); }
-
-// ------------------------------------------------ real-time transports
-// station marks -> rt transport marks (raptor.h:234-240), a thread per
-// marked (location, group) word; a marked rt transport also keeps its
-// queries in the round (any_marked)
-__global__ void k_mark_rt(state st) {
-  auto const nx = st.counters[C_X];
-  auto const& T = st.tt;
-  for (auto i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
-    auto const e = st.xlist[i];
-    auto const g = e % st.G, l = e / st.G;
-    auto const w = st.X[e] & st.run_mask[g];
-    if (w == 0u) continue;
-    auto const b = T.loc_rt_idx[l], n = T.loc_rt_idx[l + 1] - b;
-    if (n == 0u) continue;
-    if ((st.any_mask[g] & w) != w) atomicOr(&st.any_mask[g], w);
-    for (auto j = 0u; j != n; ++j) atomicOr(&st.RT_R[T.loc_rt[b + j] * st.G + g], w);  // listed by k_list_rt
+// Per slot, a warp: destination times into time_at_dest (raptor.h:224-226;
+// a minimum, so the lanes take the destinations in any order), and a slot
+// with no marked route leaves the round loop (raptor.h:243-246).
+__device__ __forceinline__ void dest_slot(state const& st, uint32_t s, uint32_t lane) {
+  auto& sl = st.slots[s];
+  if (sl.state != S_RUN) return;
+  auto const k = static_cast<uint32_t>(sl.k);
+  if (!sl.one_to_all) {
+    auto const gtag = tagcode(sl.gen_group);
+    int key = kKeyInv;
+    if (sl.intermodal_dest) {
+      key = dec(st.best[li(st, B2R_SPECIAL_END, s)], gtag);
+    } else {
+      for (auto i = lane; i < sl.n_dest; i += 32u) {
+        key = min(key, dec(st.best[li(st, st.dest_pool[sl.dest_off + i].loc, s)], gtag));
+      }
+    }
+    key = __reduce_min_sync(kFull, key);
+    if (lane >= k && lane < kK && key < sl.tad[lane]) sl.tad[lane] = static_cast<int16_t>(key);
+    if (lane == 0u && key < st.lanes[s].tad_k) st.lanes[s].tad_k = static_cast<int16_t>(key);
+  }
+  if (lane == 0u) {
+    ++sl.n_rounds;
+    if (!((st.any_mask[s >> 5] >> (s & 31u)) & 1u)) {
+      sl.state = S_COLLECT;
+      st.lanes[s].run = 0;
+    }
   }
 }
 
-// marked (rt transport, group) entries of this round
-__global__ void k_list_rt(state st) { list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, st.rtlist, C_RT); }
-
-__global__ void k_ctl_marked(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= st.S) return;
-  auto& sl = st.slots[s];
-  if (sl.state != S_RUN) return;
-  if (!((st.any_mask[s >> 5] >> (s & 31)) & 1u)) {  // raptor.h:243-246
-    sl.state = S_COLLECT;
-    st.lanes[s].run = 0;
-  }
+// The round's marked (route, group) and (real-time run, group) entries
+// listed, the slots' destination times, and the station-mark arrays swapped:
+// from here to the end of the step X[C_PAR ^ 1] holds the marks the round
+// reads and X[C_PAR] takes the marks it makes.
+__global__ void k_routes(state st) {
+  auto const lane = threadIdx.x & 31u;
+  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+  if (blockIdx.x == 0u && threadIdx.x == 0u) st.counters[C_PAR] ^= 1u;
+  for (auto s = warp; s < st.S; s += n_warps) dest_slot(st, s, lane);
+  list_nonzero(st, st.R, st.tt.n_routes * st.G, st.rlist, C_R);
+  if (st.tt.n_rt != 0u) list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, st.rtlist, C_RT);
 }
 
 // ------------------------------------------------------------ route scan
@@ -429,13 +423,13 @@ __device__ __forceinline__ void scan_arrive(state const& st, lane_t const& ln, u
     } else {
       atomicMin(tp, word);  // result unused: no round trip
     }
-    atomicOr(&st.Y[l * st.G + g], bit);  // listed by k_list_reached
+    atomicOr(&st.Y[l * st.G + g], bit);  // listed by k_reached
   }
 }
 
 // The reference's sequential walk of one (route, query) pair.
-__device__ __forceinline__ void scan_walk_seq(state const& st, lane_t const& ln, uint32_t r, uint32_t g,
-                                              uint32_t b, uint32_t sec, scan_ctr& pc) {
+__device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X, lane_t const& ln, uint32_t r,
+                                              uint32_t g, uint32_t b, uint32_t sec, scan_ctr& pc) {
   auto const& T = st.tt;
   auto const s = g * 32u + b;
   auto const bit = 1u << b;
@@ -467,7 +461,7 @@ __device__ __forceinline__ void scan_walk_seq(state const& st, lane_t const& ln,
       auto const ev = colbase[n_t * (si * 2u - (fwd ? 1u : 0u)) + et_off];
       scan_arrive<true>(st, ln, s, g, bit, l, lbv, to_delta_key(fwd, et_day, ln.base, delta_count(ev)), pc);
     }
-    if (i + 1u == n || !can_start || !(st.X[l * st.G + g] & bit)) continue;
+    if (i + 1u == n || !can_start || !(X[l * st.G + g] & bit)) continue;
     if (lbv == 0xFFFFu) break;  // raptor.h:1309-1311: no later stop of this query
     auto const board_col = n_t * (si * 2u - (fwd ? 0u : 1u));
     auto const et_time =
@@ -510,6 +504,7 @@ __device__ __forceinline__ bool scan_filters(dtt const& T, lane_t const& ln, uin
 __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ state st) {
   auto const& T = st.tt;
   auto const nr = st.counters[C_R];
+  auto const* X = st.X[st.counters[C_PAR] ^ 1u];
   scan_ctr pc{0u, 0u, 0u, 0u, 0u};
   for (auto w = blockIdx.x * blockDim.x + threadIdx.x; w < nr; w += gridDim.x * blockDim.x) {
     auto const e = st.rlist[w];
@@ -521,7 +516,7 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
       uint32_t sec = 0u;
       if (!ln.run || !scan_filters(T, ln, r, sec)) continue;
       if ((sec & 15u) == 0u && fifo) continue;  // k_route_scan's
-      scan_walk_seq(st, ln, r, g, b, sec, pc);
+      scan_walk_seq(st, X, ln, r, g, b, sec, pc);
     }
   }
   if (st.profile && (pc.stops | pc.ev | pc.days | pc.writes) != 0u) {
@@ -536,8 +531,8 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
 // One (route, query) pair, the warp's lanes over its stops.  Prof: count
 // the work for the roofline (profiling engines only).
 template <bool Prof>
-__device__ __forceinline__ void scan_pair(state const& st, lane_t const& ln, uint32_t r, uint32_t g, uint32_t b,
-                                          uint32_t lane, scan_ctr& pc) {
+__device__ __forceinline__ void scan_pair(state const& st, uint32_t const* X, lane_t const& ln, uint32_t r, uint32_t g,
+                                          uint32_t b, uint32_t lane, scan_ctr& pc) {
   auto const& T = st.tt;
   auto const s = g * 32u + b;
   uint32_t sec = 0u;
@@ -572,7 +567,7 @@ __device__ __forceinline__ void scan_pair(state const& st, lane_t const& ln, uin
     if (act) {
       stp = scan_stop_word(T, sb, n, fwd, i, sec);
       l = B2R_STOP_LOC(stp);
-      marked = (st.X[l * st.G + g] & bit) != 0u;
+      marked = (X[l * st.G + g] & bit) != 0u;
       if (!lb_off) lbv = st.lb[li(st, l, s)];
     }
     auto const can_finish = act && (fwd ? B2R_STOP_OUT(stp) : B2R_STOP_IN(stp)) != 0u;
@@ -668,6 +663,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
   auto const nr = st.counters[C_R];
+  auto const* X = st.X[st.counters[C_PAR] ^ 1u];
   scan_ctr pc{0u, 0u, 0u, 0u, 0u};
   for (auto w = warp; w < nr; w += n_warps) {
     auto const e = st.rlist[w];
@@ -680,7 +676,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       mask &= mask - 1u;
       auto const ln = st.lanes[g * 32u + b];
       if (!ln.run) continue;
-      scan_pair<Prof>(st, ln, r, g, b, lane, pc);
+      scan_pair<Prof>(st, X, ln, r, g, b, lane, pc);
       __syncwarp();
     }
   }
@@ -709,6 +705,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
 // the route flags, section by section where set on some sections only.
 __global__ void k_rt_scan(state st) {
   auto const& T = st.tt;
+  auto const* X = st.X[st.counters[C_PAR] ^ 1u];
   for_each_pair(
       st.rtlist, st.counters[C_RT],
       [&](uint32_t e) {
@@ -751,251 +748,242 @@ __global__ void k_rt_scan(state st) {
             scan_arrive<false>(st, ln, s, g, bit, l, lbv, by, pc);
           }
           if (lbv == 0xFFFFu) break;  // raptor.h:1156-1158: before the boarding test
-          if (i + 1u == n || !(fwd ? B2R_STOP_IN(w) : B2R_STOP_OUT(w)) || !(st.X[l * st.G + g] & bit)) continue;
+          if (i + 1u == n || !(fwd ? B2R_STOP_IN(w) : B2R_STOP_OUT(w)) || !(X[l * st.G + g] & bit)) continue;
           auto const by = to_key(fwd, clamp16(tm[2u * si - (fwd ? 0u : 1u)] - base_min));
           if (dec(st.rt[rti(st, k - 1u, l, s)], ln.qtag) <= by) et = true;
         }
       });
 }
 
-// frontier list of the stations marked this round (transfers, footpaths,
-// start labels): every nonzero station-mark word (location, group)
-__global__ void k_list_marked(state st) { list_nonzero(st, st.X, st.tt.n_loc * st.G, st.xlist, C_X); }
-
-// frontier list of the stations reached by the route scan: every nonzero
-// route-reached word (location, group)
-__global__ void k_list_reached(state st) { list_nonzero(st, st.Y, st.tt.n_loc * st.G, st.ylist, C_Y); }
-
-__global__ void k_clear_x(state st) {
-  auto const tid = blockIdx.x * blockDim.x + threadIdx.x;
-  auto const nx = st.counters[C_X];
-  for (auto i = tid; i < nx; i += gridDim.x * blockDim.x) st.X[st.xlist[i]] = 0u;
-}
-
-
-// ---------------------------------------------------- transfer phase
-// Destination stations of station-to-station queries first, in location
-// order, so that the time_at_dest updates they make (raptor.h:737-739) are
-// seen by later stations exactly as in the sequential loop; the timeline of
-// those updates is kept per query.
-__global__ void k_transfers_pre(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) st.counters[C_X] = 0u;  // k_clear_x has cleared the listed marks
-  if (s >= st.S) return;
-  auto& sl = st.slots[s];
-  auto const ln = st.lanes[s];
-  st.timeline_n[s] = 0u;
-  if (!ln.run) return;
-  st.tad_phase[s] = sl.tad[ln.k];
-  if (!(ln.mode & 2u)) return;
-  auto const k = ln.k;
-  auto const g = s >> 5;
-  auto const bit = 1u << (s & 31);
-  uint32_t tl_n = 0;
-  for (auto i = 0u; i != sl.n_dest; ++i) {
-    auto const d = st.dest_pool[sl.dest_off + i].loc;
-    if (!(st.Y[d * st.G + g] & bit)) continue;
-    auto const tk = dec(st.tmp[li(st, d, s)], ln.gtag);
-    if (tk == kKeyInv) continue;
-    auto const fp = key_add(tk, 0);
-    auto const bk = dec(st.best[li(st, d, s)], ln.gtag);
-    auto& rtw = st.rt[rti(st, k, d, s)];
-    if (ln.blast == 0u && fp < bk && fp < dec(rtw, ln.qtag)) {
-      rtw = enc(ln.qtag, fp);
-      touch(st, ln, k, d, s);
-    }
-    auto const tad = static_cast<int>(sl.tad[k]);
-    if (fp < bk && fp <= tad) {
-      auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, d, s)];
-      if (lbv == 0xFFFFu || fp + static_cast<int>(lbv) > tad) continue;
-      if (!within_bounds(st, s, ln.blast, k, d, fp)) continue;
-      rtw = enc(ln.qtag, fp);
-      touch(st, ln, k, d, s);
-      st.best[li(st, d, s)] = enc(ln.gtag, fp);
-      atomicOr(&st.X[d * st.G + g], bit);  // listed by k_list_marked
-      if (fp < tad && tl_n < kMaxTimeline) {
-        st.timeline[s * kMaxTimeline + tl_n++] = {d, 0u, fp};
-      } else if (fp < tad) {
-        atomicOr(&st.counters[C_ERR], 1u);
-      }
-      update_tad(sl, k, fp);
-    }
-  }
-  st.timeline_n[s] = tl_n;
-}
-
-// tad in effect at position (hi, lo) of the phase's processing order
-__device__ __forceinline__ int tad_at(state const& st, uint32_t s, uint32_t hi, uint32_t lo) {
-  auto const n = st.timeline_n[s];
-  int tad = st.tad_phase[s];
+// ------------------------------------- stations reached, destination passes
+// tad in effect at position (hi, lo) of phase `ph`'s processing order (0:
+// transfers, 1: footpaths)
+__device__ __forceinline__ int tad_at(state const& st, uint32_t ph, uint32_t s, uint32_t hi, uint32_t lo) {
+  auto const n = st.timeline_n[ph * st.S + s];
+  int tad = st.tad_phase[ph * st.S + s];
+  auto const* tl = st.timeline + (static_cast<size_t>(ph) * st.S + s) * kMaxTimeline;
   for (auto i = 0u; i != n; ++i) {
-    auto const& e = st.timeline[s * kMaxTimeline + i];
-    if (e.pos_hi < hi || (e.pos_hi == hi && e.pos_lo < lo)) tad = e.tad;
+    if (tl[i].pos_hi < hi || (tl[i].pos_hi == hi && tl[i].pos_lo < lo)) tad = tl[i].tad;
     else break;
   }
   return tad;
 }
 
-// update_transfers, raptor.h:680-743: lane per reached (station, query)
-__global__ void k_transfers(state st) {
-  for_each_pair(
-      st.ylist, st.counters[C_Y], [&](uint32_t e) { return st.Y[e]; },
-      [&](uint32_t e, uint32_t b) {
-        auto const g = e % st.G, l = e / st.G;
-        auto const s = g * 32u + b;
-        auto const ln = st.lanes[s];
-        if (!ln.run || ((ln.mode & 2u) && ((st.D[e] >> b) & 1u))) return;
-        auto const tk = dec(st.tmp[li(st, l, s)], ln.gtag);
-        if (tk == kKeyInv) return;
-        auto const slp = &st.slots[s];
-        auto const tt = static_cast<int>(adjusted<int>(slp->tts, static_cast<int>(st.tt.transfer_time[l])));
-        auto const fp = key_add(tk, tt);
-        auto const bk = dec(st.best[li(st, l, s)], ln.gtag);
-        auto& rtw = st.rt[rti(st, ln.k, l, s)];
-        if (ln.blast == 0u && fp < bk && fp < dec(rtw, ln.qtag)) {
-          rtw = enc(ln.qtag, fp);
-          touch(st, ln, ln.k, l, s);
-        }
-        auto const tad = (ln.mode & 2u) ? tad_at(st, s, l, 0u) : static_cast<int>(st.tad_phase[s]);
-        if (fp < bk && fp <= tad) {
-          auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, l, s)];
-          if (lbv != 0xFFFFu && fp + static_cast<int>(lbv) <= tad &&
-              within_bounds(st, s, ln.blast, ln.k, l, fp)) {
-            rtw = enc(ln.qtag, fp);
-            touch(st, ln, ln.k, l, s);
-            st.best[li(st, l, s)] = enc(ln.gtag, fp);
-            atomicOr(&st.X[e], 1u << b);  // listed by k_list_marked
-          }
-        }
-      });
+// one label of a destination station (key at d), in the phase's order:
+// round times, best label, mark, time_at_dest and the phase's timeline
+// (raptor.h:690-740, 790-840).  One lane.
+__device__ __forceinline__ void dest_label(state const& st, uint32_t* X, slot_t& sl, lane_t const& ln, uint32_t s,
+                                           uint32_t d, int key, uint32_t ph, uint32_t pos_hi, uint32_t pos_lo,
+                                           uint32_t& tl_n) {
+  auto const k = static_cast<uint32_t>(ln.k);
+  auto const bk = dec(st.best[li(st, d, s)], ln.gtag);
+  auto& rtw = st.rt[rti(st, k, d, s)];
+  if (ln.blast == 0u && key < bk && key < dec(rtw, ln.qtag)) {
+    rtw = enc(ln.qtag, key);
+    touch(st, ln, k, d, s);
+  }
+  auto const tad = static_cast<int>(sl.tad[k]);
+  if (key >= bk || key > tad) return;
+  auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, d, s)];
+  if (lbv == 0xFFFFu || key + static_cast<int>(lbv) > tad) return;
+  if (!within_bounds(st, s, ln.blast, k, d, key)) return;
+  rtw = enc(ln.qtag, key);
+  touch(st, ln, k, d, s);
+  st.best[li(st, d, s)] = enc(ln.gtag, key);
+  atomicOr(&X[d * st.G + (s >> 5)], 1u << (s & 31u));
+  if (key < tad) {
+    if (tl_n < kMaxTimeline) {
+      st.timeline[(static_cast<size_t>(ph) * st.S + s) * kMaxTimeline + tl_n++] = {pos_hi, pos_lo, key};
+    } else {
+      atomicOr(&st.counters[C_ERR], 1u);
+    }
+  }
+  update_tad(sl, k, key);
 }
 
-// update_intermodal_footpaths, raptor.h:954-1026: per query, its egress
-// stations in location order
-__device__ void intermodal_slot(state const& st, uint32_t s) {
-  auto const ln = st.lanes[s];
-  if (!ln.run || !(ln.mode & 1u)) return;
-  auto& sl = st.slots[s];
+// update_intermodal_footpaths, raptor.h:954-1026: the best of the egress
+// stations' END labels (every label at or below time_at_dest replaces it,
+// so the last one kept is their minimum).  A warp.
+__device__ __forceinline__ void intermodal_slot(state const& st, slot_t& sl, lane_t const& ln, uint32_t s,
+                                                uint32_t lane, int tad0) {
   auto const g = s >> 5;
-  auto const bit = 1u << (s & 31);
-  for (auto i = 0u; i != sl.n_dest; ++i) {
+  auto const bit = 1u << (s & 31u);
+  int key = kKeyInv + 1;
+  for (auto i = lane; i < sl.n_dest; i += 32u) {
     auto const dr = st.dest_pool[sl.dest_off + i];
     if (!(st.Y[dr.loc * st.G + g] & bit)) continue;
     auto const tk = dec(st.tmp[li(st, dr.loc, s)], ln.gtag);
-    if (tk == kKeyInv) continue;
-    auto const end_time = key_add(tk, static_cast<int>(dr.dist));
-    if (end_time <= sl.tad[ln.k]) {
-      st.rt[rti(st, ln.k, B2R_SPECIAL_END, s)] = enc(ln.qtag, end_time);
-      touch(st, ln, ln.k, B2R_SPECIAL_END, s);
-      st.best[li(st, B2R_SPECIAL_END, s)] = enc(ln.gtag, end_time);
-      update_tad(sl, ln.k, end_time);
-    }
+    if (tk != kKeyInv) key = min(key, key_add(tk, static_cast<int>(dr.dist)));
   }
+  key = __reduce_min_sync(kFull, key);
+  if (key > tad0) return;  // tad0 <= kKeyInv: nothing reached
+  if (lane == 0u) {
+    st.rt[rti(st, ln.k, B2R_SPECIAL_END, s)] = enc(ln.qtag, key);
+    touch(st, ln, ln.k, B2R_SPECIAL_END, s);
+    st.best[li(st, B2R_SPECIAL_END, s)] = enc(ln.gtag, key);
+    st.tad_phase[st.S + s] = static_cast<int16_t>(key);
+  }
+  if (lane >= ln.k && lane < kK && key < sl.tad[lane]) sl.tad[lane] = static_cast<int16_t>(key);
 }
 
-// ---------------------------------------------------- footpath phase
 struct fp_cand {
   uint32_t src, pos, dest;
   int key;
 };
+constexpr uint32_t kMaxFpCand = 64;
 
-// footpaths into destination stations, in the reference's processing order
-// (source location, then position in the source's footpath list)
-__device__ void footpaths_pre_slot(state const& st, uint32_t s) {
-  auto& sl = st.slots[s];
-  auto const ln = st.lanes[s];
-  st.timeline_n[s] = 0u;
-  if (!ln.run) return;
-  st.tad_phase[s] = sl.tad[ln.k];
-  if (!(ln.mode & 2u)) return;
-  auto const fwd = ln.fwd != 0;
-  auto const k = ln.k;
-  auto const g = s >> 5;
-  auto const bit = 1u << (s & 31);
+// The destination stations of a station-to-station query ahead of all other
+// stations: their transfers in location order, then the footpaths into them
+// in the reference's order (source location, position in the source's
+// list), so that the time_at_dest updates they make (raptor.h:737-739) are
+// seen by the other stations exactly as in the sequential loops; each
+// phase's timeline of those updates is kept per query.  The lanes look for
+// the labels, lane 0 takes them in order.
+__device__ __forceinline__ void station_dests_slot(state const& st, uint32_t* X, slot_t& sl, lane_t const& ln,
+                                                   uint32_t s, uint32_t lane, fp_cand* c) {
   auto const& T = st.tt;
-  constexpr int kMaxC = 64;
-  fp_cand c[kMaxC];
-  int nc = 0;
+  auto const g = s >> 5;
+  auto const bit = 1u << (s & 31u);
+  uint32_t tl_n = 0;
+  for (auto i0 = 0u; i0 < sl.n_dest; i0 += 32u) {
+    auto const i = i0 + lane;
+    uint32_t d = 0;
+    int tk = kKeyInv;
+    if (i < sl.n_dest) {
+      d = st.dest_pool[sl.dest_off + i].loc;
+      if (st.Y[d * st.G + g] & bit) tk = dec(st.tmp[li(st, d, s)], ln.gtag);
+    }
+    for (auto m = __ballot_sync(kFull, tk != kKeyInv); m != 0u; m &= m - 1u) {
+      auto const src = __ffs(m) - 1;
+      auto const xd = __shfl_sync(kFull, d, src);
+      auto const xk = __shfl_sync(kFull, tk, src);
+      if (lane == 0u) dest_label(st, X, sl, ln, s, xd, key_add(xk, 0), 0u, xd, 0u, tl_n);
+    }
+  }
+  if (lane == 0u) {
+    st.timeline_n[s] = tl_n;
+    st.tad_phase[st.S + s] = sl.tad[ln.k];
+  }
+  __syncwarp();
+  auto const fwd = ln.fwd != 0;
+  auto const prf = (static_cast<uint32_t>(ln.mode) >> 4) & 7u;
+  auto const* iidx = fp_index(T, prf, !fwd);
+  auto const* idat = fp_words(T, prf, !fwd);
+  auto const* oidx = fp_index(T, prf, fwd);
+  auto const* odat = fp_words(T, prf, fwd);
+  uint32_t nc = 0;
   for (auto i = 0u; i != sl.n_dest; ++i) {
     auto const d = st.dest_pool[sl.dest_off + i].loc;
-    auto const prf = (static_cast<uint32_t>(ln.mode) >> 4) & 7u;
-    auto const* iidx = fp_index(T, prf, !fwd);
-    auto const* idat = fp_words(T, prf, !fwd);
-    for (auto x = iidx[d]; x != iidx[d + 1]; ++x) {
-      auto const src = B2R_FP_TARGET(idat[x]);
-      if (!(st.Y[src * st.G + g] & bit)) continue;
-      auto const tk = dec(st.tmp[li(st, src, s)], ln.gtag);
-      if (tk == kKeyInv) continue;
-      auto const* oidx = fp_index(T, prf, fwd);
-      auto const* odat = fp_words(T, prf, fwd);
-      for (auto y = oidx[src]; y != oidx[src + 1]; ++y) {
-        if (B2R_FP_TARGET(odat[y]) != d) continue;
-        if (nc == kMaxC) {
-          atomicOr(&st.counters[C_ERR], 2u);
-          break;
+    auto const xe = iidx[d + 1];
+    for (auto x0 = iidx[d]; x0 < xe; x0 += 32u) {
+      auto const x = x0 + lane;
+      bool has = false;
+      fp_cand cd{};
+      if (x < xe) {
+        auto const src = B2R_FP_TARGET(idat[x]);
+        if (st.Y[src * st.G + g] & bit) {
+          auto const tk = dec(st.tmp[li(st, src, s)], ln.gtag);
+          if (tk != kKeyInv) {
+            auto const o0 = oidx[src], o1 = oidx[src + 1];
+            for (auto y = o0; y != o1; ++y) {
+              if (B2R_FP_TARGET(odat[y]) != d) continue;
+              auto const dur = adjusted<int>(sl.tts, static_cast<int>(B2R_FP_DURATION(odat[y])));
+              cd = {src, y - o0, d, key_add(tk, dur)};
+              has = true;
+              break;
+            }
+          }
         }
-        auto const dur = adjusted<int>(sl.tts, static_cast<int>(B2R_FP_DURATION(odat[y])));
-        c[nc++] = {src, y - oidx[src], d, key_add(tk, dur)};
-        break;
       }
+      auto const m = __ballot_sync(kFull, has);
+      auto const at = nc + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
+      if (has && at < kMaxFpCand) c[at] = cd;
+      if (has && at >= kMaxFpCand) atomicOr(&st.counters[C_ERR], 2u);
+      nc = min(nc + static_cast<uint32_t>(__popc(m)), kMaxFpCand);
     }
   }
-  for (int a = 1; a < nc; ++a) {  // insertion sort by (src, pos)
-    auto const x = c[a];
-    int b = a - 1;
-    while (b >= 0 && (c[b].src > x.src || (c[b].src == x.src && c[b].pos > x.pos))) {
-      c[b + 1] = c[b];
-      --b;
-    }
-    c[b + 1] = x;
-  }
-  uint32_t tl_n = 0;
-  for (int a = 0; a < nc; ++a) {
-    auto const d = c[a].dest;
-    auto const fp = c[a].key;
-    auto const bk = dec(st.best[li(st, d, s)], ln.gtag);
-    auto& rtw = st.rt[rti(st, k, d, s)];
-    if (ln.blast == 0u && fp < bk && fp < dec(rtw, ln.qtag)) {
-      rtw = enc(ln.qtag, fp);
-      touch(st, ln, k, d, s);
-    }
-    auto const tad = static_cast<int>(sl.tad[k]);
-    if (fp < bk && fp <= tad) {
-      auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, d, s)];
-      if (lbv == 0xFFFFu || fp + static_cast<int>(lbv) > tad) continue;
-      if (!within_bounds(st, s, ln.blast, k, d, fp)) continue;
-      rtw = enc(ln.qtag, fp);
-      touch(st, ln, k, d, s);
-      st.best[li(st, d, s)] = enc(ln.gtag, fp);
-      atomicOr(&st.X[d * st.G + g], bit);  // listed by k_list_marked
-      if (fp < tad && tl_n < kMaxTimeline) {
-        st.timeline[s * kMaxTimeline + tl_n++] = {c[a].src, c[a].pos, fp};
-      } else if (fp < tad) {
-        atomicOr(&st.counters[C_ERR], 1u);
+  __syncwarp();
+  if (lane == 0u) {
+    for (auto a = 1u; a < nc; ++a) {  // insertion sort by (src, pos)
+      auto const x = c[a];
+      auto b = a;
+      while (b > 0u && (c[b - 1u].src > x.src || (c[b - 1u].src == x.src && c[b - 1u].pos > x.pos))) {
+        c[b] = c[b - 1u];
+        --b;
       }
-      update_tad(sl, k, fp);
+      c[b] = x;
     }
+    tl_n = 0;
+    for (auto a = 0u; a != nc; ++a) {
+      dest_label(st, X, sl, ln, s, c[a].dest, c[a].key, 1u, c[a].src, c[a].pos, tl_n);
+    }
+    st.timeline_n[st.S + s] = tl_n;
   }
-  st.timeline_n[s] = tl_n;
 }
 
-// update_intermodal_footpaths, then the footpaths into destination
-// stations, per slot (the order of raptor.h:376-378)
-__global__ void k_intermodal_fp_pre(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= st.S) return;
-  intermodal_slot(st, s);
-  footpaths_pre_slot(st, s);
+// After the scan: the stations it reached listed (every nonzero word of Y),
+// the station marks the round read cleared, and per slot (a warp each) what
+// the round does at the query's destinations before all other stations.
+// The destination passes of both phases can run ahead of the other
+// stations' transfers because they alone write the destinations' labels:
+// k_relax leaves out transfers at, and footpaths into, destinations.
+__global__ void __launch_bounds__(256) k_reached(state st) {
+  __shared__ fp_cand cand[8][kMaxFpCand];
+  auto const lane = threadIdx.x & 31u;
+  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+  auto const par = st.counters[C_PAR];
+  for (auto s = warp; s < st.S; s += n_warps) {
+    auto const ln = st.lanes[s];
+    if (!ln.run) continue;
+    auto& sl = st.slots[s];
+    auto const tad0 = static_cast<int>(sl.tad[ln.k]);
+    if (lane < 2u) {
+      st.timeline_n[lane * st.S + s] = 0u;
+      st.tad_phase[lane * st.S + s] = static_cast<int16_t>(tad0);
+    }
+    __syncwarp();
+    if (ln.mode & 1u) intermodal_slot(st, sl, ln, s, lane, tad0);
+    else if (ln.mode & 2u) station_dests_slot(st, st.X[par], sl, ln, s, lane, cand[threadIdx.x >> 5]);
+    __syncwarp();
+  }
+  auto const n = st.tt.n_loc * st.G;
+  auto* X = st.X[par ^ 1u];
+  for (auto i = (blockIdx.x * blockDim.x + threadIdx.x) * 4u; i < n; i += gridDim.x * blockDim.x * 4u) {
+    if (i + 3u < n) {
+      auto* p = reinterpret_cast<uint4*>(X + i);
+      auto const v = *p;
+      if ((v.x | v.y | v.z | v.w) != 0u) *p = uint4{0u, 0u, 0u, 0u};
+    } else {
+      for (auto j = i; j < n; ++j) X[j] = 0u;
+    }
+  }
+  list_nonzero(st, st.Y, n, st.ylist, C_Y);
 }
 
-// update_footpaths, raptor.h:745-845: lane per reached (station, query),
-// walking the station's footpaths; labels of footpath targets are combined
-// with atomicMin (the phase's final labels and marks do not depend on the
-// processing order).
-__global__ void k_footpaths(state st) {
+// ------------------------------------------------ transfers and footpaths
+// update_transfers (raptor.h:680-743) and update_footpaths (raptor.h:745-
+// 845): a lane per reached (station, query) pair takes the station's
+// transfer, then walks its footpaths.  The pair's word of reached marks is
+// cleared as it is read.
+//
+// The reference runs all transfers before all footpaths.  Taken together
+// they give the same labels: both only lower round_times[k] and best, to
+// the minimum of the candidates that beat best at the start of the round
+// and pass the pruning, and a candidate that meets a label already lowered
+// by another one of the round is above a value that is written anyway.  The
+// pruning bounds differ between the phases, and each keeps its own
+// (tad_phase, timelines; k_reached).
+__global__ void k_relax(state st) {
   auto const& T = st.tt;
+  auto* X = st.X[st.counters[C_PAR]];
   for_each_pair(
-      st.ylist, st.counters[C_Y], [&](uint32_t e) { return st.Y[e]; },
+      st.ylist, st.counters[C_Y],
+      [&](uint32_t e) {
+        auto const m = st.Y[e];
+        st.Y[e] = 0u;
+        return m;
+      },
       [&](uint32_t e, uint32_t b) {
         auto const g = e % st.G, src = e / st.G;
         auto const s = g * 32u + b;
@@ -1003,27 +991,51 @@ __global__ void k_footpaths(state st) {
         if (!ln.run) return;
         auto const tk = dec(st.tmp[li(st, src, s)], ln.gtag);
         if (tk == kKeyInv) return;
+        auto const stations = (ln.mode & 2u) != 0u;
+        auto const& tts = st.slots[s].tts;
+        if (!stations || !((st.D[e] >> b) & 1u)) {
+          auto const tt = static_cast<int>(T.transfer_time[src]);
+          auto const fp = key_add(tk, (ln.mode & 4u) ? tt : static_cast<int>(adjusted<int>(tts, tt)));
+          if (fp < dec(st.best[li(st, src, s)], ln.gtag)) {
+            auto* rtw = &st.rt[rti(st, ln.k, src, s)];
+            // the reference writes round_times ahead of its pruning only
+            // when unbounded (raptor.h:710-714, 790-794)
+            if (ln.blast == 0u) {
+              atomicMin(rtw, enc(ln.qtag, fp));
+              touch(st, ln, ln.k, src, s);
+            }
+            auto const tad = stations ? tad_at(st, 0u, s, src, 0u) : static_cast<int>(st.tad_phase[s]);
+            auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, src, s)];
+            if (fp <= tad && lbv != 0xFFFFu && fp + static_cast<int>(lbv) <= tad &&
+                within_bounds(st, s, ln.blast, ln.k, src, fp)) {
+              if (ln.blast != 0u) {
+                atomicMin(rtw, enc(ln.qtag, fp));
+                touch(st, ln, ln.k, src, s);
+              }
+              atomicMin(&st.best[li(st, src, s)], enc(ln.gtag, fp));
+              atomicOr(&X[e], 1u << b);
+            }
+          }
+        }
         auto const fwd = ln.fwd != 0;
         auto const prf = (static_cast<uint32_t>(ln.mode) >> 4) & 7u;
         auto const* idx = fp_index(T, prf, fwd);
         auto const* dat = fp_words(T, prf, fwd);
         auto const fb = idx[src], n = idx[src + 1] - fb;
-        slot_t const* slp = &st.slots[s];
-        auto const tad_flat = (ln.mode & 2u) ? 0 : static_cast<int>(slp->tad[ln.k]);
+        auto const tad_flat = static_cast<int>(st.tad_phase[st.S + s]);
         for (auto j = 0u; j != n; ++j) {
           auto const fp = dat[fb + j];
           auto const tgt = B2R_FP_TARGET(fp);
-          if ((ln.mode & 2u) && ((st.D[tgt * st.G + g] >> b) & 1u)) continue;
-          auto const key = key_add(tk, adjusted<int>(slp->tts, static_cast<int>(B2R_FP_DURATION(fp))));
+          if (stations && ((st.D[tgt * st.G + g] >> b) & 1u)) continue;
+          auto const dur = static_cast<int>(B2R_FP_DURATION(fp));
+          auto const key = key_add(tk, (ln.mode & 4u) ? dur : adjusted<int>(tts, dur));
           auto const bk = dec(st.best[li(st, tgt, s)], ln.gtag);
           if (key >= bk) continue;
-          // the reference writes round_times ahead of its pruning only when
-          // unbounded (raptor.h:790-794)
           if (ln.blast == 0u) {
             atomicMin(&st.rt[rti(st, ln.k, tgt, s)], enc(ln.qtag, key));
             touch(st, ln, ln.k, tgt, s);
           }
-          auto const tad = (ln.mode & 2u) ? tad_at(st, s, src, j) : tad_flat;
+          auto const tad = stations ? tad_at(st, 1u, s, src, j) : tad_flat;
           if (key > tad) continue;
           auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, tgt, s)];
           if (lbv != 0xFFFFu && key + static_cast<int>(lbv) <= tad) {
@@ -1033,20 +1045,13 @@ __global__ void k_footpaths(state st) {
               touch(st, ln, ln.k, tgt, s);
             }
             atomicMin(&st.best[li(st, tgt, s)], enc(ln.gtag, key));
-            atomicOr(&st.X[tgt * st.G + g], 1u << b);  // listed by k_list_marked
+            atomicOr(&X[tgt * st.G + g], 1u << b);
           }
         }
       });
 }
 
 // ------------------------------------------------- round end / results
-__device__ void ctl_end_slot(state const& st, uint32_t s) {
-  auto& sl = st.slots[s];
-  if (sl.state != S_RUN) return;
-  sl.k = static_cast<uint8_t>(sl.k + 1);
-  if (sl.k >= sl.end_k) sl.state = S_COLLECT;
-}
-
 __host__ __device__ inline bool dominates(journey_rec const& a, journey_rec const& b) {  // journey.h:84-92
   if (a.start_time <= a.dest_time) {
     return a.transfers <= b.transfers && a.start_time >= b.start_time && a.dest_time <= b.dest_time;
@@ -1074,24 +1079,44 @@ __device__ void free_block(state const& st, uint32_t s, uint16_t blk) {
   st.blocks_used[s * words + blk / 32u] &= ~(1u << (blk % 32u));
 }
 
-// pareto_set::add, pareto_set.h:21-37
-__device__ bool pareto_add(state const& st, uint32_t s, slot_t& sl, journey_rec el) {
+// pareto_set::add, pareto_set.h:21-37, by a warp: the lanes compare the
+// journeys 32 at a time.  A journey that dominates `el` leaves the set as it
+// is (then none in the set is dominated by `el`, or the set would not be
+// Pareto); the journeys `el` dominates go, the others keep their order.
+__device__ bool pareto_add(state const& st, uint32_t s, uint32_t& n, journey_rec el, uint32_t lane) {
   auto* els = st.journeys + static_cast<size_t>(s) * st.max_j;
-  uint32_t n_removed = 0;
-  for (auto i = 0u; i < sl.n_journeys; ++i) {
-    if (dominates(els[i], el)) return true;
-    if (dominates(el, els[i])) {
-      free_block(st, s, els[i].block);
-      ++n_removed;
-      continue;
-    }
-    els[i - n_removed] = els[i];
+  for (auto i0 = 0u; i0 < n; i0 += 32u) {
+    auto const i = i0 + lane;
+    if (__any_sync(kFull, i < n && dominates(els[i], el))) return true;
   }
-  sl.n_journeys -= n_removed;
-  auto const blk = alloc_block(st, s);
-  if (blk < 0 || sl.n_journeys >= st.max_j) return false;
+  auto kept = 0u;
+  for (auto i0 = 0u; i0 < n; i0 += 32u) {
+    auto const i = i0 + lane;
+    journey_rec x{};
+    bool keep = false, drop = false;
+    if (i < n) {
+      x = els[i];
+      drop = dominates(el, x);
+      keep = !drop;
+    }
+    auto const km = __ballot_sync(kFull, keep);
+    for (auto dm = __ballot_sync(kFull, drop); dm != 0u; dm &= dm - 1u) {
+      if (static_cast<int>(lane) == __ffs(dm) - 1) free_block(st, s, x.block);
+      __syncwarp();
+    }
+    if (keep) els[kept + static_cast<uint32_t>(__popc(km & ((1u << lane) - 1u)))] = x;
+    kept += static_cast<uint32_t>(__popc(km));
+    __syncwarp();
+  }
+  n = kept;
+  auto blk = -1;
+  if (lane == 0u) blk = alloc_block(st, s);
+  blk = __shfl_sync(kFull, blk, 0);
+  if (blk < 0 || n >= st.max_j) return false;
   el.block = static_cast<uint16_t>(blk);
-  els[sl.n_journeys++] = el;
+  if (lane == 0u) els[n] = el;
+  ++n;
+  __syncwarp();
   return true;
 }
 
@@ -1106,44 +1131,54 @@ __device__ __forceinline__ bool recon_wanted(slot_t const& sl, journey_rec const
                               : false;
 }
 
-// result collection (raptor.h:393-413) and the reconstruction worklist
-// (search.h:457-475)
-__device__ void collect_slot(state const& st, uint32_t s) {
-  auto& sl = st.slots[s];
-  if (sl.state != S_COLLECT || sl.one_to_all) return;
+// result collection (raptor.h:393-413): the round times of the destinations
+// in the reference's order (destination, then round), the lanes loading 32
+// of them at once, into the slot's Pareto set.  A warp; false: out of
+// journey capacity.
+__device__ bool collect_slot(state const& st, slot_t& sl, uint32_t s, uint32_t lane) {
   auto const qtag = tagcode(sl.gen_query);
   auto const fwd = sl.fwd != 0;
-  auto const n_d = sl.intermodal_dest ? 1u : sl.n_dest;
-  for (auto i = 0u; i != n_d; ++i) {
-    auto const d = sl.intermodal_dest ? B2R_SPECIAL_END : st.dest_pool[sl.dest_off + i].loc;
-    for (auto k = 1u; k < sl.end_k; ++k) {
-      auto const key = dec(st.rt[rti(st, k, d, s)], qtag);
-      if (key == kKeyInv) continue;
+  auto const n_k = static_cast<uint32_t>(sl.end_k) - 1u;
+  auto const total = (sl.intermodal_dest ? 1u : sl.n_dest) * n_k;
+  auto n = sl.n_journeys;
+  __syncwarp();
+  bool ok = true;
+  for (auto p0 = 0u; ok && p0 < total; p0 += 32u) {
+    auto const p = p0 + lane;
+    int key = kKeyInv;
+    uint32_t d = 0, k = 0;
+    if (p < total) {
+      k = 1u + p % n_k;
+      d = sl.intermodal_dest ? B2R_SPECIAL_END : st.dest_pool[sl.dest_off + p / n_k].loc;
+      key = dec(st.rt[rti(st, k, d, s)], qtag);
+    }
+    for (auto m = __ballot_sync(kFull, key != kKeyInv); ok && m != 0u; m &= m - 1u) {
+      auto const src = __ffs(m) - 1;
       journey_rec j{};
       j.start_time = sl.cur_start_time;
-      j.dest_time = sl.base_days * 1440 + from_key(fwd, key);
-      j.dest = d;
-      j.transfers = static_cast<uint8_t>(k - 1);
-      if (!pareto_add(st, s, sl, j)) {
-        sl.error = B2R_ERR_CAPACITY;
-        sl.state = S_ERROR;
-        return;
-      }
+      j.dest_time = sl.base_days * 1440 + from_key(fwd, __shfl_sync(kFull, key, src));
+      j.dest = __shfl_sync(kFull, d, src);
+      j.transfers = static_cast<uint8_t>(__shfl_sync(kFull, k, src) - 1u);
+      ok = pareto_add(st, s, n, j, lane);
     }
   }
-  if (sl.recon_defer) return;  // rebuilt when the slot is done (k_reconstruct_done)
-  auto* els = st.journeys + static_cast<size_t>(s) * st.max_j;
-  for (auto i = 0u; i != sl.n_journeys; ++i) {
-    if (recon_wanted(sl, els[i])) st.recon_list[atomicAdd(&st.counters[C_RECON], 1u)] = (s << 16) | i;
-  }
+  if (lane == 0u) sl.n_journeys = n;
+  __syncwarp();
+  return ok;
 }
 
-// end of the round, then result collection when the group's rounds are done
-__global__ void k_end_collect(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= st.S) return;
-  ctl_end_slot(st, s);
-  collect_slot(st, s);
+// the reconstruction worklist (search.h:457-475): whether any journey of the
+// slot is to be rebuilt before its next start-time group
+__device__ bool list_recon(state const& st, slot_t const& sl, uint32_t s, uint32_t lane, uint32_t par) {
+  auto const* els = st.journeys + static_cast<size_t>(s) * st.max_j;
+  auto any = false;
+  for (auto i0 = 0u; i0 < sl.n_journeys; i0 += 32u) {
+    auto const i = i0 + lane;
+    auto const want = i < sl.n_journeys && recon_wanted(sl, els[i]);
+    if (want) st.recon_list[atomicAdd(&st.counters[recon_counter(par)], 1u)] = (s << 16) | i;
+    any = __any_sync(kFull, want) || any;
+  }
+  return any;
 }
 
 // One journey (slot s, index ji) rebuilt by the calling warp.
@@ -1185,13 +1220,15 @@ __device__ __forceinline__ void reconstruct_one(state const& st, uint32_t s, uin
   }
 }
 
-// the journeys collected in this super-step (queries with several
-// start-time groups: their next group changes the round times)
+// The journeys listed at the end of the last super-step (queries with
+// several start-time groups: their next group changes the round times).
+// Their slots wait (S_RECON) while the round kernels of the other slots run
+// beside this one; the step's k_end joins both and sends them on.
 __global__ void k_reconstruct(state st) {
   auto const lane = threadIdx.x & 31u;
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
-  auto const n = st.counters[C_RECON];
+  auto const n = st.counters[recon_counter(st.counters[C_PAR] ^ 1u)];
   for (auto i = warp; i < n; i += n_warps) {
     auto const e = st.recon_list[i];
     reconstruct_one(st, e >> 16, e & 0xFFFFu, lane);
@@ -1224,74 +1261,147 @@ __global__ void k_reconstruct_done(state st, uint32_t const* list, uint32_t n) {
 
 // early termination (search.h:477-492) and seeding of the next start-time
 // group: next_start_time + add_start (raptor.h:179-203) + the
-// time_at_dest bound of execute (raptor.h:211-214)
-__device__ void next_slot(state const& st, uint32_t s) {
-  auto& sl = st.slots[s];
-  if (sl.state != S_COLLECT && sl.state != S_START) return;
+// time_at_dest bound of execute (raptor.h:211-214).  A warp; labels are
+// combined with atomicMin (an older generation's word has a larger tag), so
+// the lanes take the group's starts in any order.
+__device__ void next_slot(state const& st, uint32_t* X, slot_t& sl, uint32_t s, uint32_t lane, bool collected) {
   auto const fwd = sl.fwd != 0;
-  if (sl.state == S_COLLECT && sl.min_connection_count > 0 && !sl.one_to_all) {
+  auto early = sl.early_term != 0;
+  if (collected && sl.min_connection_count > 0 && !sl.one_to_all) {
     uint32_t n_in = 0;
-    auto* els = st.journeys + static_cast<size_t>(s) * st.max_j;
-    for (auto i = 0u; i != sl.n_journeys; ++i) {
+    auto const* els = st.journeys + static_cast<size_t>(s) * st.max_j;
+    for (auto i = lane; i < sl.n_journeys; i += 32u) {
       n_in += sl.ontrip ? 1u : ((sl.iv_from <= els[i].start_time && els[i].start_time < sl.iv_to) ? 1u : 0u);
     }
+    n_in = __reduce_add_sync(kFull, n_in);
     if (n_in >= sl.min_connection_count &&
         ((fwd && sl.extend_earlier && !sl.extend_later) || (!fwd && !sl.extend_earlier && sl.extend_later))) {
-      sl.early_term = 1;
-      if (fwd) sl.iv_from = sl.cur_start_time;
-      else sl.iv_to = sl.cur_start_time + 1;
+      early = true;
+      if (lane == 0u) {
+        sl.early_term = 1;
+        if (fwd) sl.iv_from = sl.cur_start_time;
+        else sl.iv_to = sl.cur_start_time + 1;
+      }
     }
   }
-  if (sl.state == S_COLLECT) sl.need_sweep = 1;
+  if (lane == 0u && collected) sl.need_sweep = 1;
   auto const* starts = st.start_pool + sl.starts_off;
-  if (sl.early_term || sl.next_start >= sl.n_starts) {
-    sl.state = S_DONE;
+  auto const n_starts = sl.n_starts;
+  auto const g0 = sl.next_start;
+  if (early || g0 >= n_starts) {
+    __syncwarp();
+    if (lane == 0u) sl.state = S_DONE;
     return;
   }
   // next start-time group
-  auto const g0 = sl.next_start;
   auto const tas = starts[g0].time_at_start;
-  auto g1 = g0 + 1;
-  while (g1 < sl.n_starts && starts[g1].time_at_start == tas) ++g1;
-  if (sl.gen_group >= 0xFFFEu) {  // tag space exhausted: clear this slot's labels
-    for (auto l = 0u; l != st.tt.n_loc; ++l) {
+  auto gen = sl.gen_group;
+  __syncwarp();
+  if (gen >= 0xFFFEu) {  // tag space exhausted: clear this slot's labels
+    for (auto l = lane; l < st.tt.n_loc; l += 32u) {
       st.best[li(st, l, s)] = 0xFFFFFFFFu;
       st.tmp[li(st, l, s)] = 0xFFFFFFFFu;
     }
-    sl.gen_group = 0;
+    gen = 0;
+    __syncwarp();
   }
-  ++sl.gen_group;
-  auto const gtag = tagcode(sl.gen_group), qtag = tagcode(sl.gen_query);
+  ++gen;
+  auto const gtag = tagcode(gen), qtag = tagcode(sl.gen_query);
   auto const g = s >> 5;
-  auto const bit = 1u << (s & 31);
-  for (auto i = g0; i != g1; ++i) {
-    auto const l = starts[i].stop;
-    auto const key = to_key(fwd, clamp16(starts[i].time_at_stop - sl.base_days * 1440));
-    auto& bw = st.best[li(st, l, s)];
-    if (key < dec(bw, gtag)) bw = enc(gtag, key);
-    auto& rw = st.rt[rti(st, 0, l, s)];
-    if (key < dec(rw, qtag)) rw = enc(qtag, key);
-    atomicOr(&st.X[l * st.G + g], bit);  // listed by k_list_marked
+  auto const bit = 1u << (s & 31u);
+  auto g1 = g0;
+  while (g1 < n_starts) {
+    auto const i = g1 + lane;
+    auto const in = i < n_starts && starts[i].time_at_start == tas;
+    auto const out = __ballot_sync(kFull, !in);
+    auto const len = out == 0u ? 32u : static_cast<uint32_t>(__ffs(out) - 1);
+    if (lane < len) {
+      auto const l = starts[i].stop;
+      auto const key = to_key(fwd, clamp16(starts[i].time_at_stop - sl.base_days * 1440));
+      if (key != kKeyInv) {
+        atomicMin(&st.best[li(st, l, s)], enc(gtag, key));
+        atomicMin(&st.rt[rti(st, 0, l, s)], enc(qtag, key));
+      }
+      atomicOr(&X[l * st.G + g], bit);
+    }
+    g1 += len;
+    if (len != 32u) break;
   }
   auto const worst = tas + (fwd ? static_cast<int>(sl.span) : -static_cast<int>(sl.span));
   auto const d_worst = to_key(fwd, clamp16(worst - sl.base_days * 1440));
-  for (auto i = 0; i != kK; ++i) {
-    if (d_worst < sl.tad[i]) sl.tad[i] = static_cast<int16_t>(d_worst);
+  if (lane < kK && d_worst < sl.tad[lane]) sl.tad[lane] = static_cast<int16_t>(d_worst);
+  __syncwarp();
+  if (lane == 0u) {
+    sl.gen_group = gen;
+    sl.cur_start_time = tas;
+    sl.next_start = g1;
+    sl.k = 1;
+    sl.state = S_RUN;
+    ++sl.n_groups_run;
   }
-  sl.cur_start_time = tas;
-  sl.next_start = g1;
-  sl.k = 1;
-  sl.state = S_RUN;
-  ++sl.n_groups_run;
 }
 
-// the next start-time group, then the slot's state for the host
-__global__ void k_next_summary(state st) {
-  auto const s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= st.S) return;
-  next_slot(st, s);
-  auto const& sl = st.slots[s];
-  st.summary[s] = {sl.state, {0, 0, 0}, sl.n_journeys};
+// The end of a super-step, a warp per slot and a block per group of 32
+// slots: the round's end (raptor.h:217), collection when the group's rounds
+// are over, the journeys to rebuild listed (the slot then waits one step in
+// S_RECON), the next start-time group seeded, and the slot's views for the
+// next step (lane record, the group's run and sweep masks) and for the host
+// (summary).  seed_only: admitted slots are seeded and the views renewed,
+// nothing else (after an admission, so that a query's first super-step is
+// its first round).
+// A thread per slot walked destinations x rounds and the journey list one
+// dependent load at a time.
+__global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
+  __shared__ uint32_t run_bits, sweep_bits;
+  auto const lane = threadIdx.x & 31u;
+  auto const g = blockIdx.x;
+  auto const s = g * 32u + (threadIdx.x >> 5);
+  if (threadIdx.x == 0u) run_bits = sweep_bits = 0u;
+  __syncthreads();
+  auto const par = st.counters[C_PAR];
+  auto& sl = st.slots[s];
+  auto state = sl.state;
+  __syncwarp();
+  if (seed_only) {
+    if (state == S_START) next_slot(st, st.X[par], sl, s, lane, false);
+  } else {
+    if (state == S_RUN) {
+      auto const k = static_cast<uint8_t>(sl.k + 1u);
+      __syncwarp();
+      if (lane == 0u) sl.k = k;
+      if (k >= sl.end_k) state = S_COLLECT;
+    }
+    if (state == S_COLLECT) {
+      if (!sl.one_to_all && !collect_slot(st, sl, s, lane)) {
+        state = S_ERROR;
+        if (lane == 0u) sl.error = B2R_ERR_CAPACITY;
+      } else if (!sl.one_to_all && !sl.recon_defer && list_recon(st, sl, s, lane, par)) {
+        state = S_RECON;  // else rebuilt when the slot is done (k_reconstruct_done), or nothing to rebuild
+      } else {
+        next_slot(st, st.X[par], sl, s, lane, true);
+      }
+      if ((state == S_ERROR || state == S_RECON) && lane == 0u) sl.state = state;
+    } else if (state == S_RECON) {
+      next_slot(st, st.X[par], sl, s, lane, true);
+    } else if (state == S_START) {
+      next_slot(st, st.X[par], sl, s, lane, false);
+    }
+  }
+  __syncwarp();
+  if (lane == 0u) {
+    st.summary[s] = {sl.state, {0, 0, 0}, sl.n_journeys};
+    st.lanes[s] = lane_of(sl);
+    if (sl.state == S_RUN) {
+      atomicOr(&run_bits, 1u << (s & 31u));
+      if (sl.need_sweep) atomicOr(&sweep_bits, 1u << (s & 31u));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0u) {
+    st.run_mask[g] = run_bits;
+    st.sweep_mask[g] = sweep_bits;
+    st.any_mask[g] = 0u;
+  }
 }
 
 // ------------------------------------------------------- lower bounds
