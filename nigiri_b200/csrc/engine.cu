@@ -1139,10 +1139,15 @@ void export_slots(b2r_engine& e, std::vector<uint32_t> const& slots,
   if (e.base_recorded) B2R_CUDA(cudaEventRecord(e.ev2a, s));
   if (!recon.empty()) {
     ++e.aux_launches;
-    dev::k_reconstruct_done<<<static_cast<unsigned>(std::min<size_t>(
-                                  (recon.size() + 3) / 4, static_cast<size_t>(e.sms) * e.shape.recon_blocks_per_sm)),
-                              128, 0, s>>>(e.st, reinterpret_cast<uint32_t const*>(e.d_exp + recon_off),
-                                           static_cast<uint32_t>(recon.size()));
+    auto const n = static_cast<uint32_t>(recon.size());
+    auto const* list = reinterpret_cast<uint32_t const*>(e.d_exp + recon_off);
+    auto const most = static_cast<uint64_t>(e.sms) * e.shape.recon_blocks_per_sm;
+    // four warps a journey while the grid has a block for each
+    if (n <= most) {
+      dev::k_reconstruct_done<4><<<n, 128, 0, s>>>(e.st, list, n);
+    } else {
+      dev::k_reconstruct_done<1><<<blocks_for(n, 4U, most), 128, 0, s>>>(e.st, list, n);
+    }
     B2R_CUDA(cudaGetLastError());
   }
   uint32_t row_blocks = 1;  // spread one-to-all rows over the SMs
@@ -2531,22 +2536,26 @@ int b2r_timetable_upload(const b2r_timetable_desc* d, int device, b2r_timetable*
         dd.n_with_children = static_cast<uint32_t>(wc.size());
       }
       {  // location -> (route, stop position) pairs (reconstruct.cc:496-515 order)
-        std::vector<uint32_t> idx(nl + 1, 0U), rr;
-        std::vector<uint16_t> ss;
+        std::vector<uint32_t> idx(nl + 1, 0U), ss;
+        std::vector<uint4> rr;
         for (auto l = 0U; l != nl; ++l) {
           for (auto ri = d->location_routes_index[l]; ri != d->location_routes_index[l + 1]; ++ri) {
             auto const r = d->location_routes[ri];
-            for (auto i = d->route_stop_index[r]; i != d->route_stop_index[r + 1]; ++i) {
-              if (B2R_STOP_LOC(d->route_stops[i]) == l) {
-                rr.push_back(r);
-                ss.push_back(static_cast<uint16_t>(i - d->route_stop_index[r]));
-              }
+            auto const sb = d->route_stop_index[r], n = d->route_stop_index[r + 1] - sb;
+            auto const t0 = d->route_transport_from[r], n_t = d->route_transport_to[r] - t0;
+            for (auto i = 0U; i != n; ++i) {
+              auto const w = d->route_stops[sb + i];
+              if (B2R_STOP_LOC(w) != l) continue;
+              rr.push_back(uint4{r, d->route_stop_time_from[r] + 2U * i * n_t, t0, n_t});
+              ss.push_back(i | (i != 0U && B2R_STOP_OUT(w) ? b2r::dev::kLrsAlight : 0U) |
+                           (i + 1U != n && B2R_STOP_IN(w) ? b2r::dev::kLrsBoard : 0U) |
+                           (sorted[r] != 0U ? b2r::dev::kLrsSorted : 0U));
             }
           }
           idx[l + 1] = static_cast<uint32_t>(rr.size());
         }
         dd.lrs_idx = up(idx.data(), idx.size());
-        dd.lrs_route = up(rr.data(), rr.size());
+        dd.lrs_rec = up(rr.data(), rr.size());
         dd.lrs_stop = up(ss.data(), ss.size());
       }
       *out = t.release();
@@ -3429,7 +3438,7 @@ int b2r_raptor_reconstruct(b2r_raptor* r, const b2r_query* q, b2r_journey* j, b2
       }
       B2R_CUDA(cudaMemcpyAsync(e.st.slots, &sl, sizeof(sl), cudaMemcpyHostToDevice, s));
       B2R_CUDA(cudaMemcpyAsync(e.st.journeys, &jr, sizeof(jr), cudaMemcpyHostToDevice, s));
-      b2r::dev::k_reconstruct_one<<<1, 32, 0, s>>>(e.st, 0U, 0U);
+      b2r::dev::k_reconstruct_one<<<1, b2r::dev::kReconWarps * 32, 0, s>>>(e.st, 0U, 0U);
       B2R_CUDA(cudaGetLastError());
       B2R_CUDA(cudaMemcpyAsync(&jr, e.st.journeys, sizeof(jr), cudaMemcpyDeviceToHost, s));
       B2R_CUDA(cudaMemcpyAsync(legs, e.st.legs, b2r::dev::kMaxLegs * sizeof(b2r_leg), cudaMemcpyDeviceToHost, s));

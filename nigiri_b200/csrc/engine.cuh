@@ -26,6 +26,10 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kMaxLegs = 40;
 constexpr int kMaxTimeline = 128;
 
+// lrs_stop bits above the position: a ride can end (forward) or begin
+// (backward search) at the pair; the route's event columns are ordered
+constexpr uint32_t kLrsAlight = 1u << 16, kLrsBoard = 1u << 17, kLrsSorted = 1u << 18;
+
 // slot states
 enum : uint8_t {
   S_IDLE = 0,
@@ -83,10 +87,13 @@ struct dtt {
   uint32_t const* with_children;  // locations that have children, ascending
   uint32_t n_with_children;
   // location -> (route, stop position) pairs in the order reconstruction
-  // visits them: routes of location_routes_, then stop positions ascending
+  // visits them: routes of location_routes_, then stop positions ascending.
+  // lrs_rec: the route, its departure column at the stop (index into st; the
+  // arrival column lies n_t before it), its first transport, its number of
+  // transports n_t; lrs_stop: the position and kLrs* bits
   uint32_t const* lrs_idx;
-  uint32_t const* lrs_route;
-  uint16_t const* lrs_stop;
+  uint4 const* lrs_rec;
+  uint32_t const* lrs_stop;
   // route filters: per route, bits 0-3 transport class, 4-7 the flags set on
   // all sections, 8-11 the flags set on some sections (route_clasz_ and
   // route_flags_, timetable.h:348-355); per route stop index s of route r

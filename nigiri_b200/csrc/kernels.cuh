@@ -1181,81 +1181,92 @@ __device__ bool list_recon(state const& st, slot_t const& sl, uint32_t s, uint32
   return any;
 }
 
-// One journey (slot s, index ji) rebuilt by the calling warp.
-__device__ __forceinline__ void reconstruct_one(state const& st, uint32_t s, uint32_t ji, uint32_t lane) {
-  {
-    uint64_t t_begin = 0;
-    if (st.profile) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_begin));
-    auto& sl = st.slots[s];
-    auto& j = st.journeys[static_cast<size_t>(s) * st.max_j + ji];
-    recon_ctx c;
-    c.st = &st;
-    c.T = &st.tt;
-    c.sl = &sl;
-    c.s = s;
-    c.fwd = sl.fwd != 0;
-    c.qtag = tagcode(sl.gen_query);
-    c.base_days = sl.base_days;
-    c.base = sl.base;
-    c.ontrip = sl.ontrip != 0;
-    c.j = &j;
-    c.lane = lane;
-    c.legs = st.legs + (static_cast<size_t>(s) * st.max_j + j.block) * kMaxLegs;
-    c.run();
-    __syncwarp();
-    if (lane == 0) {
-      if (c.failed) {
-        j.error = 1;
-      } else {
-        j.reconstructed = 1;
-        j.n_legs = static_cast<uint16_t>(c.n_legs);
-      }
-      if (st.profile) {  // longest single reconstruction (ns), journeys
-        uint64_t t_end = 0;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
-        atomicMax(&st.prof[6], static_cast<unsigned long long>(t_end - t_begin));
-        atomicAdd(&st.prof[7], 1ull);
-      }
+// One journey (slot s, index ji) rebuilt by the calling group of NW warps.
+template <int NW>
+__device__ __forceinline__ void reconstruct_one(state const& st, recon_smem<NW>& sm, uint32_t s, uint32_t ji) {
+  uint64_t t_begin = 0;
+  if (st.profile) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_begin));
+  auto& sl = st.slots[s];
+  auto& j = st.journeys[static_cast<size_t>(s) * st.max_j + ji];
+  recon_ctx<NW> c;
+  c.st = &st;
+  c.T = &st.tt;
+  c.sl = &sl;
+  c.s = s;
+  c.fwd = sl.fwd != 0;
+  c.qtag = tagcode(sl.gen_query);
+  c.base_days = sl.base_days;
+  c.base = sl.base;
+  c.ontrip = sl.ontrip != 0;
+  c.j = &j;
+  c.tid = threadIdx.x % recon_ctx<NW>::kT;
+  c.lane = threadIdx.x & 31u;
+  c.wid = c.tid >> 5;
+  c.sm = &sm;
+  c.legs = sm.legs;
+  c.run();  // ends with the group in step unless it failed
+  c.sync();
+  if (!c.failed) {
+    auto* out = reinterpret_cast<uint32_t*>(st.legs + (static_cast<size_t>(s) * st.max_j + j.block) * kMaxLegs);
+    auto const* in = reinterpret_cast<uint32_t const*>(sm.legs);
+    auto const words = static_cast<uint32_t>(c.n_legs) * static_cast<uint32_t>(sizeof(b2r_leg) / 4u);
+    for (auto i = c.tid; i < words; i += recon_ctx<NW>::kT) out[i] = in[i];
+  }
+  c.sync();  // before the next journey's legs
+  if (c.tid == 0) {
+    if (c.failed) {
+      j.error = 1;
+    } else {
+      j.reconstructed = 1;
+      j.n_legs = static_cast<uint16_t>(c.n_legs);
+    }
+    if (st.profile) {  // longest single reconstruction (ns), journeys
+      uint64_t t_end = 0;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
+      atomicMax(&st.prof[6], static_cast<unsigned long long>(t_end - t_begin));
+      atomicAdd(&st.prof[7], 1ull);
     }
   }
 }
 
 // The journeys listed at the end of the last super-step (queries with
-// several start-time groups: their next group changes the round times).
-// Their slots wait (S_RECON) while the round kernels of the other slots run
-// beside this one; the step's k_end joins both and sends them on.
-__global__ void k_reconstruct(state st) {
-  auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+// several start-time groups: their next group changes the round times), a
+// block each.  Their slots wait (S_RECON) while the round kernels of the
+// other slots run beside this one; the step's k_end joins both and sends
+// them on.
+constexpr int kReconWarps = 4;
+__global__ void __launch_bounds__(kReconWarps * 32) k_reconstruct(state st) {
+  __shared__ recon_smem<kReconWarps> sm;
   auto const n = st.counters[recon_counter(st.counters[C_PAR] ^ 1u)];
-  for (auto i = warp; i < n; i += n_warps) {
+  for (auto i = blockIdx.x; i < n; i += gridDim.x) {
     auto const e = st.recon_list[i];
-    reconstruct_one(st, e >> 16, e & 0xFFFFu, lane);
+    reconstruct_one<kReconWarps>(st, sm, e >> 16, e & 0xFFFFu);
   }
 }
 
-// One given journey of slot s (index ji), one warp: the Algo interface's
-// reconstruct.
-__global__ void k_reconstruct_one(state st, uint32_t s, uint32_t ji) {
-  reconstruct_one(st, s, ji, threadIdx.x & 31u);
+// One given journey of slot s (index ji): the Algo interface's reconstruct.
+__global__ void __launch_bounds__(kReconWarps * 32) k_reconstruct_one(state st, uint32_t s, uint32_t ji) {
+  __shared__ recon_smem<kReconWarps> sm;
+  reconstruct_one<kReconWarps>(st, sm, s, ji);
 }
 
 // The journeys of finished slots whose reconstruction was deferred, listed
 // by the host as (slot << 16 | journey index): launched on the export stream
 // while the next super-steps run.  A finished slot is left alone by the
-// super-step kernels, so its round times are stable.
-__global__ void k_reconstruct_done(state st, uint32_t const* list, uint32_t n) {
-  auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
-  for (auto i = warp; i < n; i += n_warps) {
+// super-step kernels, so its round times are stable.  Blocks of 128 threads:
+// one group of four warps, or four of one.
+template <int NW>
+__global__ void __launch_bounds__(128) k_reconstruct_done(state st, uint32_t const* list, uint32_t n) {
+  constexpr auto kGroups = 4 / NW;
+  __shared__ recon_smem<NW> sm[kGroups];
+  auto const grp = threadIdx.x / (NW * 32u);
+  for (auto i = blockIdx.x * kGroups + grp; i < n; i += gridDim.x * kGroups) {
     auto const e = list[i];
     auto const s = e >> 16, ji = e & 0xFFFFu;
     auto const& sl = st.slots[s];
     if (!sl.recon_defer || ji >= sl.n_journeys) continue;
     if (!recon_wanted(sl, st.journeys[static_cast<size_t>(s) * st.max_j + ji])) continue;
-    reconstruct_one(st, s, ji, lane);
+    reconstruct_one<NW>(st, sm[grp], s, ji);
   }
 }
 

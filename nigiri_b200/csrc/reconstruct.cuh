@@ -1,18 +1,43 @@
-// Device-side journey reconstruction: one warp per journey walks the round
-// times of its query backwards (src/routing/raptor/reconstruct.cc:22-877 for
-// Vias = 0 and no real-time overlay) and then applies the footpath
-// optimisations of src/routing/raptor/optimize_footpaths.cc.  The search for
-// the transport that produced a label is split across the lanes (one
-// (route, stop position) candidate per lane); a ballot keeps the first
-// success in the reference's iteration order.  The sequential parts run
-// redundantly on all lanes; lane 0 owns the journey's leg block.
+// Device-side journey reconstruction: a group of NW warps per journey walks
+// the round times of its query backwards (src/routing/raptor/reconstruct.cc:
+// 22-877 for Vias = 0) and then applies the footpath optimisations of
+// src/routing/raptor/optimize_footpaths.cc.
+//
+// A journey is a chain of dependent loads, leg after leg, so what bounds the
+// kernel is that chain's length, not bandwidth.  The search for the
+// transport that produced a label -- every (route, stop position) pair of
+// every footpath candidate, several hundred at a busy stop -- is split
+// across the group's threads and the first success in the reference's
+// iteration order taken; each pair's record (lrs_rec) holds what its search
+// needs, so no route array stands between the pair and its event column.
+// The sequential parts run redundantly on all threads; the legs live in
+// shared memory until the journey is finished.  NW = 4 where journeys are
+// few and their latency counts (4 x 32 pairs a pass), NW = 1 where there
+// are more journeys than the device has room for groups of four.
 #pragma once
 
 #include "engine.cuh"
 
 namespace b2r::dev {
 
+// a (route, stop position) pair whose event column holds the wanted minute
+struct recon_cand {
+  uint32_t t, day, i, sec, r, owner, is_rt;
+  uint4 rec;
+};
+
+template <int NW>
+struct recon_smem {
+  b2r_leg legs[kMaxLegs];
+  recon_cand cand[NW * 32];
+  uint32_t mask[NW];
+  double pen[NW];
+  uint32_t pen_at[NW];
+};
+
+template <int NW>
 struct recon_ctx {
+  static constexpr uint32_t kT = NW * 32u;  // threads of the group
   state const* st;
   dtt const* T;
   slot_t const* sl;
@@ -23,11 +48,21 @@ struct recon_ctx {
   uint16_t base;
   bool ontrip;
   journey_rec* j;
-  b2r_leg* legs;       // kMaxLegs, written by lane 0
+  recon_smem<NW>* sm;
+  b2r_leg* legs;       // sm->legs, written by thread 0
   int n_legs;
   bool failed;
-  uint32_t lane;
-  b2r_leg last;        // last pushed leg (all lanes)
+  uint32_t lane, wid, tid;
+  b2r_leg last;        // last pushed leg (all threads)
+
+  __device__ static void sync() {
+    if constexpr (NW == 1) __syncwarp();
+    else __syncthreads();
+  }
+  __device__ static bool any(bool x) {
+    if constexpr (NW == 1) return __any_sync(kFull, x);
+    else return __syncthreads_or(x) != 0;
+  }
 
   // ------------------------------------------------------------- access
   __device__ int rt_t(unsigned k, uint32_t l) const {  // delta_t of round_times[k][l]
@@ -39,13 +74,7 @@ struct recon_ctx {
   __device__ int dir(int a) const { return fwd ? a : -a; }
   __device__ uint32_t n_stops(uint32_t r) const { return T->route_stop_idx[r + 1] - T->route_stop_idx[r]; }
   __device__ uint32_t stopw(uint32_t r, uint32_t i) const { return T->route_stops[T->route_stop_idx[r] + i]; }
-  __device__ uint16_t ev(uint32_t t, uint32_t s_idx, bool arr) const {
-    auto const r = T->transport_route[t];
-    auto const n_t = T->route_tr_to[r] - T->route_tr_from[r];
-    return T->st[T->route_st_from[r] + n_t * (s_idx * 2u - (arr ? 1u : 0u)) + (t - T->route_tr_from[r])];
-  }
-  __device__ int32_t ev_time(uint32_t t, uint16_t day, uint32_t s_idx, bool arr) const {
-    auto const e = ev(t, s_idx, arr);
+  __device__ int32_t day_time(uint16_t day, uint16_t e) const {
     return (T->internal_from_days + static_cast<int32_t>(day)) * 1440 + (e & 31) * 1440 + (e >> 5);
   }
   __device__ int unix_to_delta(int32_t t) const { return clamp16(t - base_days * 1440); }
@@ -134,32 +163,24 @@ struct recon_ctx {
       failed = true;
       return;
     }
-    if (lane == 0) legs[n_legs] = l;
+    if (tid == 0) legs[n_legs] = l;
     ++n_legs;
     last = l;
-  }
-
-  __device__ static b2r_leg shfl_leg(b2r_leg const& l, int src) {
-    static_assert(sizeof(b2r_leg) % 4 == 0, "leg size");
-    constexpr int kW = sizeof(b2r_leg) / 4;
-    uint32_t w[kW];
-    memcpy(w, &l, sizeof(b2r_leg));
-#pragma unroll
-    for (int i = 0; i < kW; ++i) w[i] = __shfl_sync(kFull, w[i], src);
-    b2r_leg out;
-    memcpy(&out, w, sizeof(b2r_leg));
-    return out;
   }
 
   // reconstruct.cc:180-280 (single pass: no vias).  The stops before the
   // exit stop are split across the lanes; the ballot keeps the first one in
   // the reference's order.  A section lacking one of the flags `sec` ends
   // the ride (reconstruct.cc:239-250): stops at or past the first such
-  // section do not count.  Called by the whole warp with equal arguments.
-  __device__ bool find_start_in_prev_round(unsigned k, uint32_t t, uint16_t day, uint32_t finish,
+  // section do not count.  rec: the exit stop's pair record.  Called by
+  // whole warps with equal arguments.
+  __device__ bool find_start_in_prev_round(unsigned k, uint4 rec, uint32_t t, uint16_t day, uint32_t finish,
                                            uint32_t sec, b2r_leg& out) const {
-    auto const r = T->transport_route[t];
-    auto const size = n_stops(r);
+    auto const sb = T->route_stop_idx[rec.x];
+    auto const size = T->route_stop_idx[rec.x + 1] - sb;
+    // event column entry of trip t at stop i: evs[2 i n_t], its arrival n_t before
+    auto const n_t = rec.w;
+    auto const* evs = T->st + (rec.y - 2u * finish * n_t) + (t - rec.z);
     auto const n = fwd ? finish + 1u : size - finish;
     for (auto i0 = 1u; i0 < n; i0 += 32u) {
       auto const i = i0 + lane;
@@ -168,14 +189,15 @@ struct recon_ctx {
       int event_time = 0;
       if (i < n) {
         si = fwd ? finish - i : finish + i;
-        auto const w = stopw(r, si);
+        auto const w = T->route_stops[sb + si];
+        auto const e = evs[fwd ? 2u * si * n_t : (2u * si - 1u) * n_t];
         l = B2R_STOP_LOC(w);
         // departure section forward, arrival section backward
-        cut = sec != 0u && !section_ok(*T, T->route_stop_idx[r], fwd ? si : si - 1u, sec);
+        cut = sec != 0u && !section_ok(*T, sb, fwd ? si : si - 1u, sec);
         // plain in / out bits for every profile: reconstruct.cc:252-253
         // passes the bool is_wheelchair as a profile index (0 or 1)
         if (!cut && !((fwd && !B2R_STOP_IN(w)) || (!fwd && !B2R_STOP_OUT(w)))) {
-          event_time = unix_to_delta(ev_time(t, day, si, !fwd));
+          event_time = unix_to_delta(day_time(day, e));
           auto const round_time = rt_t(k - 1, l);
           ok = beq(round_time, event_time) ||
                (k == 1 && sl->start_mode == B2R_MATCH_EQUIVALENT && is_journey_start(l) &&
@@ -190,8 +212,8 @@ struct recon_ctx {
         si = __shfl_sync(kFull, si, src);
         l = __shfl_sync(kFull, l, src);
         event_time = __shfl_sync(kFull, event_time, src);
-        out = make_leg(l, B2R_STOP_LOC(stopw(r, finish)), delta_to_unix(event_time),
-                       ev_time(t, day, finish, fwd));
+        auto const e = evs[fwd ? (2u * finish - 1u) * n_t : 2u * finish * n_t];
+        out = make_leg(l, B2R_STOP_LOC(T->route_stops[sb + finish]), delta_to_unix(event_time), day_time(day, e));
         set_run(out, t, day, si, finish);
         return true;
       }
@@ -245,16 +267,16 @@ struct recon_ctx {
     return false;
   }
 
-  // The transports of route r whose event at stop si has the minutes after
-  // midnight of `time` (reconstruct.cc:292-373), one at a time from
-  // `cursor`: columns are ordered by minutes after midnight, so they form
-  // one run found by binary search and visited in index order.
-  __device__ uint32_t first_cursor(int time, uint32_t r, uint32_t si) const {
-    if (!T->route_sorted[r]) return 0u;
+  // The transports of a pair's route whose event at its stop has the minutes
+  // after midnight of `time` (reconstruct.cc:292-373), one at a time from
+  // `cursor`: columns are ordered by minutes after midnight (kLrsSorted), so
+  // they form one run found by binary search and visited in index order.
+  __device__ uint16_t const* pair_col(uint4 rec) const { return T->st + rec.y - (fwd ? rec.w : 0u); }
+  __device__ uint32_t first_cursor(int time, uint4 rec, bool sorted) const {
+    if (!sorted) return 0u;
     auto const mam = static_cast<int16_t>((static_cast<int>(base) * 1440 + time) % 1440);
-    auto const n_t = T->route_tr_to[r] - T->route_tr_from[r];
-    auto const* col = T->st + T->route_st_from[r] + n_t * (si * 2u - (fwd ? 1u : 0u));
-    uint32_t lo = 0, hi = n_t;
+    auto const* col = pair_col(rec);
+    uint32_t lo = 0, hi = rec.w;
     while (lo < hi) {
       auto const mid = (lo + hi) >> 1;
       if ((col[mid] >> 5) < static_cast<uint16_t>(mam < 0 ? 0 : mam)) lo = mid + 1;
@@ -262,28 +284,27 @@ struct recon_ctx {
     }
     return lo;
   }
-  __device__ bool next_transport(int time, uint32_t r, uint32_t si, uint32_t& cursor, uint32_t& t,
-                                 uint16_t& tday) const {
+  __device__ bool next_transport(int time, uint4 rec, bool sorted, uint32_t& cursor, uint32_t& t,
+                                 uint32_t& tday) const {
     auto const minutes = static_cast<int>(base) * 1440 + time;
     auto const day = static_cast<uint16_t>(minutes / 1440);
     auto const mam = static_cast<int16_t>(minutes % 1440);
-    auto const t0 = T->route_tr_from[r], n_t = T->route_tr_to[r] - t0;
-    auto const* col = T->st + T->route_st_from[r] + n_t * (si * 2u - (fwd ? 1u : 0u));
-    for (auto x = cursor; x < n_t; ++x) {
+    auto const* col = pair_col(rec);
+    for (auto x = cursor; x < rec.w; ++x) {
       auto const cnt = delta_count(col[x]);
       auto const m = static_cast<int16_t>(cnt % 1440);
       if (m != mam) {
-        if (T->route_sorted[r] && m > mam) break;
+        if (sorted && m > mam) break;
         continue;
       }
       auto const td = static_cast<uint16_t>(static_cast<int>(day) - cnt / 1440);
-      if (!bf_test(*T, T->transport_bf[t0 + x], td)) continue;
+      if (!bf_test(*T, T->transport_bf[rec.z + x], td)) continue;
       cursor = x + 1u;
-      t = t0 + x;
+      t = rec.z + x;
       tday = td;
       return true;
     }
-    cursor = n_t;
+    cursor = rec.w;
     return false;
   }
 
@@ -292,10 +313,10 @@ struct recon_ctx {
   // `time(f)`; its real-time (run, stop position) pairs and then its (route,
   // stop position) pairs are visited in the reference's order
   // (reconstruct.cc:381-452 first).  All pairs of all candidates form one
-  // sequence that the lanes take 32 at a time; the first success in
+  // sequence that the group takes kT at a time; the first success in
   // sequence order wins.
-  // get(f, target, time) describes candidate f (lane-local); returns the
-  // winning candidate or -1.
+  // get(f, target, time) describes candidate f (lane-local; false: no such
+  // candidate); returns the winning candidate or -1.
   template <typename Get>
   __device__ int get_transport(unsigned k, uint32_t n_cand, Get&& get, b2r_leg& out) const {
     for (auto f0 = 0u; f0 < n_cand; f0 += 32u) {
@@ -303,8 +324,7 @@ struct recon_ctx {
       auto const f = f0 + lane;
       uint32_t tg = 0, pb = 0, cnt = 0, rb = 0, rcnt = 0;
       int tm = 0;
-      if (f < n_cand) {
-        get(f, tg, tm);
+      if (f < n_cand && get(f, tg, tm)) {
         pb = T->lrs_idx[tg];
         rb = T->lrs_rt_idx[tg];
         rcnt = T->lrs_rt_idx[tg + 1] - rb;
@@ -316,8 +336,8 @@ struct recon_ctx {
         if (lane >= o) end += v;
       }
       auto const total = __shfl_sync(kFull, end, 31);
-      for (auto p0 = 0u; p0 < total; p0 += 32u) {
-        auto const p = p0 + lane;
+      for (auto p0 = 0u; p0 < total; p0 += kT) {
+        auto const p = p0 + tid;
         // owner candidate of pair p: the first lane whose prefix end > p
         uint32_t owner = 0;
         for (auto b = 16u; b > 0u; b >>= 1) {
@@ -331,51 +351,67 @@ struct recon_ctx {
         auto const o_cnt = __shfl_sync(kFull, cnt, static_cast<int>(owner));
         auto const o_rb = __shfl_sync(kFull, rb, static_cast<int>(owner));
         auto const o_rcnt = __shfl_sync(kFull, rcnt, static_cast<int>(owner));
-        bool has = false, is_rt = false;
-        uint32_t r = 0, i = 0, cursor = 0, t = 0, sec = 0;
-        uint16_t tday = 0;
+        bool has = false, sorted = false;
+        recon_cand c{};
+        c.owner = owner;
+        uint32_t cursor = 0;
         if (p < total && p - (o_end - o_cnt) < o_rcnt) {  // a real-time run at the stop
           auto const x = o_rb + (p - (o_end - o_cnt));
-          is_rt = true;
-          r = T->lrs_rt[x];
-          i = static_cast<uint32_t>(T->lrs_rt_stop[x]);
-          auto const sb = T->rt_stop_idx[r];
-          auto const n = T->rt_stop_idx[r + 1] - sb;
-          auto const w = T->rt_stops[sb + i];
+          c.is_rt = 1u;
+          c.r = T->lrs_rt[x];
+          c.i = static_cast<uint32_t>(T->lrs_rt_stop[x]);
+          auto const sb = T->rt_stop_idx[c.r];
+          auto const n = T->rt_stop_idx[c.r + 1] - sb;
+          auto const w = T->rt_stops[sb + c.i];
           auto const allowed = (sl->allowed_claszes == 0xFFFFu && sl->req_flags == 0u) ||
-                               filter_allowed(T->rt_filter[r], sl->allowed_claszes, sl->req_flags, sec);
+                               filter_allowed(T->rt_filter[c.r], sl->allowed_claszes, sl->req_flags, c.sec);
           // an earlier arrival than the label is accepted (reconstruct.cc:437-440)
           has = allowed &&
-                !((fwd && (i == 0u || !B2R_STOP_OUT(w))) || (!fwd && (i + 1u == n || !B2R_STOP_IN(w)))) &&
-                beq(T->rt_times[2ull * (sb - r) + 2u * i - (fwd ? 1u : 0u)], delta_to_unix(o_tm));
+                !((fwd && (c.i == 0u || !B2R_STOP_OUT(w))) || (!fwd && (c.i + 1u == n || !B2R_STOP_IN(w)))) &&
+                beq(T->rt_times[2ull * (sb - c.r) + 2u * c.i - (fwd ? 1u : 0u)], delta_to_unix(o_tm));
         } else if (p < total) {
           auto const x = o_pb + (p - (o_end - o_cnt) - o_rcnt);
-          r = T->lrs_route[x];
-          i = static_cast<uint32_t>(T->lrs_stop[x]);
-          auto const w = stopw(r, i);
-          auto const n = n_stops(r);
+          c.rec = T->lrs_rec[x];
+          auto const w = T->lrs_stop[x];
+          c.r = c.rec.x;
+          c.i = w & 0xFFFFu;
+          sorted = (w & kLrsSorted) != 0u;
           auto const allowed = (sl->allowed_claszes == 0xFFFFu && sl->req_flags == 0u) ||
-                               route_allowed(*T, r, sl->allowed_claszes, sl->req_flags, sec);
-          if (allowed &&
-              !((fwd && (i == 0u || !B2R_STOP_OUT(w))) || (!fwd && (i + 1u == n || !B2R_STOP_IN(w))))) {
-            cursor = first_cursor(o_tm, r, i);
-            has = next_transport(o_tm, r, i, cursor, t, tday);
+                               route_allowed(*T, c.r, sl->allowed_claszes, sl->req_flags, c.sec);
+          // arrivals: not at the first stop, and alighting allowed (backward: departures)
+          if (allowed && (w & (fwd ? kLrsAlight : kLrsBoard)) != 0u) {
+            cursor = first_cursor(o_tm, c.rec, sorted);
+            has = next_transport(o_tm, c.rec, sorted, cursor, c.t, c.day);
           }
         }
-        for (auto m = __ballot_sync(kFull, has); m != 0u; m = __ballot_sync(kFull, has)) {
-          auto const src = static_cast<int>(__ffs(m) - 1);
-          auto const bt = __shfl_sync(kFull, t, src);
-          auto const bday = static_cast<uint16_t>(__shfl_sync(kFull, static_cast<uint32_t>(tday), src));
-          auto const bi = __shfl_sync(kFull, i, src);
-          auto const bsec = __shfl_sync(kFull, sec, src);
-          auto const brt = __shfl_sync(kFull, is_rt ? 1u : 0u, src) != 0u;
-          auto const bx = __shfl_sync(kFull, r, src);
-          if (brt ? find_start_in_prev_round_rt(k, bx, bi, bsec, out)
-                  : find_start_in_prev_round(k, bt, bday, bi, bsec, out)) {
-            return static_cast<int>(f0 + __shfl_sync(kFull, owner, src));
+        if (!any(has)) continue;
+        if (has) sm->cand[tid] = c;
+        auto const mine = __ballot_sync(kFull, has);
+        if (lane == 0u) sm->mask[wid] = mine;
+        sync();
+        while (true) {
+          uint32_t w = 0, m = 0;
+          for (; w != NW; ++w) {
+            m = sm->mask[w];
+            if (m != 0u) break;
           }
-          if (static_cast<int>(lane) == src) has = !is_rt && next_transport(o_tm, r, i, cursor, t, tday);
+          if (m == 0u) break;
+          auto const src = w * 32u + static_cast<uint32_t>(__ffs(m) - 1);
+          auto const& b = sm->cand[src];
+          if (b.is_rt != 0u ? find_start_in_prev_round_rt(k, b.r, b.i, b.sec, out)
+                            : find_start_in_prev_round(k, b.rec, b.t, static_cast<uint16_t>(b.day), b.i, b.sec, out)) {
+            auto const won = static_cast<int>(f0 + b.owner);
+            sync();  // read by all before the next search writes
+            return won;
+          }
+          sync();
+          if (tid == src) {  // its next trip at the same minute
+            if (c.is_rt == 0u && next_transport(o_tm, c.rec, sorted, cursor, c.t, c.day)) sm->cand[tid] = c;
+            else sm->mask[w] = m & (m - 1u);
+          }
+          sync();
         }
+        sync();
       }
     }
     return -1;
@@ -390,6 +426,7 @@ struct recon_ctx {
     auto const one = [&](uint32_t, uint32_t& tg, int& tm) {
       tg = target;
       tm = fp_start;
+      return true;
     };
     if (get_transport(k, 1u, one, tr_leg) < 0) return false;
     fp_leg = make_leg(target, l, delta_to_unix(fp_start), delta_to_unix(fp_start + dir(d)));
@@ -402,6 +439,35 @@ struct recon_ctx {
     auto const curr = rt_t(k, l);
     if (sl->dest_mode == B2R_MATCH_INTERMODAL && k == j->transfers + 1u) {
       auto const* o = dest_offs();
+      // destinations without generated tracks: their offsets are the
+      // candidates of one search, in order
+      auto tracks = false;
+      if (T->children_idx != nullptr && T->loc_type != nullptr) {
+        for (auto i = lane; i < sl->n_doff; i += 32u) {
+          for (auto c = T->children_idx[o[i].target]; c != T->children_idx[o[i].target + 1]; ++c) {
+            tracks = tracks || T->loc_type[T->children[c]] == B2R_LOC_GENERATED_TRACK;
+          }
+        }
+        tracks = __any_sync(kFull, tracks);
+      }
+      if (!tracks) {
+        auto const start_of = [&](b2r_offset const& x) {
+          return static_cast<int>(static_cast<int16_t>(curr - dir(static_cast<int>(x.duration))));
+        };
+        auto const get = [&](uint32_t f, uint32_t& tg, int& tm) {
+          auto const x = o[f];
+          tg = x.target;
+          tm = start_of(x);
+          return x.duration < 511;
+        };
+        auto const f = get_transport(k, sl->n_doff, get, tr_leg);
+        if (f < 0) return false;
+        auto const x = o[f];
+        auto const fp_start = start_of(x);
+        fp_leg = make_leg(x.target, l, delta_to_unix(fp_start), delta_to_unix(fp_start + dir(static_cast<int>(x.duration))));
+        set_off(fp_leg, x);
+        return true;
+      }
       for (auto i = 0u; i != sl->n_doff; ++i) {
         if (o[i].duration >= 511) continue;
         auto found = false;
@@ -455,6 +521,7 @@ struct recon_ctx {
       int dur = 0;
       raw(f, tg, dur);
       tm = static_cast<int>(static_cast<int16_t>(curr - dir(eff(f, dur))));
+      return true;
     };
     auto const f = get_transport(k, 1u + (idx[l + 1] - fb), get, tr_leg);
     if (f < 0) return false;
@@ -509,152 +576,176 @@ struct recon_ctx {
   }
 
   // ---------------------------------------------- optimize_footpaths.cc
-  // the stops and event times of a leg's run (rt::frun): a real-time run's
-  // own, else the static trip's
-  __device__ uint32_t r_of(b2r_leg const& l) const { return T->transport_route[l.transport]; }
-  __device__ uint32_t word_at(b2r_leg const& l, uint32_t si) const {
-    if (l.rt_transport != B2R_INVALID_IDX) return T->rt_stops[T->rt_stop_idx[l.rt_transport] + si];
-    return stopw(r_of(l), si);
-  }
-  __device__ uint32_t loc_at(b2r_leg const& l, uint32_t si) const { return B2R_STOP_LOC(word_at(l, si)); }
-  __device__ int32_t time_at(b2r_leg const& l, uint32_t si, bool arr) const {
+  // The stops and event times of a leg's run (rt::frun): a real-time run's
+  // own, else the static trip's.
+  struct run_view {
+    uint32_t const* words;
+    uint32_t size;
+    int32_t const* rt;    // real-time: departure of stop i at [2 i], arrival before it
+    uint16_t const* evs;  // static: departure of stop i at [2 i n_t], arrival n_t before it
+    uint32_t n_t;
+    int32_t day_min;
+    __device__ uint32_t word(uint32_t i) const { return words[i]; }
+    __device__ int32_t time(uint32_t i, bool arr) const {
+      if (rt != nullptr) return rt[2u * i - (arr ? 1u : 0u)];
+      auto const e = evs[(2u * i - (arr ? 1u : 0u)) * n_t];
+      return day_min + (e & 31) * 1440 + (e >> 5);
+    }
+  };
+  __device__ run_view view_of(b2r_leg const& l) const {
+    run_view v{};
     if (l.rt_transport != B2R_INVALID_IDX) {
       auto const x = l.rt_transport;
-      return T->rt_times[2ull * (T->rt_stop_idx[x] - x) + 2u * si - (arr ? 1u : 0u)];
+      auto const sb = T->rt_stop_idx[x];
+      v.words = T->rt_stops + sb;
+      v.size = T->rt_stop_idx[x + 1] - sb;
+      v.rt = T->rt_times + 2ull * (sb - x);
+    } else {
+      auto const r = T->transport_route[l.transport];
+      auto const sb = T->route_stop_idx[r];
+      auto const t0 = T->route_tr_from[r];
+      v.words = T->route_stops + sb;
+      v.size = T->route_stop_idx[r + 1] - sb;
+      v.n_t = T->route_tr_to[r] - t0;
+      v.evs = T->st + T->route_st_from[r] + (l.transport - t0);
+      v.day_min = (T->internal_from_days + static_cast<int32_t>(l.day)) * 1440;
     }
-    return ev_time(l.transport, l.day, si, arr);
-  }
-  __device__ uint32_t run_size(b2r_leg const& l) const {
-    if (l.rt_transport != B2R_INVALID_IDX) return T->rt_stop_idx[l.rt_transport + 1] - T->rt_stop_idx[l.rt_transport];
-    return n_stops(r_of(l));
+    return v;
   }
 
-  // optimize_footpaths.cc:15-60; `offs` = start offsets of the journey query
-  __device__ void opt_initial_departure(b2r_offset const* offs, uint32_t n_offs) {
-    if (n_legs <= 1 || legs[0].kind != B2R_LEG_OFFSET || legs[1].kind != B2R_LEG_TRANSPORT) return;
-    auto& ol = legs[0];
-    auto& tl = legs[1];
+  // The four passes over the first / last ride (optimize_footpaths.cc:
+  // 15-257) by one warp: the reference walks the ride's stops and takes every
+  // improvement in order; few stops can be reached by the offset or footpath
+  // at all, so the lanes look for those 32 stops at a time and the walk
+  // visits only them.
+  //
+  // offsets at the ride's stops: departure side (15-60), arrival side
+  // (122-187); `offs` = start / destination offsets of the journey query
+  __device__ void opt_offset(b2r_offset const* offs, uint32_t n_offs, bool dep) {
+    if (n_legs <= 1) return;
+    auto& ol = legs[dep ? 0 : n_legs - 1];
+    auto& tl = legs[dep ? 1 : n_legs - 2];
+    if (ol.kind != B2R_LEG_OFFSET || tl.kind != B2R_LEG_TRANSPORT) return;
+    auto const v = view_of(tl);
+    auto const from = dep ? 0u : static_cast<uint32_t>(tl.stop_from + 1u);
+    auto const end = dep ? static_cast<uint32_t>(tl.stop_to - 1u) : v.size;
     auto best = static_cast<int>(ol.duration);
-    auto const end = static_cast<uint32_t>(tl.stop_to - 1u);
-    for (auto si = 0u; si < end; ++si) {
-      if (!B2R_STOP_IN(word_at(tl, si))) continue;
-      for (auto i = 0u; i != n_offs; ++i) {
-        auto const& o = offs[i];
-        if (best <= o.duration || o.target != loc_at(tl, si)) continue;
-        auto const dep = time_at(tl, si, false);
-        auto const o_start = dep - o.duration;
-        if (ol.dep_time <= o_start) {
-          ol.to = loc_at(tl, si);
-          ol.dep_time = o_start;
-          ol.arr_time = dep;
-          set_off(ol, o);
-          tl.from = loc_at(tl, si);
-          tl.dep_time = dep;
-          tl.stop_from = static_cast<uint16_t>(si);
-          best = o.duration;
+    auto bound = dep ? ol.dep_time : ol.arr_time;
+    uint32_t at = B2R_INVALID_IDX, at_loc = 0, which = 0;
+    int32_t at_time = 0;
+    for (auto s0 = from; s0 < end; s0 += 32u) {
+      auto const si = s0 + lane;
+      auto has = false;
+      uint32_t loc = 0;
+      int32_t tm = 0;
+      if (si < end) {
+        auto const w = v.word(si);
+        loc = B2R_STOP_LOC(w);
+        if (dep ? B2R_STOP_IN(w) : B2R_STOP_OUT(w)) {
+          for (auto i = 0u; i != n_offs; ++i) has = has || (offs[i].target == loc && offs[i].duration < best);
         }
+        if (has) tm = v.time(si, !dep);
       }
-    }
-  }
-
-  __device__ void opt_initial_start_footpath() {  // :62-120
-    if (n_legs <= 1 || legs[0].kind != B2R_LEG_FOOTPATH || legs[1].kind != B2R_LEG_TRANSPORT) return;
-    auto& fl = legs[0];
-    auto& tl = legs[1];
-    auto const start_loc = fl.from;
-    auto best = static_cast<int>(adjusted<int16_t>(sl->tts, fl.duration));
-    auto const end = static_cast<uint32_t>(tl.stop_to - 1u);
-    for (auto si = 0u; si < end; ++si) {
-      if (!B2R_STOP_IN(word_at(tl, si))) continue;
-      auto const* oidx = fp_index(*T, sl->prf, true);  // optimize_footpaths.cc:91
-      auto const* ofp = fp_words(*T, sl->prf, true);
-      for (auto i = oidx[start_loc]; i != oidx[start_loc + 1]; ++i) {
-        auto const fp = ofp[i];
-        if (B2R_FP_TARGET(fp) != loc_at(tl, si)) continue;
-        auto const d = static_cast<int>(adjusted<int16_t>(sl->tts, static_cast<int16_t>(B2R_FP_DURATION(fp))));
-        if (d < best) {
-          auto const dep = time_at(tl, si, false);
-          auto const fp_start = dep - d;
-          if (fl.dep_time <= fp_start) {
-            fl.to = loc_at(tl, si);
-            fl.dep_time = fp_start;
-            fl.arr_time = dep;
-            set_fp(fl, loc_at(tl, si), d);
-            tl.from = loc_at(tl, si);
-            tl.dep_time = dep;
-            tl.stop_from = static_cast<uint16_t>(si);
-            best = d;
+      for (auto m = __ballot_sync(kFull, has); m != 0u; m &= m - 1u) {
+        auto const src = __ffs(m) - 1;
+        auto const x_loc = __shfl_sync(kFull, loc, src);
+        auto const x_tm = __shfl_sync(kFull, tm, src);
+        for (auto i = 0u; i != n_offs; ++i) {
+          auto const o = offs[i];
+          if (best <= o.duration || o.target != x_loc) continue;
+          auto const o_time = dep ? x_tm - o.duration : x_tm + o.duration;
+          if (dep ? bound <= o_time : o_time <= bound) {
+            bound = o_time;
+            best = o.duration;
+            at = s0 + static_cast<uint32_t>(src);
+            at_loc = x_loc;
+            at_time = x_tm;
+            which = i;
           }
         }
-        break;
       }
+    }
+    __syncwarp();
+    if (at == B2R_INVALID_IDX || lane != 0u) return;
+    set_off(ol, offs[which]);
+    if (dep) {
+      ol.to = tl.from = at_loc;
+      ol.dep_time = bound;
+      ol.arr_time = tl.dep_time = at_time;
+      tl.stop_from = static_cast<uint16_t>(at);
+    } else {
+      ol.from = tl.to = at_loc;
+      ol.dep_time = tl.arr_time = at_time;
+      ol.arr_time = bound;
+      tl.stop_to = static_cast<uint16_t>(at + 1u);
     }
   }
 
-  __device__ void opt_last_arrival(b2r_offset const* offs, uint32_t n_offs) {  // :122-187
-    if (n_legs <= 1 || legs[n_legs - 1].kind != B2R_LEG_OFFSET || legs[n_legs - 2].kind != B2R_LEG_TRANSPORT) {
-      return;
-    }
-    auto& ol = legs[n_legs - 1];
-    auto& tl = legs[n_legs - 2];
-    auto best = static_cast<int>(ol.duration);
-    auto const from = static_cast<uint32_t>(tl.stop_from + 1u);
-    auto const size = run_size(tl);
-    for (auto si = from; si < size; ++si) {
-      if (!B2R_STOP_OUT(word_at(tl, si))) continue;
-      for (auto i = 0u; i != n_offs; ++i) {
-        auto const& o = offs[i];
-        if (best <= o.duration || o.target != loc_at(tl, si)) continue;
-        auto const arr = time_at(tl, si, true);
-        auto const o_end = arr + o.duration;
-        if (o_end <= ol.arr_time) {
-          ol.from = loc_at(tl, si);
-          ol.dep_time = arr;
-          ol.arr_time = o_end;
-          set_off(ol, o);
-          tl.to = loc_at(tl, si);
-          tl.arr_time = arr;
-          tl.stop_to = static_cast<uint16_t>(si + 1u);
-          best = o.duration;
-        }
-      }
-    }
-  }
-
-  __device__ void opt_final_egress_footpath() {  // :189-257
-    if (n_legs <= 1 || legs[n_legs - 1].kind != B2R_LEG_FOOTPATH || legs[n_legs - 2].kind != B2R_LEG_TRANSPORT) {
-      return;
-    }
-    auto& fl = legs[n_legs - 1];
-    auto& tl = legs[n_legs - 2];
-    auto const dest_loc = fl.to;
+  // footpaths between the journey's start / destination and the ride's
+  // stops: departure side (62-120), arrival side (189-257)
+  __device__ void opt_footpath(bool dep) {
+    if (n_legs <= 1) return;
+    auto& fl = legs[dep ? 0 : n_legs - 1];
+    auto& tl = legs[dep ? 1 : n_legs - 2];
+    if (fl.kind != B2R_LEG_FOOTPATH || tl.kind != B2R_LEG_TRANSPORT) return;
+    auto const v = view_of(tl);
+    auto const end_loc = dep ? fl.from : fl.to;
+    auto const from = dep ? 0u : static_cast<uint32_t>(tl.stop_from + 1u);
+    auto const end = dep ? static_cast<uint32_t>(tl.stop_to - 1u) : v.size;
+    auto const* idx = fp_index(*T, sl->prf, dep);  // optimize_footpaths.cc:91, 215
+    auto const* fps = fp_words(*T, sl->prf, dep);
+    auto const fb = idx[end_loc], fe = idx[end_loc + 1];
     auto best = static_cast<int>(adjusted<int16_t>(sl->tts, fl.duration));
-    auto const from = static_cast<uint32_t>(tl.stop_from + 1u);
-    auto const size = run_size(tl);
-    for (auto si = from; si < size; ++si) {
-      if (!B2R_STOP_OUT(word_at(tl, si))) continue;
-      auto const* iidx = fp_index(*T, sl->prf, false);  // optimize_footpaths.cc:215
-      auto const* ifp = fp_words(*T, sl->prf, false);
-      for (auto i = iidx[dest_loc]; i != iidx[dest_loc + 1]; ++i) {
-        auto const fp = ifp[i];
-        if (B2R_FP_TARGET(fp) != loc_at(tl, si)) continue;
-        auto const d = static_cast<int>(adjusted<int16_t>(sl->tts, static_cast<int16_t>(B2R_FP_DURATION(fp))));
-        if (d < best) {
-          auto const arr = time_at(tl, si, true);
-          auto const fp_end = arr + d;
-          if (fp_end <= fl.arr_time) {
-            fl.from = loc_at(tl, si);
-            fl.dep_time = arr;
-            fl.arr_time = fp_end;
-            set_fp(fl, dest_loc, d);
-            tl.to = loc_at(tl, si);
-            tl.arr_time = arr;
-            tl.stop_to = static_cast<uint16_t>(si + 1u);
-            best = d;
+    auto bound = dep ? fl.dep_time : fl.arr_time;
+    uint32_t at = B2R_INVALID_IDX, at_loc = 0;
+    int32_t at_time = 0;
+    for (auto s0 = from; s0 < end; s0 += 32u) {
+      auto const si = s0 + lane;
+      auto has = false;
+      uint32_t loc = 0;
+      int32_t tm = 0;
+      int d = 0;
+      if (si < end) {
+        auto const w = v.word(si);
+        loc = B2R_STOP_LOC(w);
+        if (dep ? B2R_STOP_IN(w) : B2R_STOP_OUT(w)) {
+          for (auto i = fb; i != fe; ++i) {
+            if (B2R_FP_TARGET(fps[i]) != loc) continue;
+            d = static_cast<int>(adjusted<int16_t>(sl->tts, static_cast<int16_t>(B2R_FP_DURATION(fps[i]))));
+            has = d < best;
+            break;
           }
         }
-        break;
+        if (has) tm = v.time(si, !dep);
       }
+      for (auto m = __ballot_sync(kFull, has); m != 0u; m &= m - 1u) {
+        auto const src = __ffs(m) - 1;
+        auto const x_loc = __shfl_sync(kFull, loc, src);
+        auto const x_tm = __shfl_sync(kFull, tm, src);
+        auto const x_d = __shfl_sync(kFull, d, src);
+        auto const f_time = dep ? x_tm - x_d : x_tm + x_d;
+        if (x_d < best && (dep ? bound <= f_time : f_time <= bound)) {
+          bound = f_time;
+          best = x_d;
+          at = s0 + static_cast<uint32_t>(src);
+          at_loc = x_loc;
+          at_time = x_tm;
+        }
+      }
+    }
+    __syncwarp();
+    if (at == B2R_INVALID_IDX || lane != 0u) return;
+    set_fp(fl, dep ? at_loc : end_loc, best);
+    if (dep) {
+      fl.to = tl.from = at_loc;
+      fl.dep_time = bound;
+      fl.arr_time = tl.dep_time = at_time;
+      tl.stop_from = static_cast<uint16_t>(at);
+    } else {
+      fl.from = tl.to = at_loc;
+      fl.dep_time = tl.arr_time = at_time;
+      fl.arr_time = bound;
+      tl.stop_to = static_cast<uint16_t>(at + 1u);
     }
   }
 
@@ -674,43 +765,44 @@ struct recon_ctx {
 
   // optimize_footpaths.cc:285-450 (no vias).  For each transport-footpath-
   // transport triple the (exit stop, entry stop) pairs are split across the
-  // lanes; pairs do not depend on each other except through the running best
+  // group; pairs do not depend on each other except through the running best
   // penalty, so the sequential loop keeps the first pair (in its order) with
-  // the smallest penalty below the initial one, which is what the warp
-  // reduction over (penalty, pair index) selects.  Called by the whole warp;
-  // lane 0 writes the legs.
+  // the smallest penalty below the initial one, which is what the reduction
+  // over (penalty, pair index) selects.  Called by the whole group; the
+  // winning pair's thread writes the legs.
   __device__ void opt_transfers() {
     for (auto i = 0; i + 2 < n_legs; ++i) {
-      __syncwarp();
+      sync();
       auto const lf = legs[i];
       auto const lp = legs[i + 1];
       auto const lt = legs[i + 2];
       if (lf.kind != B2R_LEG_TRANSPORT || lp.kind != B2R_LEG_FOOTPATH || lt.kind != B2R_LEG_TRANSPORT) continue;
+      auto const vf = view_of(lf), vt = view_of(lt);
       auto const from_start = static_cast<uint32_t>(lf.stop_from + 1u);
-      auto const from_size = run_size(lf);
       auto const to_end = static_cast<uint32_t>(lt.stop_to - 1u);
       auto const pbest0 = penalty(lp.duration, lt.dep_time - lp.arr_time, lf.from, lt.to);
-      auto const n_sf = from_size > from_start ? from_size - from_start : 0u;
+      auto const n_sf = vf.size > from_start ? vf.size - from_start : 0u;
       auto const n_pairs = n_sf * to_end;
+      auto const* oidx = fp_index(*T, sl->prf, true);  // optimize_footpaths.cc:405
+      auto const* ofp = fp_words(*T, sl->prf, true);
       double best = pbest0;
       uint32_t best_idx = 0xFFFFFFFFu, best_fp = 0;
       int32_t best_arr = 0, best_dep = 0, best_d = 0;
-      for (auto x = lane; x < n_pairs; x += 32u) {
+      for (auto x = tid; x < n_pairs; x += kT) {
         auto const sf = from_start + x / to_end, s2 = x % to_end;
-        if (!B2R_STOP_OUT(word_at(lf, sf)) || !B2R_STOP_IN(word_at(lt, s2))) continue;
-        auto const a = loc_at(lf, sf), b = loc_at(lt, s2);
-        auto const* oidx = fp_index(*T, sl->prf, true);  // optimize_footpaths.cc:405
-        auto const* ofp = fp_words(*T, sl->prf, true);
-        for (auto y = oidx[a]; y != oidx[a + 1]; ++y) {
+        auto const wf = vf.word(sf), wt = vt.word(s2);
+        if (!B2R_STOP_OUT(wf) || !B2R_STOP_IN(wt)) continue;
+        auto const a = B2R_STOP_LOC(wf), b = B2R_STOP_LOC(wt);
+        for (auto y = oidx[a], ye = oidx[a + 1]; y != ye; ++y) {
           auto const fp = ofp[y];
           if (B2R_FP_TARGET(fp) != b) continue;
           auto const d = static_cast<int>(adjusted<int16_t>(sl->tts, static_cast<int16_t>(B2R_FP_DURATION(fp))));
-          auto const arr = time_at(lf, sf, true);
-          auto const dep = time_at(lt, s2, false);
+          auto const arr = vf.time(sf, true);
+          auto const dep = vt.time(s2, false);
           auto const arr_fp = arr + d;
           if (arr_fp <= dep) {
             auto const pen = penalty(d, dep - arr_fp, a, b);
-            if (pen < best) {  // lanes visit their pairs in increasing order
+            if (pen < best) {  // threads visit their pairs in increasing order
               best = pen;
               best_idx = x;
               best_fp = fp;
@@ -722,43 +814,48 @@ struct recon_ctx {
           break;
         }
       }
-      // (penalty, pair index) minimum over the warp
+      // (penalty, pair index) minimum over the group
       auto win_pen = best;
       auto win_idx = best_idx;
-      for (auto o = 16; o > 0; o >>= 1) {
-        auto const op = __shfl_xor_sync(kFull, win_pen, o);
-        auto const oi = __shfl_xor_sync(kFull, win_idx, o);
+      auto const take = [&](double op, uint32_t oi) {
         if (op < win_pen || (op == win_pen && oi < win_idx)) {
           win_pen = op;
           win_idx = oi;
         }
+      };
+      for (auto o = 16; o > 0; o >>= 1) {
+        take(__shfl_xor_sync(kFull, win_pen, o), __shfl_xor_sync(kFull, win_idx, o));
       }
-      if (win_idx == 0xFFFFFFFFu) continue;  // no pair below the initial penalty
-      auto const owner = static_cast<int>(win_idx % 32u);
-      auto const w_fp = __shfl_sync(kFull, best_fp, owner);
-      auto const w_arr = __shfl_sync(kFull, best_arr, owner);
-      auto const w_dep = __shfl_sync(kFull, best_dep, owner);
-      auto const w_d = __shfl_sync(kFull, best_d, owner);
-      if (lane == 0) {
+      if constexpr (NW > 1) {
+        if (lane == 0u) {
+          sm->pen[wid] = win_pen;
+          sm->pen_at[wid] = win_idx;
+        }
+        sync();
+        for (auto w = 0; w != NW; ++w) take(sm->pen[w], sm->pen_at[w]);
+      } else {
+        sync();  // the legs are read by all before they change
+      }
+      if (win_idx != 0xFFFFFFFFu && win_idx % kT == tid) {  // a pair below the initial penalty
         auto const sf = from_start + win_idx / to_end, s2 = win_idx % to_end;
-        auto const a = loc_at(lf, sf), b = loc_at(lt, s2);
+        auto const a = B2R_STOP_LOC(vf.word(sf)), b = B2R_STOP_LOC(vt.word(s2));
         auto& wf = legs[i];
         auto& wp = legs[i + 1];
         auto& wt = legs[i + 2];
         wf.to = a;
-        wf.arr_time = w_arr;
+        wf.arr_time = best_arr;
         wf.stop_to = static_cast<uint16_t>(sf + 1u);
         wt.from = b;
-        wt.dep_time = w_dep;
+        wt.dep_time = best_dep;
         wt.stop_from = static_cast<uint16_t>(s2);
         wp.from = a;
         wp.to = b;
-        wp.dep_time = w_arr;
-        wp.arr_time = w_arr + w_d;
-        set_fp(wp, B2R_FP_TARGET(w_fp), static_cast<int>(B2R_FP_DURATION(w_fp)));
+        wp.dep_time = best_arr;
+        wp.arr_time = best_arr + best_d;
+        set_fp(wp, B2R_FP_TARGET(best_fp), static_cast<int>(B2R_FP_DURATION(best_fp)));
       }
     }
-    __syncwarp();
+    sync();
   }
 
   // reconstruct.cc:792-877 + optimize_footpaths(journey_q)
@@ -784,14 +881,15 @@ struct recon_ctx {
       else if (has) push(init);
     }
     if (failed) return;
-    if (lane == 0) {
+    sync();
+    if (wid == 0u) {
       if (fwd) {
-        for (auto a = 0, b = n_legs - 1; a < b; ++a, --b) {
+        for (auto a = static_cast<int>(lane); a < n_legs / 2; a += 32) {
           auto const x = legs[a];
-          legs[a] = legs[b];
-          legs[b] = x;
+          legs[a] = legs[n_legs - 1 - a];
+          legs[n_legs - 1 - a] = x;
         }
-      } else {
+      } else if (lane == 0u) {
         for (auto i = 1; i < n_legs; ++i) {
           if (legs[i].kind != B2R_LEG_FOOTPATH) continue;
           auto const diff = legs[i].dep_time - legs[i - 1].arr_time;
@@ -799,15 +897,15 @@ struct recon_ctx {
           legs[i].arr_time -= diff;
         }
       }
+      __syncwarp();
       // optimize_footpaths on the journey query (flipped for backward search)
-      auto const* jq_start = fwd ? start_offs() : dest_offs();
-      auto const n_jq_start = fwd ? sl->n_soff : sl->n_doff;
-      auto const* jq_dest = fwd ? dest_offs() : start_offs();
-      auto const n_jq_dest = fwd ? sl->n_doff : sl->n_soff;
-      opt_initial_departure(jq_start, n_jq_start);
-      opt_initial_start_footpath();
-      opt_last_arrival(jq_dest, n_jq_dest);
-      opt_final_egress_footpath();
+      opt_offset(fwd ? start_offs() : dest_offs(), fwd ? sl->n_soff : sl->n_doff, true);
+      __syncwarp();
+      opt_footpath(true);
+      __syncwarp();
+      opt_offset(fwd ? dest_offs() : start_offs(), fwd ? sl->n_doff : sl->n_soff, false);
+      __syncwarp();
+      opt_footpath(false);
     }
     opt_transfers();
   }
