@@ -646,9 +646,11 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
     ev_b = e.prof_ev[e.prof_used++];
     B2R_CUDA(cudaEventRecord(ev_a, s));
   }
-  dev::k_route_scan_seq<<<list_blocks, 256, 0, s>>>(st);
+  if (e.tt->n_unordered != 0U) dev::k_route_scan_seq<<<list_blocks, 256, 0, s>>>(st);
   {
-    auto const grid = e.sms * e.shape.scan_blocks_per_sm, block = e.shape.scan_threads;
+    auto const block = e.shape.scan_threads;
+    auto const grid = blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, block / dev::kTile,
+                                 static_cast<uint64_t>(e.sms) * e.shape.scan_blocks_per_sm);
     if (e.cfg.profile == 1U) {
       dev::k_route_scan<4, true><<<grid, block, 0, s>>>(st);
     } else if (e.shape.scan_occupancy == 2U) {
@@ -674,7 +676,7 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
   dev::k_end<<<e.G, 1024, 0, s>>>(st, false);
 }
 uint64_t launches_per_step(b2r_engine const& e, bool recon) {
-  return 7U + (recon ? 1U : 0U) + (e.st.tt.n_rt != 0U ? 1U : 0U);
+  return 6U + (recon ? 1U : 0U) + (e.st.tt.n_rt != 0U ? 1U : 0U) + (e.tt->n_unordered != 0U ? 1U : 0U);
 }
 
 // a super-step as its graph (recon: the one with the reconstruction branch)
@@ -2521,6 +2523,18 @@ int b2r_timetable_upload(const b2r_timetable_desc* d, int device, b2r_timetable*
       dd.route_fifo = up(fifo.data(), nr);
       dd.route_filter = up(rfilter.data(), nr);
       dd.route_sec = up(rsec.data(), rsec.size());
+      t->routes.resize(nr);
+      for (auto r = 0U; r != nr; ++r) {
+        auto const t0 = d->route_transport_from[r], n_t = d->route_transport_to[r] - t0;
+        auto flags = static_cast<uint32_t>(fifo[r]) | (sorted[r] != 0U ? b2r::dev::kRouteSorted : 0U);
+        auto one = true;
+        for (auto x = 0U; x != n_t && one; ++x) one = d->transport_traffic_days[t0 + x] == d->route_traffic_days[r];
+        if (one) flags |= b2r::dev::kRouteOneDays;
+        t->routes[r] = {d->route_stop_index[r], d->route_stop_index[r + 1] - d->route_stop_index[r],
+                        d->route_stop_time_from[r], t0, n_t, d->route_traffic_days[r], flags, rfilter[r]};
+        t->n_unordered += fifo[r] == 0U ? 1U : 0U;
+      }
+      dd.routes = up(t->routes.data(), nr);
       dd.lbg_fwd_idx = up(d->lb_fwd_index, nl + 1);
       dd.lbg_fwd = up(d->lb_fwd, d->lb_fwd_index[nl]);
       dd.lbg_bwd_idx = up(d->lb_bwd_index, nl + 1);
@@ -2607,7 +2621,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
                               (sizeof(b2r::dev::journey_rec) + b2r::dev::kMaxLegs * sizeof(b2r_leg)) +
                           e->max_starts * sizeof(b2r::dev::start_rec) +
                           e->max_dest * sizeof(b2r::dev::dest_rec) + e->max_off * sizeof(b2r_offset) +
-                          2U * b2r::dev::kMaxTimeline * sizeof(b2r::dev::tl_entry) +
+                          b2r::dev::kMaxTimeline * sizeof(b2r::dev::tl_entry) +
                           (static_cast<uint64_t>(nl) * (4 + b2r::dev::kK) + tt->d.n_routes) / 8 + 256;
       auto by_budget = cfg.hbm_budget / std::max<uint64_t>(1, e->bytes_per_slot);
       auto slots = std::min<uint64_t>(std::max(32U, cfg.max_slots), by_budget);
@@ -3501,6 +3515,9 @@ int b2r_rt_upload(b2r_timetable* tt, const b2r_rt_desc* desc, b2r_rt** out) {
       bf.insert(bf.end(), h.changed_days.begin(), h.changed_days.end());
       for (auto i = 0U; i != h.changed_transport.size(); ++i) tbf[h.changed_transport[i]] = n_bf + i;
       d.transport_bf = up(tbf.data(), tbf.size());
+      auto routes = tt->routes;  // a changed transport no longer runs on its route's days
+      for (auto const x : h.changed_transport) routes[tt->transport_route[x]].flags &= ~b2r::dev::kRouteOneDays;
+      d.routes = up(routes.data(), routes.size());
       d.bf = up(bf.data(), bf.size());
       auto const n_rt = h.d.n_rt_transports;
       d.n_rt = n_rt;

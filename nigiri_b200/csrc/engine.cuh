@@ -42,6 +42,22 @@ enum : uint8_t {
 };
 
 // ------------------------------------------------------- timetable image
+// what a scan of a route needs before its stops and events, in two 16-byte
+// loads (the same values as the arrays of dtt)
+struct __align__(16) route_rec {
+  uint32_t sb;      // route_stop_idx
+  uint32_t n;       // stops
+  uint32_t st;      // route_st_from
+  uint32_t t0;      // route_tr_from
+  uint32_t n_t;     // transports
+  uint32_t bf;      // route_bf
+  uint32_t flags;   // kRoute*
+  uint32_t filter;  // route_filter
+};
+// flags: bits 0-1 route_fifo, route_sorted, and whether every transport's
+// traffic days are the route's
+constexpr uint32_t kRouteOrder = 3u, kRouteSorted = 4u, kRouteOneDays = 8u;
+
 struct dtt {
   uint32_t n_loc, n_routes, n_transports, n_groups_unused;
   int32_t internal_from_days;
@@ -79,6 +95,7 @@ struct dtt {
   // do (columns ordered by minute, every first departure on its service day,
   // fewer than 16384 transports)
   uint8_t const* route_fifo;
+  route_rec const* routes;
   // lower-bound graphs (build_lb_graph.h), packed footpath words
   uint32_t const* lbg_fwd_idx;
   uint32_t const* lbg_fwd;
@@ -249,7 +266,7 @@ struct state {
   uint32_t* rtlist; // frontier list of (rt transport * G + g)
   uint32_t* D;      // is-destination bits [n_loc][G]
   uint32_t* ylist;  // frontier lists of (loc * G + g)
-  uint32_t* rlist;
+  uint4* rlist;     // {route, group, its marks, 0}
   uint32_t* counters;  // C_*: list lengths, mark parity, error bits
   uint32_t* run_mask;  // [G]
   uint32_t* sweep_mask;  // [G]
@@ -314,21 +331,16 @@ __device__ __forceinline__ bool bf_test(dtt const& T, uint32_t bf, uint32_t i) {
 // required flag is on none of its sections; `sec` receives the required
 // flags that are on some but not all sections, which the walk along the
 // route checks section by section (raptor.h:1194-1217).
-__device__ __forceinline__ bool route_allowed(dtt const& T, uint32_t r, uint32_t claszes, uint32_t req,
-                                              uint32_t& sec) {
-  auto const f = static_cast<uint32_t>(T.route_filter[r]);
+// f: the filter word (rt transports have one of the same layout, with the
+// class of the first section, raptor.h:583-588).
+__device__ __forceinline__ bool filter_allowed(uint32_t f, uint32_t claszes, uint32_t req, uint32_t& sec) {
   auto const need = req & ~(f >> 4);  // required, not on all sections
   sec = need;
   return ((claszes >> (f & 15u)) & 1u) != 0u && (need & ~(f >> 8) & 15u) == 0u;
 }
-
-// the same for a filter word of that layout (rt transports: the class of
-// the first section, raptor.h:583-588)
-__device__ __forceinline__ bool filter_allowed(uint16_t fw, uint32_t claszes, uint32_t req, uint32_t& sec) {
-  auto const f = static_cast<uint32_t>(fw);
-  auto const need = req & ~(f >> 4);
-  sec = need;
-  return ((claszes >> (f & 15u)) & 1u) != 0u && (need & ~(f >> 8) & 15u) == 0u;
+__device__ __forceinline__ bool route_allowed(dtt const& T, uint32_t r, uint32_t claszes, uint32_t req,
+                                              uint32_t& sec) {
+  return filter_allowed(static_cast<uint32_t>(T.route_filter[r]), claszes, req, sec);
 }
 
 // whether section s of route r (from its stop s to s + 1) carries every

@@ -276,12 +276,13 @@ __global__ void k_mark(state st) {
   sweep(st, lane, warp, n_warps);
 }
 
-// The indices of the non-zero words of W[0, n) appended to `list` (in no
-// particular order).  Each thread reads 4 words with one 16-byte load
-// (W comes from cudaMalloc and i is a multiple of 4), the block scans the
-// counts and reserves its range with one atomicAdd per 4 * blockDim words.
-__device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W, uint32_t n,
-                                             uint32_t* list, uint32_t counter) {
+// The non-zero words of W[0, n) listed in no particular order: emit(at, i,
+// word).  Each thread reads 4 words with one 16-byte load (W comes from
+// cudaMalloc and i is a multiple of 4), the block scans the counts and
+// reserves its range with one atomicAdd per 4 * blockDim words.
+template <typename Emit>
+__device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W, uint32_t n, uint32_t counter,
+                                             Emit&& emit) {
   __shared__ uint32_t warp_off[32];
   __shared__ uint32_t base;
   auto const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
@@ -320,7 +321,7 @@ __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W,
     __syncthreads();
     auto at = base + warp_off[warp] + (incl - cnt);
     for (auto j = 0u; j != 4u; ++j) {
-      if (w[j] != 0u) list[at++] = i + j;
+      if (w[j] != 0u) emit(at++, i + j, w[j]);
     }
     __syncthreads();  // warp_off and base are reused by the next pass
   }
@@ -366,8 +367,13 @@ __global__ void k_routes(state st) {
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
   if (blockIdx.x == 0u && threadIdx.x == 0u) st.counters[C_PAR] ^= 1u;
   for (auto s = warp; s < st.S; s += n_warps) dest_slot(st, s, lane);
-  list_nonzero(st, st.R, st.tt.n_routes * st.G, st.rlist, C_R);
-  if (st.tt.n_rt != 0u) list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, st.rtlist, C_RT);
+  list_nonzero(st, st.R, st.tt.n_routes * st.G, C_R, [&](uint32_t at, uint32_t e, uint32_t marks) {
+    st.rlist[at] = uint4{e / st.G, e % st.G, marks, 0u};
+    st.R[e] = 0u;
+  });
+  if (st.tt.n_rt != 0u) {
+    list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, C_RT, [&](uint32_t at, uint32_t e, uint32_t) { st.rtlist[at] = e; });
+  }
 }
 
 // ------------------------------------------------------------ route scan
@@ -382,20 +388,29 @@ __global__ void k_routes(state st) {
 // one (route, query) pair is a chain of dependent loads as long as the
 // route.
 //
-// Here a warp takes one pair and its lanes take the stops, 32 at a time:
-// * every boardable stop looks up its own earliest trip at once (the
-//   lookup depends only on that stop's labels);
+// Here 8 lanes take one pair, a warp four pairs, 32 stops at a time:
+// * the lanes read the stops' marks, four stops each, and the marked
+//   boardable ones are numbered;
+// * the i-th lane looks up the earliest trip of the i-th marked stop (the
+//   lookup depends only on that stop's labels), so that the searches of
+//   four pairs run side by side whatever stops they start from;
 // * on a route whose trips keep one order at every event
 //   (b2r_timetable: route_fifo), "switch when at least as good at this
 //   stop" is "keep the best trip so far, the later stop on ties", whatever
-//   stop compares them, so a warp prefix-minimum over the lanes gives the
+//   stop compares them, so a prefix minimum over the candidates gives the
 //   trip each stop is reached by;
 // * every stop then reads its arrival event of that trip.
-// The result equals the sequential walk's; routes without that order and
-// queries with per-section filters take the sequential walk
-// (k_route_scan_seq).
+// A section that lacks a flag the query requires drops the trip carried
+// into it (raptor.h:1194-1217): the minimum starts anew there.
+// The result equals the sequential walk's; routes without that order take
+// the sequential walk (k_route_scan_seq).
 // Labels are combined with atomicMin and marks with atomicOr, so the order
 // of the pairs does not matter.
+//
+// The kernel is bound by instruction issue and the dependent loads of the
+// trip searches.  With a warp per pair (lanes over 32 stops) a pair cost
+// about 890 warp instructions, most of them in searches that two or three
+// lanes ran while the others waited.
 
 struct scan_ctr {
   uint32_t stops, ev, days, writes, warp_steps;
@@ -427,18 +442,26 @@ __device__ __forceinline__ void scan_arrive(state const& st, lane_t const& ln, u
   }
 }
 
+// The filters of a (route, query) pair: false if the route is filtered
+// out; sec receives the flags checked per section (bits 0-3) and bit 8 for
+// the wheelchair profile's stop bits.
+__device__ __forceinline__ bool scan_filters(uint32_t filter, lane_t const& ln, uint32_t& sec) {
+  sec = 0u;
+  if ((ln.claszes != 0xFFFFu || ln.req != 0u) && !filter_allowed(filter, ln.claszes, ln.req, sec)) return false;
+  if ((ln.mode & 0x70u) == (B2R_PROFILE_WHEELCHAIR << 4)) sec |= 0x100u;
+  return true;
+}
+
 // The reference's sequential walk of one (route, query) pair.
-__device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X, lane_t const& ln, uint32_t r,
+__device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X, lane_t const& ln, route_rec const& R,
                                               uint32_t g, uint32_t b, uint32_t sec, scan_ctr& pc) {
   auto const& T = st.tt;
   auto const s = g * 32u + b;
   auto const bit = 1u << b;
   auto const fwd = ln.fwd != 0;
   auto const k = static_cast<uint32_t>(ln.k);
-  auto const sb = T.route_stop_idx[r];
-  auto const n = T.route_stop_idx[r + 1] - sb;
-  auto const n_t = T.route_tr_to[r] - T.route_tr_from[r];
-  auto const* colbase = T.st + T.route_st_from[r];
+  auto const sb = R.sb, n = R.n, n_t = R.n_t;
+  auto const* colbase = T.st + R.st;
   auto const lb_off = (ln.mode & 8u) != 0u;
   bool et_valid = false;
   uint32_t et_off = 0;
@@ -471,7 +494,7 @@ __device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X
     auto const minutes = static_cast<int>(ln.base) * 1440 + from_key(fwd, prt);
     uint32_t nt = 0;
     uint16_t nd = 0;
-    if (!et_search(T, fwd, r, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440, static_cast<int>(lbv),
+    if (!et_search(T, fwd, R, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440, static_cast<int>(lbv),
                    ln.tad_k, ln.base, nt, nd, pc.ev, pc.days)) {
       continue;
     }
@@ -487,36 +510,25 @@ __device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X
   }
 }
 
-// The filters of a (route, query) pair: false if the route is filtered
-// out; sec receives the flags checked per section (bits 0-3) and bit 8 for
-// the wheelchair profile's stop bits.
-__device__ __forceinline__ bool scan_filters(dtt const& T, lane_t const& ln, uint32_t r, uint32_t& sec) {
-  sec = 0u;
-  if ((ln.claszes != 0xFFFFu || ln.req != 0u) && !route_allowed(T, r, ln.claszes, ln.req, sec)) return false;
-  if ((ln.mode & 0x70u) == (B2R_PROFILE_WHEELCHAIR << 4)) sec |= 0x100u;
-  return true;
-}
-
 // The pairs the parallel scan leaves to the sequential walk: routes without
-// one trip order at every event, queries with per-section filters.  A
-// thread per marked (route, group) entry, before k_route_scan (which clears
-// the route marks).
+// one trip order at every event (launched only if the timetable has any).
+// A thread per marked (route, group) entry.
 __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ state st) {
   auto const& T = st.tt;
   auto const nr = st.counters[C_R];
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
   scan_ctr pc{0u, 0u, 0u, 0u, 0u};
   for (auto w = blockIdx.x * blockDim.x + threadIdx.x; w < nr; w += gridDim.x * blockDim.x) {
-    auto const e = st.rlist[w];
-    auto const g = e % st.G, r = e / st.G;
-    auto const fifo = __ldg(T.route_fifo + r) != 0u;
-    for (auto mask = st.R[e]; mask != 0u; mask &= mask - 1u) {
+    auto const en = st.rlist[w];
+    auto const R = load_route(T, en.x);
+    if ((R.flags & kRouteOrder) != 0u) continue;  // k_route_scan's
+    auto const g = en.y;
+    for (auto mask = en.z; mask != 0u; mask &= mask - 1u) {
       auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
       auto const ln = st.lanes[g * 32u + b];
       uint32_t sec = 0u;
-      if (!ln.run || !scan_filters(T, ln, r, sec)) continue;
-      if ((sec & 15u) == 0u && fifo) continue;  // k_route_scan's
-      scan_walk_seq(st, X, ln, r, g, b, sec, pc);
+      if (!ln.run || !scan_filters(R.filter, ln, sec)) continue;
+      scan_walk_seq(st, X, ln, R, g, b, sec, pc);
     }
   }
   if (st.profile && (pc.stops | pc.ev | pc.days | pc.writes) != 0u) {
@@ -528,156 +540,225 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
   }
 }
 
-// One (route, query) pair, the warp's lanes over its stops.  Prof: count
-// the work for the roofline (profiling engines only).
-template <bool Prof>
-__device__ __forceinline__ void scan_pair(state const& st, uint32_t const* X, lane_t const& ln, uint32_t r, uint32_t g,
-                                          uint32_t b, uint32_t lane, scan_ctr& pc) {
+// the parallel scan (above).  Builds with four, five or six blocks of 256
+// threads resident per SM (the launch shape picks one), and with work
+// counters for profiling engines (Prof).  Every loop that shuffles or
+// ballots is uniform over the warp; a tile without work takes part idle.
+constexpr uint32_t kTile = 8;
+template <int MinBlocks, bool Prof>
+__global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
+  constexpr uint32_t kPer = 32u / kTile;  // stops a lane takes of each 32; pairs of a warp
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
   auto const& T = st.tt;
-  auto const s = g * 32u + b;
-  uint32_t sec = 0u;
-  if (!scan_filters(T, ln, r, sec)) return;
-  auto const order = static_cast<uint32_t>(__ldg(T.route_fifo + r));
-  if ((sec & 15u) != 0u || order == 0u) return;  // k_route_scan_seq's
-  auto const bit = 1u << b;
-  auto const fwd = ln.fwd != 0;
-  auto const k = static_cast<uint32_t>(ln.k);
-  auto const sb = __ldg(T.route_stop_idx + r);
-  auto const n = __ldg(T.route_stop_idx + r + 1) - sb;
-  auto const n_t = __ldg(T.route_tr_to + r) - __ldg(T.route_tr_from + r);
-  auto const* colbase = T.st + __ldg(T.route_st_from + r);
-  auto const lb_off = (ln.mode & 8u) != 0u;
+  auto const lane = threadIdx.x & 31u;
+  auto const tl = lane % kTile, tb = lane - tl;  // lane of the tile, its first lane
+  auto const n_tiles = (gridDim.x * blockDim.x) / kTile;
+  auto const nr = st.counters[C_R];
+  auto const* X = st.X[st.counters[C_PAR] ^ 1u];
+  auto const tile_bits = [&](bool x) { return (__ballot_sync(kFull, x) >> tb) & ((1u << kTile) - 1u); };
+  auto const tile_shfl = [&](uint32_t x, uint32_t src) {
+    return __shfl_sync(kFull, x, static_cast<int>(src), static_cast<int>(kTile));
+  };
+  scan_ctr pc{0u, 0u, 0u, 0u, 0u};
+  // the tile's entry and pair
+  auto w = (blockIdx.x * blockDim.x + threadIdx.x) / kTile;
+  uint32_t g = 0, mask = 0, s = 0, sec = 0, i0 = 0;
+  route_rec R{};
+  lane_t ln{};
+  bool have = false;
   // The trips' order key, below 2^21, smaller is better: with route_fifo
   // bit 1 (service day - base + 64) * n_t + transport offset (the service
   // day lies within 64 days of the base day, n_t < 2^14), else the time at
   // the route's first departure event (|t| < 2^20 minutes) + 2^20; both
   // mirrored backward, where later is better.
-  // The trip carried over from the earlier chunks: key, offset, day.
+  // The trip carried over from the earlier stops: key, offset, day.
   bool c_valid = false;
-  uint32_t c_key = 0;
-  uint32_t c_off = 0;
-  uint16_t c_day = 0;
-  for (auto i0 = 0u; i0 < n; i0 += 32u) {
-    auto const i = i0 + lane;
-    auto const act = i < n;
-    auto const si = fwd ? i : n - 1u - i;
-    uint32_t stp = 0, l = 0;
-    bool marked = false;
-    uint16_t lbv = 0;
-    if (act) {
-      stp = scan_stop_word(T, sb, n, fwd, i, sec);
-      l = B2R_STOP_LOC(stp);
-      marked = (X[l * st.G + g] & bit) != 0u;
-      if (!lb_off) lbv = st.lb[li(st, l, s)];
+  uint32_t c_key = 0, c_off = 0, c_day = 0;
+  while (true) {
+    while (!have) {
+      if (mask == 0u) {
+        if (w >= nr) break;
+        auto const en = st.rlist[w];
+        w += n_tiles;
+        g = en.y;
+        R = load_route(T, en.x);
+        mask = (R.flags & kRouteOrder) != 0u ? en.z : 0u;  // else k_route_scan_seq's
+        continue;
+      }
+      auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
+      mask &= mask - 1u;
+      s = g * 32u + b;
+      ln = st.lanes[s];
+      if (!ln.run || !scan_filters(R.filter, ln, sec)) continue;
+      have = true;
+      i0 = 0u;
+      c_valid = false;
     }
-    auto const can_finish = act && (fwd ? B2R_STOP_OUT(stp) : B2R_STOP_IN(stp)) != 0u;
-    auto const boardable = act && i + 1u != n && (fwd ? B2R_STOP_IN(stp) : B2R_STOP_OUT(stp)) != 0u && marked;
-    // raptor.h:1309-1311: the walk ends at the first boardable stop the
-    // query cannot reach, after that stop's arrival
-    auto const brk = __ballot_sync(kFull, boardable && lbv == 0xFFFFu);
-    auto const fb = brk != 0u ? static_cast<uint32_t>(__ffs(brk) - 1) : 32u;
-    // this stop's earliest boardable trip (raptor.h:1313-1327)
-    bool cand = false, cb_bad = false;
-    uint32_t nt = 0;
-    uint16_t nd = 0;
-    uint32_t key = 0;
-    if (boardable && lane < fb) {
-      auto const prt = dec(st.rt[rti(st, k - 1u, l, s)], ln.qtag);
-      if (prt != kKeyInv) {
+    if (!__any_sync(kFull, have)) break;
+    auto const fwd = ln.fwd != 0;
+    auto const bit = 1u << (s & 31u);
+    auto const lb_off = (ln.mode & 8u) != 0u;
+    auto const n_blk = have ? min(32u, R.n - i0) : 0u;
+    // the block's stop words; its marked boardable stops (m) and the stops
+    // entered through a section that drops the trip (cuts)
+    uint32_t sw[kPer];
+    uint32_t m = 0, cuts = 0;
+#pragma unroll
+    for (auto c = 0u; c != kPer; ++c) {
+      auto const p = c * kTile + tl;
+      sw[c] = p < n_blk ? scan_stop_word(T, R.sb, R.n, fwd, i0 + p, sec) : 0u;
+    }
+#pragma unroll
+    for (auto c = 0u; c != kPer; ++c) {
+      auto const p = c * kTile + tl;
+      auto const board = p < n_blk && i0 + p + 1u != R.n && (fwd ? B2R_STOP_IN(sw[c]) : B2R_STOP_OUT(sw[c])) != 0u;
+      m |= tile_bits(board && (X[B2R_STOP_LOC(sw[c]) * st.G + g] & bit) != 0u) << (c * kTile);
+    }
+    if (__any_sync(kFull, have && (sec & 15u) != 0u)) {
+#pragma unroll
+      for (auto c = 0u; c != kPer; ++c) {
+        auto const i = i0 + c * kTile + tl;
+        auto const check = c * kTile + tl < n_blk && (sec & 15u) != 0u && i != 0u;
+        cuts |= tile_bits(check && !section_ok(T, R.sb, fwd ? i - 1u : R.n - 1u - i, sec & 15u)) << (c * kTile);
+      }
+    }
+    if constexpr (Prof) {
+      if (lane == 0u) ++pc.warp_steps;
+      if (tl == 0u) pc.stops += n_blk;
+    }
+    // segments of the block: up to kTile marked stops, up to the next cut
+    uint32_t lo = 0;
+    bool ends = false;
+    auto todo = have && (m != 0u || c_valid);
+    while (__any_sync(kFull, todo)) {
+      // a marked stop before lo (the last segment's end) is searched before
+      // a cut at lo drops what was carried
+      auto const pending = lo < 32u ? m & ((1u << lo) - 1u) : m;
+      auto const from = pending != 0u ? lo : lo + 1u;
+      if (todo && lo < 32u && pending == 0u && ((cuts >> lo) & 1u) != 0u) c_valid = false;
+      auto const later = from < 32u ? cuts >> from << from : 0u;
+      auto const cut = later != 0u ? static_cast<uint32_t>(__ffs(later) - 1) : 32u;
+      auto const sm = cut < 32u ? m & ((1u << cut) - 1u) : m;  // marked stops before the cut
+      auto rest = sm;  // without the first kTile of them
+#pragma unroll
+      for (auto x = 0u; x != kTile; ++x) rest &= rest - 1u;
+      auto const seg = todo ? sm & ~rest : 0u;
+      auto hi = (rest != 0u ? static_cast<uint32_t>(__ffs(rest)) : min(cut, n_blk)) - 1u;  // last stop reached
+      // this lane's marked stop and its earliest trip (raptor.h:1313-1327)
+      auto sel = seg;
+      for (auto x = tl; x != 0u; --x) sel &= sel - 1u;
+      auto const pos = sel != 0u ? static_cast<uint32_t>(__ffs(sel) - 1) : 0u;
+      auto const si = fwd ? i0 + pos : R.n - 1u - (i0 + pos);
+      uint32_t nt = 0, key = 0;
+      uint16_t nd = 0;
+      bool cand = false, stop_here = false;
+      uint32_t l = 0;
+      uint16_t lbv = 0;
+      int prt = kKeyInv;
+      if (sel != 0u) {
+        l = B2R_STOP_LOC(__ldg(T.route_stops + R.sb + si));
+        if (!lb_off) lbv = st.lb[li(st, l, s)];
+        prt = dec(st.rt[rti(st, ln.k - 1u, l, s)], ln.qtag);
+        // raptor.h:1309-1311: the walk ends at the first boardable stop the
+        // query cannot reach, after that stop's arrival
+        stop_here = lbv == 0xFFFFu;
+      }
+      if (sel != 0u && !stop_here && prt != kKeyInv) {
         auto const minutes = static_cast<int>(ln.base) * 1440 + from_key(fwd, prt);
         uint32_t n_ev = 0, n_days = 0;
-        auto const found = et_search(T, fwd, r, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440,
-                                     static_cast<int>(lbv), ln.tad_k, ln.base, nt, nd, n_ev, n_days);
+        cand = et_search(T, fwd, R, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440, static_cast<int>(lbv),
+                         ln.tad_k, ln.base, nt, nd, n_ev, n_days);
         if constexpr (Prof) {
           pc.ev += n_ev;
           pc.days += n_days;
         }
-        if (found) {
-          cand = true;
-          cb_bad = dec(st.best[li(st, l, s)], ln.gtag) == kKeyInv && dec(st.tmp[li(st, l, s)], ln.gtag) == kKeyInv;
-          if ((order & 2u) != 0u) {
-            auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(ln.base) + 64) * n_t + nt;
+        if (cand) {
+          // a marked station always carries a best label of its start time
+          // (marks come with best updates), so the boarding rule never meets
+          // an invalid current_best; were it to, the query is failed loudly
+          if (dec(st.best[li(st, l, s)], ln.gtag) == kKeyInv && dec(st.tmp[li(st, l, s)], ln.gtag) == kKeyInv) {
+            atomicOr(&st.counters[C_ERR], 4u);
+          }
+          if ((R.flags & 2u) != 0u) {
+            auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(ln.base) + 64) * R.n_t + nt;
             key = fwd ? x : (1u << 21) - 1u - x;
           } else {
-            auto const t = (static_cast<int>(nd) - static_cast<int>(ln.base)) * 1440 + delta_count(__ldg(colbase + nt));
+            auto const t =
+                (static_cast<int>(nd) - static_cast<int>(ln.base)) * 1440 + delta_count(__ldg(T.st + R.st + nt));
             key = static_cast<uint32_t>((fwd ? t : -t) + (1 << 20));
           }
         }
       }
-    }
-    // a marked station always carries a best label of its start time
-    // (marks come with best updates), so the boarding rule never meets an
-    // invalid current_best; were it to, the query is failed loudly
-    if (cb_bad) atomicOr(&st.counters[C_ERR], 4u);
-    if constexpr (Prof) {
-      if (lane == 0u) {
-        pc.stops += min(n - i0, min(fb + 1u, 32u));
-        ++pc.warp_steps;
+      auto const fb = tile_bits(stop_here);
+      auto const f = fb != 0u ? static_cast<uint32_t>(__ffs(fb) - 1) : 0u;
+      auto const f_pos = tile_shfl(pos, f);
+      if (fb != 0u) {
+        ends = true;
+        hi = f_pos;
+        if (tl >= f) cand = false;
       }
-    }
-    // prefix minimum of (key, later stop first) over the lanes: the key's
-    // 21 bits above 5 for the lane
-    auto v = cand ? (key << 5) | (31u - lane) : 0xFFFFFFFFu;
-    for (auto o = 1u; o < 32u; o <<= 1) {
-      auto const y = __shfl_up_sync(kFull, v, o);
-      if (lane >= o) v = min(v, y);
-    }
-    auto ex = __shfl_up_sync(kFull, v, 1);  // best candidate before this stop
-    if (lane == 0u) ex = 0xFFFFFFFFu;
-    auto const tot = __shfl_sync(kFull, v, 31);
-    auto const src = static_cast<int>(31u - (ex & 31u));
-    auto const x_off = __shfl_sync(kFull, nt, src);
-    auto const x_day = static_cast<uint16_t>(__shfl_sync(kFull, static_cast<uint32_t>(nd), src));
-    // the carried trip loses ties to the later stops of this chunk
-    auto const use_x = ex != 0xFFFFFFFFu && (!c_valid || (ex >> 5) <= c_key);
-    auto const et_valid = use_x || c_valid;
-    if (act && lane <= fb && et_valid && can_finish) {
-      auto const et_off = use_x ? x_off : c_off;
-      auto const et_day = use_x ? x_day : c_day;
-      auto const ev = __ldg(colbase + n_t * (si * 2u - (fwd ? 1u : 0u)) + et_off);
-      scan_arrive<Prof>(st, ln, s, g, bit, l, lbv, to_delta_key(fwd, et_day, ln.base, delta_count(ev)), pc);
-    }
-    if (fb != 32u) return;
-    if (tot != 0xFFFFFFFFu) {
-      auto const t_src = static_cast<int>(31u - (tot & 31u));
-      auto const t_off = __shfl_sync(kFull, nt, t_src);
-      auto const t_day = static_cast<uint16_t>(__shfl_sync(kFull, static_cast<uint32_t>(nd), t_src));
-      auto const t_key = tot >> 5;
-      if (!c_valid || t_key <= c_key) {
+      // prefix minimum of (key, later stop first) over the candidates
+      auto v = cand ? (key << 3) | (kTile - 1u - tl) : kNone;
+#pragma unroll
+      for (auto o = 1u; o < kTile; o <<= 1) {
+        auto const y = __shfl_up_sync(kFull, v, o, kTile);
+        if (tl >= o) v = min(v, y);
+      }
+      // arrivals (raptor.h:1219-1302): stop p by the best candidate before it
+      if constexpr (Prof) {
+        if (fb != 0u && tl == 0u) pc.stops -= n_blk - (hi + 1u);  // not scanned
+      }
+      uint32_t off[kPer];
+      uint16_t ev[kPer], lbs[kPer], day[kPer];
+      bool go[kPer];
+#pragma unroll
+      for (auto c = 0u; c != kPer; ++c) {
+        auto const p = c * kTile + tl;
+        auto const before = static_cast<uint32_t>(__popc(seg & ((1u << p) - 1u)));
+        auto const best = tile_shfl(v, (before - 1u) & (kTile - 1u));
+        auto const ex = before != 0u ? best : kNone;
+        auto const src = (kTile - 1u) - (ex & (kTile - 1u));
+        auto const x_off = tile_shfl(nt, src);
+        auto const x_day = tile_shfl(nd, src);
+        // the carried trip loses ties to the later stops of this segment
+        auto const use_x = ex != kNone && (!c_valid || (ex >> 3) <= c_key);
+        go[c] = todo && p >= lo && p <= hi && (use_x || c_valid) &&
+                (fwd ? B2R_STOP_OUT(sw[c]) : B2R_STOP_IN(sw[c])) != 0u;
+        off[c] = use_x ? x_off : c_off;
+        day[c] = static_cast<uint16_t>(use_x ? x_day : c_day);
+        ev[c] = lbs[c] = 0;
+        if (go[c]) {
+          auto const i = i0 + p;
+          auto const at = fwd ? 2u * i - 1u : 2u * (R.n - 1u - i);
+          ev[c] = __ldg(T.st + R.st + R.n_t * at + off[c]);
+          if (!lb_off) lbs[c] = st.lb[li(st, B2R_STOP_LOC(sw[c]), s)];
+        }
+      }
+#pragma unroll
+      for (auto c = 0u; c != kPer; ++c) {
+        if (!go[c]) continue;
+        scan_arrive<Prof>(st, ln, s, g, bit, B2R_STOP_LOC(sw[c]), lbs[c],
+                          to_delta_key(fwd, day[c], ln.base, delta_count(ev[c])), pc);
+      }
+      // the segment's best trip is carried on
+      auto const tot = tile_shfl(v, kTile - 1u);
+      auto const t_src = (kTile - 1u) - (tot & (kTile - 1u));
+      auto const t_off = tile_shfl(nt, t_src);
+      auto const t_day = tile_shfl(nd, t_src);
+      if (tot != kNone && (!c_valid || (tot >> 3) <= c_key)) {
         c_valid = true;
-        c_key = t_key;
+        c_key = tot >> 3;
         c_off = t_off;
         c_day = t_day;
       }
+      m &= ~seg;
+      lo = hi + 1u;
+      // the last mark may lie on the last stop: it is searched, for the next block
+      todo = todo && !ends && (m != 0u || (c_valid && lo < n_blk));
     }
-  }
-}
-
-// A warp per marked (route, group of 32 queries) entry, one pair of the
-// entry after the other.  Builds with four, five or six blocks of 256
-// threads resident per SM (the launch shape picks one), and with work
-// counters for profiling engines.
-template <int MinBlocks, bool Prof>
-__global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
-  auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
-  auto const nr = st.counters[C_R];
-  auto const* X = st.X[st.counters[C_PAR] ^ 1u];
-  scan_ctr pc{0u, 0u, 0u, 0u, 0u};
-  for (auto w = warp; w < nr; w += n_warps) {
-    auto const e = st.rlist[w];
-    auto mask = st.R[e];
-    __syncwarp();
-    if (lane == 0u) st.R[e] = 0u;
-    auto const g = e % st.G, r = e / st.G;
-    while (mask != 0u) {
-      auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
-      mask &= mask - 1u;
-      auto const ln = st.lanes[g * 32u + b];
-      if (!ln.run) continue;
-      scan_pair<Prof>(st, X, ln, r, g, b, lane, pc);
-      __syncwarp();
+    if (have) {
+      i0 += 32u;
+      if (ends || i0 >= R.n) have = false;
     }
   }
   if constexpr (Prof) {  // work counters for the roofline (warp-reduced)
@@ -698,61 +779,86 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
     }
   }
 }
-// update_rt_transport, raptor.h:1068-1175 (no vias), a lane per marked
-// (rt transport, query) pair walking the run in search direction: et is
-// whether the query rides the run when it passes the stop.  The filters are
-// loop_rt_routes' (raptor.h:583-626): the class of the first section and
-// the route flags, section by section where set on some sections only.
-__global__ void k_rt_scan(state st) {
+
+// update_rt_transport, raptor.h:1068-1175 (no vias), a warp per marked
+// (rt transport, query) pair, the lanes over the run's stops: et is whether
+// the query rides the run when it passes the stop, i.e. whether it could
+// board at an earlier stop with no section in between that lacks a required
+// flag.  The walk ends at the first stop the query cannot reach, boardable
+// or not (raptor.h:1156-1158).  The filters are loop_rt_routes'
+// (raptor.h:583-626): the class of the first section and the route flags,
+// section by section where set on some sections only.
+// A lane per pair walked the run one stop at a time, four dependent loads
+// each.
+__global__ void __launch_bounds__(256) k_rt_scan(const __grid_constant__ state st) {
   auto const& T = st.tt;
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
-  for_each_pair(
-      st.rtlist, st.counters[C_RT],
-      [&](uint32_t e) {
-        auto const m = st.RT_R[e];
-        st.RT_R[e] = 0u;
-        return m;
-      },
-      [&](uint32_t e, uint32_t b) {
-        auto const g = e % st.G, x = e / st.G;
-        auto const s = g * 32u + b;
-        auto const ln = st.lanes[s];
-        if (!ln.run) return;
-        uint32_t sec = 0u;
-        if ((ln.claszes != 0xFFFFu || ln.req != 0u) && !filter_allowed(T.rt_filter[x], ln.claszes, ln.req, sec)) {
-          return;
+  auto const lane = threadIdx.x & 31u;
+  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+  auto const n_list = st.counters[C_RT];
+  scan_ctr pc{};
+  for (auto w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_list; w += n_warps) {
+    auto const e = st.rtlist[w];
+    auto mask = st.RT_R[e];
+    __syncwarp();
+    if (lane == 0u) st.RT_R[e] = 0u;
+    auto const g = e % st.G, x = e / st.G;
+    auto const sb = T.rt_stop_idx[x];
+    auto const n = T.rt_stop_idx[x + 1] - sb;
+    auto const* tm = T.rt_times + 2ull * (sb - x);
+    for (; mask != 0u; mask &= mask - 1u) {
+      auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
+      auto const s = g * 32u + b;
+      auto const ln = st.lanes[s];
+      uint32_t sec = 0u;
+      if (!ln.run || !scan_filters(T.rt_filter[x], ln, sec)) continue;
+      auto const bit = 1u << b;
+      auto const fwd = ln.fwd != 0;
+      auto const base_min = (T.internal_from_days + static_cast<int32_t>(ln.base)) * 1440;
+      auto const lb_off = (ln.mode & 8u) != 0u;
+      bool carried = false;  // riding into the chunk
+      for (auto i0 = 0u; i0 < n; i0 += 32u) {
+        auto const i = i0 + lane;
+        auto const act = i < n;
+        auto const si = fwd ? i : n - 1u - i;
+        uint32_t sw = 0, l = 0;
+        uint16_t lbv = 0;
+        bool cut = false, marked = false;
+        if (act) {
+          sw = T.rt_stops[sb + si];
+          if ((sec & 0x100u) != 0u) sw = (sw & 0xCFFFFFFFu) | ((sw >> 2) & 0x30000000u);
+          l = B2R_STOP_LOC(sw);
+          if (!lb_off) lbv = st.lb[li(st, l, s)];
+          marked = (X[l * st.G + g] & bit) != 0u;
+          cut = (sec & 15u) != 0u && i != 0u &&
+                (static_cast<uint32_t>(T.rt_sec[sb + (fwd ? si - 1u : si)]) & (sec & 15u)) != (sec & 15u);
         }
-        if ((ln.mode & 0x70u) == (B2R_PROFILE_WHEELCHAIR << 4)) sec |= 0x100u;
-        auto const bit = 1u << b;
-        auto const fwd = ln.fwd != 0;
-        auto const k = static_cast<uint32_t>(ln.k);
-        auto const sb = T.rt_stop_idx[x];
-        auto const n = T.rt_stop_idx[x + 1] - sb;
-        auto const* tm = T.rt_times + 2ull * (sb - x);
-        auto const base_min = (T.internal_from_days + static_cast<int32_t>(ln.base)) * 1440;
-        auto const lb_off = (ln.mode & 8u) != 0u;
-        scan_ctr pc{};
-        bool et = false;
-        for (auto i = 0u; i != n; ++i) {
-          auto const si = fwd ? i : n - 1u - i;
-          auto w = T.rt_stops[sb + si];
-          if ((sec & 0x100u) != 0u) w = (w & 0xCFFFFFFFu) | ((w >> 2) & 0x30000000u);
-          auto const l = B2R_STOP_LOC(w);
-          if ((sec & 15u) != 0u && i != 0u &&
-              (static_cast<uint32_t>(T.rt_sec[sb + (fwd ? si - 1u : si)]) & (sec & 15u)) != (sec & 15u)) {
-            et = false;
-          }
-          auto const lbv = lb_off ? uint16_t{0} : st.lb[li(st, l, s)];
-          if (et && (fwd ? si != 0u : si + 1u != n) && (fwd ? B2R_STOP_OUT(w) : B2R_STOP_IN(w))) {
-            auto const by = to_key(fwd, clamp16(tm[2u * si - (fwd ? 1u : 0u)] - base_min));
-            scan_arrive<false>(st, ln, s, g, bit, l, lbv, by, pc);
-          }
-          if (lbv == 0xFFFFu) break;  // raptor.h:1156-1158: before the boarding test
-          if (i + 1u == n || !(fwd ? B2R_STOP_IN(w) : B2R_STOP_OUT(w)) || !(X[l * st.G + g] & bit)) continue;
-          auto const by = to_key(fwd, clamp16(tm[2u * si - (fwd ? 0u : 1u)] - base_min));
-          if (dec(st.rt[rti(st, k - 1u, l, s)], ln.qtag) <= by) et = true;
+        auto const closed = __ballot_sync(kFull, act && lbv == 0xFFFFu);
+        auto const end = closed != 0u ? static_cast<uint32_t>(__ffs(closed) - 1) : 32u;
+        auto board = act && lane < end && i + 1u != n && marked && (fwd ? B2R_STOP_IN(sw) : B2R_STOP_OUT(sw)) != 0u;
+        if (board) {
+          auto const dep = to_key(fwd, clamp16(tm[2u * si - (fwd ? 0u : 1u)] - base_min));
+          board = dec(st.rt[rti(st, ln.k - 1u, l, s)], ln.qtag) <= dep;
         }
-      });
+        auto const boards = __ballot_sync(kFull, board), cuts = __ballot_sync(kFull, cut);
+        if (!carried && boards == 0u) {
+          if (end != 32u) break;
+          continue;
+        }
+        auto const cut_to = cuts & ((2u << lane) - 1u);  // cuts up to this stop (lane 31: all)
+        auto const from = cut_to != 0u ? 31u - static_cast<uint32_t>(__clz(cut_to)) : 0u;
+        auto const et = ((boards & ((1u << lane) - 1u)) >> from) != 0u || (carried && cut_to == 0u);
+        if (et && act && lane < end && (fwd ? si != 0u : si + 1u != n) &&
+            (fwd ? B2R_STOP_OUT(sw) : B2R_STOP_IN(sw)) != 0u) {
+          auto const by = to_key(fwd, clamp16(tm[2u * si - (fwd ? 1u : 0u)] - base_min));
+          scan_arrive<false>(st, ln, s, g, bit, l, lbv, by, pc);
+        }
+        if (end != 32u) break;
+        carried = (boards >> (cuts != 0u ? 31u - static_cast<uint32_t>(__clz(cuts)) : 0u)) != 0u ||
+                  (carried && cuts == 0u);
+      }
+    }
+  }
 }
 
 // ------------------------------------- stations reached, destination passes
@@ -958,7 +1064,7 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
       for (auto j = i; j < n; ++j) X[j] = 0u;
     }
   }
-  list_nonzero(st, st.Y, n, st.ylist, C_Y);
+  list_nonzero(st, st.Y, n, C_Y, [&](uint32_t at, uint32_t e, uint32_t) { st.ylist[at] = e; });
 }
 
 // ------------------------------------------------ transfers and footpaths

@@ -272,7 +272,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
             auto const mam = minutes % 1440;
             uint32_t nt = 0;
             uint16_t nd = 0;
-            if (dev::et_search(T, fwd, r, si, day, mam, 0, tad, P.base, nt, nd, n_ev, n_days)) {
+            if (dev::et_search(T, fwd, dev::load_route(T, r), si, day, mam, 0, tad, P.base, nt, nd, n_ev, n_days)) {
               // current_best (raptor.h:1328-1329) is valid whenever the
               // arrival part ran or the station carries a label
               auto const cb_valid = arrival_ran || ldk(&best[l]) != kInv || ldk(&tmp[l]) != kInv;

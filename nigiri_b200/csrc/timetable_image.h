@@ -33,6 +33,8 @@ struct b2r_timetable {
     std::vector<uint32_t> lists[8];
   };
   profile_copy profiles[B2R_N_PROFILES - 1];
+  std::vector<b2r::dev::route_rec> routes;  // host copy (an overlay changes flags)
+  uint32_t n_unordered{0};                  // routes whose trips keep no one order (k_route_scan_seq)
   b2r::host_view view{};
   // all-pairs lower-bound tables [source][location] (u16 minutes, 0xFFFF
   // unreachable) for forward and backward searches, built by the first
