@@ -389,16 +389,17 @@ __global__ void k_routes(state st) {
 // route.
 //
 // Here 8 lanes take one pair, a warp four pairs, 32 stops at a time:
-// * the lanes read the stops' marks, four stops each, and the marked
-//   boardable ones are numbered;
-// * the i-th lane looks up the earliest trip of the i-th marked stop (the
-//   lookup depends only on that stop's labels), so that the searches of
-//   four pairs run side by side whatever stops they start from;
+// * the lanes read the stops' marks, four stops each, and for the marked
+//   boardable ones the label to board from; those that time_at_dest does
+//   not rule out are the searches;
+// * the searches of the four pairs are numbered through and the warp's
+//   lanes take 32 of them at once (a search depends only on its stop's
+//   labels; what it needs of its pair lies in shared memory);
 // * on a route whose trips keep one order at every event
 //   (b2r_timetable: route_fifo), "switch when at least as good at this
-//   stop" is "keep the best trip so far, the later stop on ties", whatever
-//   stop compares them, so a prefix minimum over the candidates gives the
-//   trip each stop is reached by;
+//   stop" is "keep the best trip so far", whatever stop compares them (on a
+//   tie both are the same trip or equal at every event), so a prefix
+//   minimum over the stops gives the trip each stop is reached by;
 // * every stop then reads its arrival event of that trip.
 // A section that lacks a flag the query requires drops the trip carried
 // into it (raptor.h:1194-1217): the minimum starts anew there.
@@ -407,10 +408,11 @@ __global__ void k_routes(state st) {
 // Labels are combined with atomicMin and marks with atomicOr, so the order
 // of the pairs does not matter.
 //
-// The kernel is bound by instruction issue and the dependent loads of the
-// trip searches.  With a warp per pair (lanes over 32 stops) a pair cost
-// about 890 warp instructions, most of them in searches that two or three
-// lanes ran while the others waited.
+// The kernel is bound by instruction issue, and the trip searches are most
+// of it.  With a warp per pair a pair cost about 890 warp instructions, its
+// searches running on the few lanes whose stops were marked; on the
+// regional batch of 1,024 a warp's four pairs bring 24 searches per 32
+// stops, so numbering them fills the lanes.
 
 struct scan_ctr {
   uint32_t stops, ev, days, writes, warp_steps;
@@ -540,22 +542,46 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
   }
 }
 
+// position of the n-th (from 0) set bit of m
+__device__ __forceinline__ uint32_t nth_bit(uint32_t m, uint32_t n) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (auto w = 16u; w != 0u; w >>= 1) {
+    auto const c = static_cast<uint32_t>(__popc(m & ((1u << w) - 1u)));
+    if (n >= c) {
+      n -= c;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
+}
+
 // the parallel scan (above).  Builds with four, five or six blocks of 256
 // threads resident per SM (the launch shape picks one), and with work
 // counters for profiling engines (Prof).  Every loop that shuffles or
 // ballots is uniform over the warp; a tile without work takes part idle.
-constexpr uint32_t kTile = 8;
+constexpr uint32_t kTile = 8;            // lanes of a pair
+constexpr uint32_t kPer = 32u / kTile;   // stops a lane takes of each 32; pairs of a warp
+struct scan_smem {                       // of a warp
+  uint4 pair[kPer][4];      // route record (2), lane record, {first stop of the 32, 0, 0, 0}
+  uint32_t key[kPer][32];   // per stop: what its search needs (previous label, bound), then the
+                            // candidate (order key << 6 | stop), kNone without one
+  uint2 trip[kPer][33];     // per stop: the candidate's offset and day; 32: the trip carried in
+};
 template <int MinBlocks, bool Prof>
 __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
-  constexpr uint32_t kPer = 32u / kTile;  // stops a lane takes of each 32; pairs of a warp
   constexpr uint32_t kNone = 0xFFFFFFFFu;
+  constexpr uint32_t kCarried = 32u;
+  __shared__ scan_smem smem[8];
   auto const& T = st.tt;
   auto const lane = threadIdx.x & 31u;
-  auto const tl = lane % kTile, tb = lane - tl;  // lane of the tile, its first lane
+  auto const tile = lane / kTile, tl = lane % kTile;
+  auto& sm = smem[threadIdx.x >> 5];
   auto const n_tiles = (gridDim.x * blockDim.x) / kTile;
   auto const nr = st.counters[C_R];
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
-  auto const tile_bits = [&](bool x) { return (__ballot_sync(kFull, x) >> tb) & ((1u << kTile) - 1u); };
+  auto const tile_bits = [&](bool x) { return (__ballot_sync(kFull, x) >> (tile * kTile)) & ((1u << kTile) - 1u); };
   auto const tile_shfl = [&](uint32_t x, uint32_t src) {
     return __shfl_sync(kFull, x, static_cast<int>(src), static_cast<int>(kTile));
   };
@@ -571,9 +597,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
   // day lies within 64 days of the base day, n_t < 2^14), else the time at
   // the route's first departure event (|t| < 2^20 minutes) + 2^20; both
   // mirrored backward, where later is better.
-  // The trip carried over from the earlier stops: key, offset, day.
-  bool c_valid = false;
-  uint32_t c_key = 0, c_off = 0, c_day = 0;
+  uint32_t carry = kNone;  // the trip carried over from the earlier stops: key << 6 | kCarried
   while (true) {
     while (!have) {
       if (mask == 0u) {
@@ -592,17 +616,16 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       if (!ln.run || !scan_filters(R.filter, ln, sec)) continue;
       have = true;
       i0 = 0u;
-      c_valid = false;
+      carry = kNone;
     }
     if (!__any_sync(kFull, have)) break;
     auto const fwd = ln.fwd != 0;
     auto const bit = 1u << (s & 31u);
     auto const lb_off = (ln.mode & 8u) != 0u;
     auto const n_blk = have ? min(32u, R.n - i0) : 0u;
-    // the block's stop words; its marked boardable stops (m) and the stops
-    // entered through a section that drops the trip (cuts)
+    // the block's stop words, marks and boarding labels
     uint32_t sw[kPer];
-    uint32_t m = 0, cuts = 0;
+    bool marked[kPer];
 #pragma unroll
     for (auto c = 0u; c != kPer; ++c) {
       auto const p = c * kTile + tl;
@@ -611,126 +634,134 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
 #pragma unroll
     for (auto c = 0u; c != kPer; ++c) {
       auto const p = c * kTile + tl;
-      auto const board = p < n_blk && i0 + p + 1u != R.n && (fwd ? B2R_STOP_IN(sw[c]) : B2R_STOP_OUT(sw[c])) != 0u;
-      m |= tile_bits(board && (X[B2R_STOP_LOC(sw[c]) * st.G + g] & bit) != 0u) << (c * kTile);
+      marked[c] = p < n_blk && i0 + p + 1u != R.n && (fwd ? B2R_STOP_IN(sw[c]) : B2R_STOP_OUT(sw[c])) != 0u &&
+                  (X[B2R_STOP_LOC(sw[c]) * st.G + g] & bit) != 0u;
     }
-    if (__any_sync(kFull, have && (sec & 15u) != 0u)) {
+    uint32_t m = 0, closed = 0, cuts = 0;
 #pragma unroll
-      for (auto c = 0u; c != kPer; ++c) {
-        auto const i = i0 + c * kTile + tl;
-        auto const check = c * kTile + tl < n_blk && (sec & 15u) != 0u && i != 0u;
-        cuts |= tile_bits(check && !section_ok(T, R.sb, fwd ? i - 1u : R.n - 1u - i, sec & 15u)) << (c * kTile);
+    for (auto c = 0u; c != kPer; ++c) {
+      uint32_t label = kNone;
+      bool shut = false;
+      if (marked[c]) {
+        auto const at = li(st, B2R_STOP_LOC(sw[c]), s);
+        auto const lbv = lb_off ? uint16_t{0} : st.lb[at];
+        auto const prt = dec(st.rt[static_cast<size_t>(ln.k - 1u) * T.n_loc * st.S + at], ln.qtag);
+        // a marked station always carries a best label of its start time
+        // (marks come with best updates), so the boarding rule never meets
+        // an invalid current_best; were it to, the query is failed loudly
+        if (prt != kKeyInv && dec(st.best[at], ln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
+        shut = lbv == 0xFFFFu;
+        // every event of the search is at or after prt: pruned with it
+        if (!shut && prt != kKeyInv && prt + static_cast<int>(lbv) <= ln.tad_k) {
+          label = (static_cast<uint32_t>(static_cast<uint16_t>(prt)) << 16) | lbv;
+        }
       }
+      sm.key[tile][c * kTile + tl] = label;
+      m |= tile_bits(label != kNone) << (c * kTile);
+      closed |= tile_bits(shut) << (c * kTile);
     }
+    // raptor.h:1309-1311: the walk ends at the first boardable stop the
+    // query cannot reach, after that stop's arrival
+    auto const ends = closed != 0u;
+    auto const first_closed = static_cast<uint32_t>(__ffs(closed) - 1);
+    if (ends) m &= (1u << first_closed) - 1u;
+    auto const limit = ends ? first_closed + 1u : n_blk;
     if constexpr (Prof) {
       if (lane == 0u) ++pc.warp_steps;
-      if (tl == 0u) pc.stops += n_blk;
+      if (tl == 0u) pc.stops += limit;
     }
-    // segments of the block: up to kTile marked stops, up to the next cut
-    uint32_t lo = 0;
-    bool ends = false;
-    auto todo = have && (m != 0u || c_valid);
-    while (__any_sync(kFull, todo)) {
-      // a marked stop before lo (the last segment's end) is searched before
-      // a cut at lo drops what was carried
-      auto const pending = lo < 32u ? m & ((1u << lo) - 1u) : m;
-      auto const from = pending != 0u ? lo : lo + 1u;
-      if (todo && lo < 32u && pending == 0u && ((cuts >> lo) & 1u) != 0u) c_valid = false;
-      auto const later = from < 32u ? cuts >> from << from : 0u;
-      auto const cut = later != 0u ? static_cast<uint32_t>(__ffs(later) - 1) : 32u;
-      auto const sm = cut < 32u ? m & ((1u << cut) - 1u) : m;  // marked stops before the cut
-      auto rest = sm;  // without the first kTile of them
+    if (__any_sync(kFull, m != 0u || carry != kNone)) {
+      if (__any_sync(kFull, have && (sec & 15u) != 0u)) {
 #pragma unroll
-      for (auto x = 0u; x != kTile; ++x) rest &= rest - 1u;
-      auto const seg = todo ? sm & ~rest : 0u;
-      auto hi = (rest != 0u ? static_cast<uint32_t>(__ffs(rest)) : min(cut, n_blk)) - 1u;  // last stop reached
-      // this lane's marked stop and its earliest trip (raptor.h:1313-1327)
-      auto sel = seg;
-      for (auto x = tl; x != 0u; --x) sel &= sel - 1u;
-      auto const pos = sel != 0u ? static_cast<uint32_t>(__ffs(sel) - 1) : 0u;
-      auto const si = fwd ? i0 + pos : R.n - 1u - (i0 + pos);
-      uint32_t nt = 0, key = 0;
-      uint16_t nd = 0;
-      bool cand = false, stop_here = false;
-      uint32_t l = 0;
-      uint16_t lbv = 0;
-      int prt = kKeyInv;
-      if (sel != 0u) {
-        l = B2R_STOP_LOC(__ldg(T.route_stops + R.sb + si));
-        if (!lb_off) lbv = st.lb[li(st, l, s)];
-        prt = dec(st.rt[rti(st, ln.k - 1u, l, s)], ln.qtag);
-        // raptor.h:1309-1311: the walk ends at the first boardable stop the
-        // query cannot reach, after that stop's arrival
-        stop_here = lbv == 0xFFFFu;
-      }
-      if (sel != 0u && !stop_here && prt != kKeyInv) {
-        auto const minutes = static_cast<int>(ln.base) * 1440 + from_key(fwd, prt);
-        uint32_t n_ev = 0, n_days = 0;
-        cand = et_search(T, fwd, R, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440, static_cast<int>(lbv),
-                         ln.tad_k, ln.base, nt, nd, n_ev, n_days);
-        if constexpr (Prof) {
-          pc.ev += n_ev;
-          pc.days += n_days;
+        for (auto c = 0u; c != kPer; ++c) {
+          auto const i = i0 + c * kTile + tl;
+          auto const check = c * kTile + tl < n_blk && (sec & 15u) != 0u && i != 0u;
+          cuts |= tile_bits(check && !section_ok(T, R.sb, fwd ? i - 1u : R.n - 1u - i, sec & 15u)) << (c * kTile);
         }
-        if (cand) {
-          // a marked station always carries a best label of its start time
-          // (marks come with best updates), so the boarding rule never meets
-          // an invalid current_best; were it to, the query is failed loudly
-          if (dec(st.best[li(st, l, s)], ln.gtag) == kKeyInv && dec(st.tmp[li(st, l, s)], ln.gtag) == kKeyInv) {
-            atomicOr(&st.counters[C_ERR], 4u);
+      }
+      // the searches (raptor.h:1313-1327), 32 at a time over the warp's pairs
+      if (tl == 0u && m != 0u) {
+        sm.pair[tile][0] = uint4{R.sb, R.n, R.st, R.t0};
+        sm.pair[tile][1] = uint4{R.n_t, R.bf, R.flags, R.filter};
+        sm.pair[tile][2] = *reinterpret_cast<uint4 const*>(&ln);
+        sm.pair[tile][3] = uint4{i0, 0u, 0u, 0u};
+      }
+      __syncwarp();
+      auto const cnt = static_cast<uint32_t>(__popc(m));
+      auto const e1 = __shfl_sync(kFull, cnt, 0);
+      auto const e2 = e1 + __shfl_sync(kFull, cnt, kTile);
+      auto const e3 = e2 + __shfl_sync(kFull, cnt, 2 * kTile);
+      auto const total = e3 + __shfl_sync(kFull, cnt, 3 * kTile);
+      for (auto q0 = 0u; q0 < total; q0 += 32u) {
+        auto const q = q0 + lane;
+        auto const o = (q >= e1 ? 1u : 0u) + (q >= e2 ? 1u : 0u) + (q >= e3 ? 1u : 0u);
+        auto const om = __shfl_sync(kFull, m, static_cast<int>(o * kTile));
+        if (q < total) {
+          auto const pos = nth_bit(om, q - (o == 0u ? 0u : o == 1u ? e1 : o == 2u ? e2 : e3));
+          auto const a = sm.pair[o][0], b = sm.pair[o][1], c = sm.pair[o][2];
+          route_rec const oR{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          auto const oln = *reinterpret_cast<lane_t const*>(&c);
+          auto const ofwd = oln.fwd != 0;
+          auto const i = sm.pair[o][3].x + pos;
+          auto const label = sm.key[o][pos];
+          auto const prt = static_cast<int>(static_cast<int16_t>(label >> 16));
+          auto const minutes = static_cast<int>(oln.base) * 1440 + from_key(ofwd, prt);
+          uint32_t nt = 0, v = kNone, n_ev = 0, n_days = 0;
+          uint16_t nd = 0;
+          if (et_search(T, ofwd, oR, ofwd ? i : oR.n - 1u - i, static_cast<uint16_t>(minutes / 1440), minutes % 1440,
+                        static_cast<int>(label & 0xFFFFu), oln.tad_k, oln.base, nt, nd, n_ev, n_days)) {
+            uint32_t key;
+            if ((oR.flags & 2u) != 0u) {
+              auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(oln.base) + 64) * oR.n_t + nt;
+              key = ofwd ? x : (1u << 21) - 1u - x;
+            } else {
+              auto const t =
+                  (static_cast<int>(nd) - static_cast<int>(oln.base)) * 1440 + delta_count(__ldg(T.st + oR.st + nt));
+              key = static_cast<uint32_t>((ofwd ? t : -t) + (1 << 20));
+            }
+            v = (key << 6) | pos;
+            sm.trip[o][pos] = uint2{nt, nd};
           }
-          if ((R.flags & 2u) != 0u) {
-            auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(ln.base) + 64) * R.n_t + nt;
-            key = fwd ? x : (1u << 21) - 1u - x;
-          } else {
-            auto const t =
-                (static_cast<int>(nd) - static_cast<int>(ln.base)) * 1440 + delta_count(__ldg(T.st + R.st + nt));
-            key = static_cast<uint32_t>((fwd ? t : -t) + (1 << 20));
+          sm.key[o][pos] = v;
+          if constexpr (Prof) {
+            pc.ev += n_ev;
+            pc.days += n_days;
           }
         }
       }
-      auto const fb = tile_bits(stop_here);
-      auto const f = fb != 0u ? static_cast<uint32_t>(__ffs(fb) - 1) : 0u;
-      auto const f_pos = tile_shfl(pos, f);
-      if (fb != 0u) {
-        ends = true;
-        hi = f_pos;
-        if (tl >= f) cand = false;
-      }
-      // prefix minimum of (key, later stop first) over the candidates
-      auto v = cand ? (key << 3) | (kTile - 1u - tl) : kNone;
+      __syncwarp();
+      // the trip each stop is reached by: the minimum over the stops before
+      // it, from the last cut on
+      uint32_t by[kPer];
+      auto run = carry;
 #pragma unroll
-      for (auto o = 1u; o < kTile; o <<= 1) {
-        auto const y = __shfl_up_sync(kFull, v, o, kTile);
-        if (tl >= o) v = min(v, y);
+      for (auto c = 0u; c != kPer; ++c) {
+        auto const cc = (cuts >> (c * kTile)) & ((1u << kTile) - 1u);
+        auto v = ((m >> (c * kTile + tl)) & 1u) != 0u ? sm.key[tile][c * kTile + tl] : kNone;
+#pragma unroll
+        for (auto o = 1u; o < kTile; o <<= 1) {
+          auto const y = __shfl_up_sync(kFull, v, o, kTile);
+          if (tl >= o && ((cc >> (tl + 1u - o)) & ((1u << o) - 1u)) == 0u) v = min(v, y);
+        }
+        auto const up = __shfl_up_sync(kFull, v, 1, kTile);
+        auto const before = tl == 0u || ((cc >> tl) & 1u) != 0u ? kNone : up;
+        by[c] = (cc & ((2u << tl) - 1u)) == 0u ? min(before, run) : before;
+        auto const last = tile_shfl(v, kTile - 1u);
+        run = cc == 0u ? min(run, last) : last;
       }
-      // arrivals (raptor.h:1219-1302): stop p by the best candidate before it
-      if constexpr (Prof) {
-        if (fb != 0u && tl == 0u) pc.stops -= n_blk - (hi + 1u);  // not scanned
-      }
-      uint32_t off[kPer];
+      // arrivals (raptor.h:1219-1302)
       uint16_t ev[kPer], lbs[kPer], day[kPer];
       bool go[kPer];
 #pragma unroll
       for (auto c = 0u; c != kPer; ++c) {
         auto const p = c * kTile + tl;
-        auto const before = static_cast<uint32_t>(__popc(seg & ((1u << p) - 1u)));
-        auto const best = tile_shfl(v, (before - 1u) & (kTile - 1u));
-        auto const ex = before != 0u ? best : kNone;
-        auto const src = (kTile - 1u) - (ex & (kTile - 1u));
-        auto const x_off = tile_shfl(nt, src);
-        auto const x_day = tile_shfl(nd, src);
-        // the carried trip loses ties to the later stops of this segment
-        auto const use_x = ex != kNone && (!c_valid || (ex >> 3) <= c_key);
-        go[c] = todo && p >= lo && p <= hi && (use_x || c_valid) &&
-                (fwd ? B2R_STOP_OUT(sw[c]) : B2R_STOP_IN(sw[c])) != 0u;
-        off[c] = use_x ? x_off : c_off;
-        day[c] = static_cast<uint16_t>(use_x ? x_day : c_day);
-        ev[c] = lbs[c] = 0;
+        go[c] = p < limit && by[c] != kNone && (fwd ? B2R_STOP_OUT(sw[c]) : B2R_STOP_IN(sw[c])) != 0u;
+        ev[c] = lbs[c] = day[c] = 0;
         if (go[c]) {
+          auto const t = sm.trip[tile][by[c] & 63u];
           auto const i = i0 + p;
-          auto const at = fwd ? 2u * i - 1u : 2u * (R.n - 1u - i);
-          ev[c] = __ldg(T.st + R.st + R.n_t * at + off[c]);
+          day[c] = static_cast<uint16_t>(t.y);
+          ev[c] = __ldg(T.st + (R.st + R.n_t * (fwd ? 2u * i - 1u : 2u * (R.n - 1u - i)) + t.x));
           if (!lb_off) lbs[c] = st.lb[li(st, B2R_STOP_LOC(sw[c]), s)];
         }
       }
@@ -740,22 +771,14 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
         scan_arrive<Prof>(st, ln, s, g, bit, B2R_STOP_LOC(sw[c]), lbs[c],
                           to_delta_key(fwd, day[c], ln.base, delta_count(ev[c])), pc);
       }
-      // the segment's best trip is carried on
-      auto const tot = tile_shfl(v, kTile - 1u);
-      auto const t_src = (kTile - 1u) - (tot & (kTile - 1u));
-      auto const t_off = tile_shfl(nt, t_src);
-      auto const t_day = tile_shfl(nd, t_src);
-      if (tot != kNone && (!c_valid || (tot >> 3) <= c_key)) {
-        c_valid = true;
-        c_key = tot >> 3;
-        c_off = t_off;
-        c_day = t_day;
+      __syncwarp();  // the trips are read before the one carried on is put aside
+      if (run != kNone && (run & 63u) != kCarried) {
+        if (tl == 0u) sm.trip[tile][kCarried] = sm.trip[tile][run & 63u];
+        run = (run & ~63u) | kCarried;
       }
-      m &= ~seg;
-      lo = hi + 1u;
-      // the last mark may lie on the last stop: it is searched, for the next block
-      todo = todo && !ends && (m != 0u || (c_valid && lo < n_blk));
+      carry = run;
     }
+    __syncwarp();  // before the next block's labels
     if (have) {
       i0 += 32u;
       if (ends || i0 >= R.n) have = false;
@@ -770,7 +793,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       pc.writes += __shfl_xor_sync(kFull, pc.writes, o);
       pc.warp_steps += __shfl_xor_sync(kFull, pc.warp_steps, o);
     }
-    if (lane == 0) {
+    if (lane == 0 && pc.warp_steps != 0u) {
       atomicAdd(&st.prof[0], static_cast<unsigned long long>(pc.stops));
       atomicAdd(&st.prof[1], static_cast<unsigned long long>(pc.ev));
       atomicAdd(&st.prof[2], static_cast<unsigned long long>(pc.days));
