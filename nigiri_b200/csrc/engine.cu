@@ -608,12 +608,11 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
   auto const& st = e.st;
   auto const words = static_cast<uint64_t>(st.tt.n_loc) * e.G;
   auto const pair_blocks = static_cast<uint64_t>(e.sms) * e.shape.pair_blocks_per_sm;
-  auto const slot_blocks = static_cast<uint64_t>((e.S + 7U) / 8U);  // a warp per slot
+  auto const slot_blocks = (e.S + 7U) / 8U;  // a warp per slot
   auto const list_blocks = static_cast<uint64_t>(e.sms) * 8U;
   dev::k_mark<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
-  dev::k_routes<<<std::max(blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks),
-                           blocks_for(slot_blocks, 1U, list_blocks)),
-                  256, 0, s>>>(st);
+  dev::k_routes<<<slot_blocks + blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks), 256, 0,
+                  s>>>(st);
   cudaEvent_t rc_a = nullptr, rc_b = nullptr;
   if (recon) {
     auto* s2 = e.stream_recon;
@@ -669,8 +668,7 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
     if (idx < b2r_engine::kProfRows) k_prof_row<<<1, 1, 0, s>>>(st, e.d_prof_rows, idx);
   }
   if (st.tt.n_rt != 0U) dev::k_rt_scan<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_reached<<<std::max(blocks_for(words, 1024U, list_blocks), blocks_for(slot_blocks, 1U, list_blocks)), 256, 0,
-                   s>>>(st);
+  dev::k_reached<<<slot_blocks + blocks_for(words, 1024U, list_blocks), 256, 0, s>>>(st);
   dev::k_relax<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
   if (recon) B2R_CUDA(cudaStreamWaitEvent(s, e.ev_join, 0));
   dev::k_end<<<e.G, 1024, 0, s>>>(st, false);
@@ -2660,7 +2658,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.rlist, static_cast<size_t>(tt->d.n_routes) * G);
       al(st.counters, 16);
       al(st.run_mask, G);
-      al(st.sweep_mask, G);
+      al(st.sweep_k, G * b2r::dev::kK);
       al(st.any_mask, G);
       al(st.start_pool, S * e->max_starts);
       al(st.dest_pool, S * e->max_dest);
@@ -2703,7 +2701,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       B2R_CUDA(cudaMemset(st.X[1], 0, static_cast<size_t>(nl) * G * 4));
       B2R_CUDA(cudaMemset(st.lanes, 0, S * sizeof(b2r::dev::lane_t)));
       B2R_CUDA(cudaMemset(st.run_mask, 0, G * 4));
-      B2R_CUDA(cudaMemset(st.sweep_mask, 0, G * 4));
+      B2R_CUDA(cudaMemset(st.sweep_k, 0, G * b2r::dev::kK * 4));
       B2R_CUDA(cudaMemset(st.any_mask, 0, G * 4));
       B2R_CUDA(cudaMemset(st.Y, 0, static_cast<size_t>(nl) * G * 4));
       B2R_CUDA(cudaMemset(st.R, 0, static_cast<size_t>(tt->d.n_routes) * G * 4));

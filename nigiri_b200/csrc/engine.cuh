@@ -269,7 +269,7 @@ struct state {
   uint4* rlist;     // {route, group, its marks, 0}
   uint32_t* counters;  // C_*: list lengths, mark parity, error bits
   uint32_t* run_mask;  // [G]
-  uint32_t* sweep_mask;  // [G]
+  uint32_t* sweep_k;   // [G][K] slots to sweep that are at round k
   uint32_t* any_mask;  // [G]
   start_rec* start_pool;
   dest_rec* dest_pool;

@@ -41,9 +41,25 @@ __device__ __forceinline__ void mark_warp(state const& st, uint32_t* M, uint32_t
   if (want && lane == static_cast<uint32_t>(__ffs(peers) - 1)) mark(st, M, list, counter, e, peers);
 }
 
-// Visits the (entry, query) pairs of a frontier list: a warp takes 32 list
-// entries (a location or route with a group of 32 queries), and its lanes
-// take their set query bits, one pair per lane per pass.  Resident queries
+// position of the n-th (from 0) set bit of m
+__device__ __forceinline__ uint32_t nth_bit(uint32_t m, uint32_t n) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (auto w = 16u; w != 0u; w >>= 1) {
+    auto const c = static_cast<uint32_t>(__popc(m & ((1u << w) - 1u)));
+    if (n >= c) {
+      n -= c;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
+}
+
+// Visits the (entry, query) pairs of a frontier list: a warp takes up to 32
+// list entries (a location or route with a group of 32 queries; 8 when the
+// list is short, to keep more warps busy), and its lanes take their set
+// query bits, one pair per lane per pass.  Resident queries
 // are unrelated, so an entry holds few of its 32 queries; a lane per query of
 // one entry would leave most lanes idle.  word(e) returns the entry's query
 // bits; f(e, b) runs for every set bit b.  f must not synchronise the warp.
@@ -52,10 +68,11 @@ __device__ __forceinline__ void for_each_pair(uint32_t const* list, uint32_t n, 
   auto const lane = threadIdx.x & 31u;
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
-  for (auto w0 = warp * 32u; w0 < n; w0 += n_warps * 32u) {
+  auto const per = n >= n_warps * 8u ? 32u : 8u;
+  for (auto w0 = warp * per; w0 < n; w0 += n_warps * per) {
     auto const w = w0 + lane;
     uint32_t e = 0, mask = 0;
-    if (w < n) {
+    if (lane < per && w < n) {
       e = list[w];
       mask = word(e);
     }
@@ -138,59 +155,75 @@ __device__ __forceinline__ lane_t lane_of(slot_t const& sl) {
 // the (location, slot) pairs, over its lanes: every lane loads one round
 // time and best label, independent of the others.  Bits whose entry belongs
 // to an earlier query of the slot (its tag no longer matches) are cleared
-// here; any later write sets them again.  Slots of one group at different
-// rounds are taken one round at a time.
+// here; any later write sets them again.  The slots of one group that are
+// at the same round (sweep_k) are taken together, and each (group, round)
+// pair gets its share of the warps, so that slots at a dozen different
+// rounds do not queue behind each other.
 __device__ __forceinline__ void sweep(state const& st, uint32_t lane, uint32_t warp, uint32_t n_warps) {
   auto const n_loc = st.tt.n_loc;
   auto const n_chunks = (n_loc + 31u) / 32u;
-  for (auto g = 0u; g != st.G; ++g) {
-    auto const m = st.sweep_mask[g];
-    if (m == 0u) continue;
+  // the (group, round) pairs to sweep: how many, and the warp's
+  auto const n_words = st.G * kK;
+  uint32_t n_pairs = 0;
+  for (auto q0 = 0u; q0 < n_words; q0 += 32u) {
+    auto const w = q0 + lane < n_words ? st.sweep_k[q0 + lane] : 0u;
+    n_pairs += static_cast<uint32_t>(__popc(__ballot_sync(kFull, w != 0u)));
+  }
+  if (n_pairs == 0u) return;
+  auto const per = max(1u, n_warps / n_pairs);  // warps of a pair
+  for (auto pair = warp / per; pair < n_pairs; pair += n_warps / per) {
+    uint32_t same = 0, at_word = 0;
+    for (auto q0 = 0u, seen = 0u; q0 < n_words; q0 += 32u) {
+      auto const w = q0 + lane < n_words ? st.sweep_k[q0 + lane] : 0u;
+      auto const q = __ballot_sync(kFull, w != 0u);
+      auto const c = static_cast<uint32_t>(__popc(q));
+      if (pair < seen + c) {
+        auto const src = nth_bit(q, pair - seen);
+        same = __shfl_sync(kFull, w, static_cast<int>(src));
+        at_word = q0 + src;
+        break;
+      }
+      seen += c;
+    }
+    auto const g = at_word / kK, k = at_word % kK;
+    auto* tw = st.touched + (static_cast<size_t>(k) * st.G + g) * n_loc;
     auto const ln = st.lanes[g * 32u + lane];
-    auto const mine = ((m >> lane) & 1u) != 0u;
-    auto pending = m;
-    while (pending != 0u) {
-      auto const k = __shfl_sync(kFull, static_cast<uint32_t>(ln.k), __ffs(pending) - 1);
-      auto const same = __ballot_sync(kFull, mine && static_cast<uint32_t>(ln.k) == k);
-      pending &= ~same;
-      auto* tw = st.touched + (static_cast<size_t>(k) * st.G + g) * n_loc;
-      for (auto c = warp; c < n_chunks; c += n_warps) {
-        auto const l = c * 32u + lane;
-        auto const word = l < n_loc ? (tw[l] & same) : 0u;
-        if (__ballot_sync(kFull, word != 0u) == 0u) continue;
-        auto const cnt = static_cast<uint32_t>(__popc(word));
-        auto end = cnt;  // inclusive prefix sum of the pair counts
-        for (auto o = 1u; o < 32u; o <<= 1) {
-          auto const y = __shfl_up_sync(kFull, end, o);
-          if (lane >= o) end += y;
+    for (auto c = warp % per; c < n_chunks; c += per) {
+      auto const l = c * 32u + lane;
+      auto const word = l < n_loc ? (tw[l] & same) : 0u;
+      if (__ballot_sync(kFull, word != 0u) == 0u) continue;
+      auto const cnt = static_cast<uint32_t>(__popc(word));
+      auto end = cnt;  // inclusive prefix sum of the pair counts
+      for (auto o = 1u; o < 32u; o <<= 1) {
+        auto const y = __shfl_up_sync(kFull, end, o);
+        if (lane >= o) end += y;
+      }
+      auto const total = __shfl_sync(kFull, end, 31);
+      for (auto p0 = 0u; p0 < total; p0 += 32u) {
+        auto const p = p0 + lane;
+        uint32_t owner = 0;  // first lane whose prefix end exceeds p
+        for (auto b = 16u; b > 0u; b >>= 1) {
+          if (__shfl_sync(kFull, end, static_cast<int>(owner + b - 1u)) <= p) owner += b;
         }
-        auto const total = __shfl_sync(kFull, end, 31);
-        for (auto p0 = 0u; p0 < total; p0 += 32u) {
-          auto const p = p0 + lane;
-          uint32_t owner = 0;  // first lane whose prefix end exceeds p
-          for (auto b = 16u; b > 0u; b >>= 1) {
-            if (__shfl_sync(kFull, end, static_cast<int>(owner + b - 1u)) <= p) owner += b;
-          }
-          auto o_word = __shfl_sync(kFull, word, static_cast<int>(owner));
-          auto const o_first = __shfl_sync(kFull, end, static_cast<int>(owner)) -
-                               __shfl_sync(kFull, cnt, static_cast<int>(owner));
-          uint32_t b = 0u;
-          if (p < total) {
-            for (auto x = p - o_first; x != 0u; --x) o_word &= o_word - 1u;
-            b = static_cast<uint32_t>(__ffs(o_word) - 1);
-          }
-          auto const qtag = __shfl_sync(kFull, static_cast<uint32_t>(ln.qtag), static_cast<int>(b));
-          auto const gtag = __shfl_sync(kFull, static_cast<uint32_t>(ln.gtag), static_cast<int>(b));
-          if (p < total) {
-            auto const at = c * 32u + owner;
-            auto const s = g * 32u + b;
-            auto const r = dec(st.rt[rti(st, k, at, s)], static_cast<uint16_t>(qtag));
-            if (r == kKeyInv) {
-              atomicAnd(tw + at, ~(1u << b));
-            } else {
-              auto& bw = st.best[li(st, at, s)];
-              if (r < dec(bw, static_cast<uint16_t>(gtag))) bw = enc(static_cast<uint16_t>(gtag), r);
-            }
+        auto o_word = __shfl_sync(kFull, word, static_cast<int>(owner));
+        auto const o_first = __shfl_sync(kFull, end, static_cast<int>(owner)) -
+                             __shfl_sync(kFull, cnt, static_cast<int>(owner));
+        uint32_t b = 0u;
+        if (p < total) {
+          for (auto x = p - o_first; x != 0u; --x) o_word &= o_word - 1u;
+          b = static_cast<uint32_t>(__ffs(o_word) - 1);
+        }
+        auto const qtag = __shfl_sync(kFull, static_cast<uint32_t>(ln.qtag), static_cast<int>(b));
+        auto const gtag = __shfl_sync(kFull, static_cast<uint32_t>(ln.gtag), static_cast<int>(b));
+        if (p < total) {
+          auto const at = c * 32u + owner;
+          auto const s = g * 32u + b;
+          auto const r = dec(st.rt[rti(st, k, at, s)], static_cast<uint16_t>(qtag));
+          if (r == kKeyInv) {
+            atomicAnd(tw + at, ~(1u << b));
+          } else {
+            auto& bw = st.best[li(st, at, s)];
+            if (r < dec(bw, static_cast<uint16_t>(gtag))) bw = enc(static_cast<uint16_t>(gtag), r);
           }
         }
       }
@@ -206,6 +239,13 @@ __device__ __forceinline__ void sweep(state const& st, uint32_t lane, uint32_t w
 // stations with many routes do not hold one lane.  Reading the marks where
 // they lie saves a frontier list and its launch: the words of a step are
 // read in full once here and once where they are cleared (k_reached).
+// Where one pass takes all words, a warp's 32 lie n_warps apart: marks
+// cluster (a query's frontier is a few districts), and a warp with 32
+// neighbours of one cluster has 600 routes to mark one pass after the other
+// while most warps have none (17.1 -> 14.5 us at 128 slots on 40,000
+// stops).  With more words every warp has enough to do and neighbours are
+// better: their marks fall on the same routes (31 us at 1,024 slots, 49 us
+// apart).
 // The per-group "any route marked" word is read before its atomicOr: it only
 // gains bits during the kernel, so a read that shows the bits set makes the
 // atomic redundant, and same-address atomics would queue in L2.  A marked
@@ -225,9 +265,9 @@ __global__ void k_mark(state st) {
   }
   auto const n = T.n_loc * st.G;
   auto const step = n_warps * 32u;
-  auto i = warp * 32u + lane;
+  auto i = n <= step ? lane * n_warps + warp : warp * 32u + lane;
   auto x = i < n ? X[i] : 0u;
-  for (auto w0 = warp * 32u; w0 < n; w0 += step) {
+  for (auto w0 = 0u; w0 < n; w0 += step) {
     auto const e = i;
     auto w = x;
     i += step;
@@ -269,7 +309,10 @@ __global__ void k_mark(state st) {
       auto const o_w = __shfl_sync(kFull, w, static_cast<int>(owner));
       if (p < total) {
         auto const r = __ldg(T.loc_routes + o_rb + (p - o_first));
-        atomicOr(&st.R[r * st.G + o_g], o_w);  // listed by k_routes
+        // a corridor's stops mark the same routes over and over: a read that
+        // shows the bits saves the atomic
+        auto* rw = &st.R[r * st.G + o_g];
+        if ((*rw & o_w) != o_w) atomicOr(rw, o_w);  // listed by k_routes
       }
     }
   }
@@ -280,14 +323,15 @@ __global__ void k_mark(state st) {
 // word).  Each thread reads 4 words with one 16-byte load (W comes from
 // cudaMalloc and i is a multiple of 4), the block scans the counts and
 // reserves its range with one atomicAdd per 4 * blockDim words.
+// Block `block` of `n_blocks`.
 template <typename Emit>
 __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W, uint32_t n, uint32_t counter,
-                                             Emit&& emit) {
+                                             uint32_t block, uint32_t n_blocks, Emit&& emit) {
   __shared__ uint32_t warp_off[32];
   __shared__ uint32_t base;
   auto const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
   auto const per_block = blockDim.x * 4u;
-  for (auto b0 = blockIdx.x * per_block; b0 < n; b0 += gridDim.x * per_block) {
+  for (auto b0 = block * per_block; b0 < n; b0 += n_blocks * per_block) {
     auto const i = b0 + threadIdx.x * 4u;
     uint32_t w[4] = {0u, 0u, 0u, 0u};
     if (i + 3u < n) {
@@ -360,19 +404,25 @@ __device__ __forceinline__ void dest_slot(state const& st, uint32_t s, uint32_t 
 // The round's marked (route, group) and (real-time run, group) entries
 // listed, the slots' destination times, and the station-mark arrays swapped:
 // from here to the end of the step X[C_PAR ^ 1] holds the marks the round
-// reads and X[C_PAR] takes the marks it makes.
-__global__ void k_routes(state st) {
+// reads and X[C_PAR] takes the marks it makes.  The first blocks take the
+// slots, 8 each, the others the lists, so that neither waits for the other.
+__global__ void __launch_bounds__(256) k_routes(state st) {
   auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
   if (blockIdx.x == 0u && threadIdx.x == 0u) st.counters[C_PAR] ^= 1u;
-  for (auto s = warp; s < st.S; s += n_warps) dest_slot(st, s, lane);
-  list_nonzero(st, st.R, st.tt.n_routes * st.G, C_R, [&](uint32_t at, uint32_t e, uint32_t marks) {
+  auto const slot_blocks = (st.S + 7u) / 8u;
+  if (blockIdx.x < slot_blocks) {
+    auto const s = blockIdx.x * 8u + (threadIdx.x >> 5);
+    if (s < st.S) dest_slot(st, s, lane);
+    return;
+  }
+  auto const block = blockIdx.x - slot_blocks, n_blocks = gridDim.x - slot_blocks;
+  list_nonzero(st, st.R, st.tt.n_routes * st.G, C_R, block, n_blocks, [&](uint32_t at, uint32_t e, uint32_t marks) {
     st.rlist[at] = uint4{e / st.G, e % st.G, marks, 0u};
     st.R[e] = 0u;
   });
   if (st.tt.n_rt != 0u) {
-    list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, C_RT, [&](uint32_t at, uint32_t e, uint32_t) { st.rtlist[at] = e; });
+    list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, C_RT, block, n_blocks,
+                 [&](uint32_t at, uint32_t e, uint32_t) { st.rtlist[at] = e; });
   }
 }
 
@@ -540,21 +590,6 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
     atomicAdd(&st.prof[3], static_cast<unsigned long long>(pc.writes));
     atomicAdd(&st.prof[5], static_cast<unsigned long long>(pc.warp_steps));
   }
-}
-
-// position of the n-th (from 0) set bit of m
-__device__ __forceinline__ uint32_t nth_bit(uint32_t m, uint32_t n) {
-  uint32_t pos = 0;
-#pragma unroll
-  for (auto w = 16u; w != 0u; w >>= 1) {
-    auto const c = static_cast<uint32_t>(__popc(m & ((1u << w) - 1u)));
-    if (n >= c) {
-      n -= c;
-      m >>= w;
-      pos += w;
-    }
-  }
-  return pos;
 }
 
 // the parallel scan (above).  Builds with four, five or six blocks of 256
@@ -1056,15 +1091,17 @@ __device__ __forceinline__ void station_dests_slot(state const& st, uint32_t* X,
 // The destination passes of both phases can run ahead of the other
 // stations' transfers because they alone write the destinations' labels:
 // k_relax leaves out transfers at, and footpaths into, destinations.
+// The first blocks take the slots, 8 each, the others the words.
 __global__ void __launch_bounds__(256) k_reached(state st) {
   __shared__ fp_cand cand[8][kMaxFpCand];
   auto const lane = threadIdx.x & 31u;
-  auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  auto const n_warps = (gridDim.x * blockDim.x) >> 5;
   auto const par = st.counters[C_PAR];
-  for (auto s = warp; s < st.S; s += n_warps) {
+  auto const slot_blocks = (st.S + 7u) / 8u;
+  if (blockIdx.x < slot_blocks) {
+    auto const s = blockIdx.x * 8u + (threadIdx.x >> 5);
+    if (s >= st.S) return;
     auto const ln = st.lanes[s];
-    if (!ln.run) continue;
+    if (!ln.run) return;
     auto& sl = st.slots[s];
     auto const tad0 = static_cast<int>(sl.tad[ln.k]);
     if (lane < 2u) {
@@ -1074,11 +1111,12 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
     __syncwarp();
     if (ln.mode & 1u) intermodal_slot(st, sl, ln, s, lane, tad0);
     else if (ln.mode & 2u) station_dests_slot(st, st.X[par], sl, ln, s, lane, cand[threadIdx.x >> 5]);
-    __syncwarp();
+    return;
   }
+  auto const block = blockIdx.x - slot_blocks, n_blocks = gridDim.x - slot_blocks;
   auto const n = st.tt.n_loc * st.G;
   auto* X = st.X[par ^ 1u];
-  for (auto i = (blockIdx.x * blockDim.x + threadIdx.x) * 4u; i < n; i += gridDim.x * blockDim.x * 4u) {
+  for (auto i = (block * blockDim.x + threadIdx.x) * 4u; i < n; i += n_blocks * blockDim.x * 4u) {
     if (i + 3u < n) {
       auto* p = reinterpret_cast<uint4*>(X + i);
       auto const v = *p;
@@ -1087,7 +1125,7 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
       for (auto j = i; j < n; ++j) X[j] = 0u;
     }
   }
-  list_nonzero(st, st.Y, n, C_Y, [&](uint32_t at, uint32_t e, uint32_t) { st.ylist[at] = e; });
+  list_nonzero(st, st.Y, n, C_Y, block, n_blocks, [&](uint32_t at, uint32_t e, uint32_t) { st.ylist[at] = e; });
 }
 
 // ------------------------------------------------ transfers and footpaths
@@ -1152,29 +1190,40 @@ __global__ void k_relax(state st) {
         auto const* dat = fp_words(T, prf, fwd);
         auto const fb = idx[src], n = idx[src + 1] - fb;
         auto const tad_flat = static_cast<int>(st.tad_phase[st.S + s]);
-        for (auto j = 0u; j != n; ++j) {
-          auto const fp = dat[fb + j];
-          auto const tgt = B2R_FP_TARGET(fp);
-          if (stations && ((st.D[tgt * st.G + g] >> b) & 1u)) continue;
-          auto const dur = static_cast<int>(B2R_FP_DURATION(fp));
-          auto const key = key_add(tk, (ln.mode & 4u) ? dur : adjusted<int>(tts, dur));
-          auto const bk = dec(st.best[li(st, tgt, s)], ln.gtag);
-          if (key >= bk) continue;
-          if (ln.blast == 0u) {
-            atomicMin(&st.rt[rti(st, ln.k, tgt, s)], enc(ln.qtag, key));
-            touch(st, ln, ln.k, tgt, s);
+        // four footpaths at a time: their targets' labels load together
+        for (auto j0 = 0u; j0 < n; j0 += 4u) {
+          uint32_t fps[4];
+          int bks[4];
+#pragma unroll
+          for (auto x = 0u; x != 4u; ++x) fps[x] = j0 + x < n ? dat[fb + j0 + x] : B2R_INVALID_IDX;
+#pragma unroll
+          for (auto x = 0u; x != 4u; ++x) {
+            bks[x] = j0 + x < n ? dec(st.best[li(st, B2R_FP_TARGET(fps[x]), s)], ln.gtag) : -32768;
           }
-          auto const tad = stations ? tad_at(st, 1u, s, src, j) : tad_flat;
-          if (key > tad) continue;
-          auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, tgt, s)];
-          if (lbv != 0xFFFFu && key + static_cast<int>(lbv) <= tad) {
-            if (ln.blast != 0u) {
-              if (!within_bounds(st, s, ln.blast, ln.k, tgt, key)) continue;
+#pragma unroll
+          for (auto x = 0u; x != 4u; ++x) {
+            auto const j = j0 + x;
+            auto const tgt = B2R_FP_TARGET(fps[x]);
+            auto const dur = static_cast<int>(B2R_FP_DURATION(fps[x]));
+            auto const key = key_add(tk, (ln.mode & 4u) ? dur : adjusted<int>(tts, dur));
+            if (key >= bks[x]) continue;  // no key is below -32768: the places past the end too
+            if (stations && ((st.D[tgt * st.G + g] >> b) & 1u)) continue;
+            if (ln.blast == 0u) {
               atomicMin(&st.rt[rti(st, ln.k, tgt, s)], enc(ln.qtag, key));
               touch(st, ln, ln.k, tgt, s);
             }
-            atomicMin(&st.best[li(st, tgt, s)], enc(ln.gtag, key));
-            atomicOr(&X[tgt * st.G + g], 1u << b);
+            auto const tad = stations ? tad_at(st, 1u, s, src, j) : tad_flat;
+            if (key > tad) continue;
+            auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[li(st, tgt, s)];
+            if (lbv != 0xFFFFu && key + static_cast<int>(lbv) <= tad) {
+              if (ln.blast != 0u) {
+                if (!within_bounds(st, s, ln.blast, ln.k, tgt, key)) continue;
+                atomicMin(&st.rt[rti(st, ln.k, tgt, s)], enc(ln.qtag, key));
+                touch(st, ln, ln.k, tgt, s);
+              }
+              atomicMin(&st.best[li(st, tgt, s)], enc(ln.gtag, key));
+              atomicOr(&X[tgt * st.G + g], 1u << b);
+            }
           }
         }
       });
@@ -1485,18 +1534,20 @@ __device__ void next_slot(state const& st, uint32_t* X, slot_t& sl, uint32_t s, 
 // slots: the round's end (raptor.h:217), collection when the group's rounds
 // are over, the journeys to rebuild listed (the slot then waits one step in
 // S_RECON), the next start-time group seeded, and the slot's views for the
-// next step (lane record, the group's run and sweep masks) and for the host
+// next step (lane record, the group's run mask and, per round, its slots to
+// sweep) and for the host
 // (summary).  seed_only: admitted slots are seeded and the views renewed,
 // nothing else (after an admission, so that a query's first super-step is
 // its first round).
 // A thread per slot walked destinations x rounds and the journey list one
 // dependent load at a time.
 __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
-  __shared__ uint32_t run_bits, sweep_bits;
+  __shared__ uint32_t run_bits, sweep_bits[kK];
   auto const lane = threadIdx.x & 31u;
   auto const g = blockIdx.x;
   auto const s = g * 32u + (threadIdx.x >> 5);
-  if (threadIdx.x == 0u) run_bits = sweep_bits = 0u;
+  if (threadIdx.x == 0u) run_bits = 0u;
+  if (threadIdx.x < kK) sweep_bits[threadIdx.x] = 0u;
   __syncthreads();
   auto const par = st.counters[C_PAR];
   auto& sl = st.slots[s];
@@ -1533,15 +1584,15 @@ __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
     st.lanes[s] = lane_of(sl);
     if (sl.state == S_RUN) {
       atomicOr(&run_bits, 1u << (s & 31u));
-      if (sl.need_sweep) atomicOr(&sweep_bits, 1u << (s & 31u));
+      if (sl.need_sweep) atomicOr(&sweep_bits[sl.k], 1u << (s & 31u));
     }
   }
   __syncthreads();
   if (threadIdx.x == 0u) {
     st.run_mask[g] = run_bits;
-    st.sweep_mask[g] = sweep_bits;
     st.any_mask[g] = 0u;
   }
+  if (threadIdx.x < kK) st.sweep_k[g * kK + threadIdx.x] = sweep_bits[threadIdx.x];
 }
 
 // ------------------------------------------------------- lower bounds
