@@ -155,7 +155,10 @@ struct b2r_engine {
   uint64_t bytes_per_slot{0}, bytes{0};
   b2r::dev::state st{};
   cudaStream_t stream{nullptr};
-  cudaGraphExec_t graph[2]{nullptr, nullptr};  // the super-step, without and with journeys rebuilt beside it
+  // the super-step without and with journeys rebuilt beside it ([0], [1]);
+  // graph_steps of them ([2], [3], if more than one)
+  cudaGraphExec_t graph[4]{nullptr, nullptr, nullptr, nullptr};
+  uint32_t graph_steps{0};
   cudaStream_t stream_recon{nullptr};           // the latter's branch
   cudaEvent_t ev_fork{nullptr}, ev_join{nullptr};
   cudaStream_t stream2{nullptr};  // exports overlapping the super-steps
@@ -600,19 +603,39 @@ unsigned blocks_for(uint64_t n, uint64_t per, uint64_t most) {
   return static_cast<unsigned>(std::min<uint64_t>(most, std::max<uint64_t>(1U, (n + per - 1U) / per)));
 }
 
+template <typename... P, typename... A>
+void launch(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, bool early, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = early ? 1U : 0U;
+  B2R_CUDA(cudaLaunchKernelEx(&c, k, P(args)...));
+}
+
 // One round of every running slot.  recon: some resident query runs several
 // start-time groups, so journeys are rebuilt between them; that kernel runs
 // on stream2 beside the round's, from the swap of the mark arrays (k_routes)
-// to the end of the step.
-void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
+// to the end of the step.  follows: another super-step is the work before
+// this one on the stream.
+// Every kernel after the first is launched with a programmatic dependency on
+// the one before (step_begin in kernels.cuh), which takes its launch off the
+// step's path; not where a step's kernels are timed one by one, and not
+// across the join with the reconstruction branch.
+void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon, bool follows) {
   auto const& st = e.st;
   auto const words = static_cast<uint64_t>(st.tt.n_loc) * e.G;
   auto const pair_blocks = static_cast<uint64_t>(e.sms) * e.shape.pair_blocks_per_sm;
   auto const slot_blocks = (e.S + 7U) / 8U;  // a warp per slot
   auto const list_blocks = static_cast<uint64_t>(e.sms) * 8U;
-  dev::k_mark<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
-  dev::k_routes<<<slot_blocks + blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks), 256, 0,
-                  s>>>(st);
+  auto const early = e.cfg.profile == 0U;
+  launch(dev::k_mark, blocks_for(words, 256U, pair_blocks), 256U, s, early && follows, st);
+  launch(dev::k_routes, slot_blocks + blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks), 256U,
+         s, early, st);
   cudaEvent_t rc_a = nullptr, rc_b = nullptr;
   if (recon) {
     auto* s2 = e.stream_recon;
@@ -645,19 +668,19 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
     ev_b = e.prof_ev[e.prof_used++];
     B2R_CUDA(cudaEventRecord(ev_a, s));
   }
-  if (e.tt->n_unordered != 0U) dev::k_route_scan_seq<<<list_blocks, 256, 0, s>>>(st);
+  if (e.tt->n_unordered != 0U) launch(dev::k_route_scan_seq, static_cast<unsigned>(list_blocks), 256U, s, early, st);
   {
     auto const block = e.shape.scan_threads;
     auto const grid = blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, block / dev::kTile,
                                  static_cast<uint64_t>(e.sms) * e.shape.scan_blocks_per_sm);
     if (e.cfg.profile == 1U) {
-      dev::k_route_scan<4, true><<<grid, block, 0, s>>>(st);
+      launch(dev::k_route_scan<4, true>, grid, block, s, early, st);
     } else if (e.shape.scan_occupancy == 2U) {
-      dev::k_route_scan<6, false><<<grid, block, 0, s>>>(st);
+      launch(dev::k_route_scan<6, false>, grid, block, s, early, st);
     } else if (e.shape.scan_occupancy == 1U) {
-      dev::k_route_scan<5, false><<<grid, block, 0, s>>>(st);
+      launch(dev::k_route_scan<5, false>, grid, block, s, early, st);
     } else {
-      dev::k_route_scan<4, false><<<grid, block, 0, s>>>(st);
+      launch(dev::k_route_scan<4, false>, grid, block, s, early, st);
     }
   }
   if (e.cfg.profile == 2U) {
@@ -667,25 +690,26 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon) {
     auto const idx = static_cast<uint32_t>(e.prof_used / 2 - 1);
     if (idx < b2r_engine::kProfRows) k_prof_row<<<1, 1, 0, s>>>(st, e.d_prof_rows, idx);
   }
-  if (st.tt.n_rt != 0U) dev::k_rt_scan<<<pair_blocks, 256, 0, s>>>(st);
-  dev::k_reached<<<slot_blocks + blocks_for(words, 1024U, list_blocks), 256, 0, s>>>(st);
-  dev::k_relax<<<blocks_for(words, 256U, pair_blocks), 256, 0, s>>>(st);
+  if (st.tt.n_rt != 0U) launch(dev::k_rt_scan, static_cast<unsigned>(pair_blocks), 256U, s, early, st);
+  launch(dev::k_reached, slot_blocks + blocks_for(words, 1024U, list_blocks), 256U, s, early, st);
+  launch(dev::k_relax, blocks_for(words, 256U, pair_blocks), 256U, s, early, st);
   if (recon) B2R_CUDA(cudaStreamWaitEvent(s, e.ev_join, 0));
-  dev::k_end<<<e.G, 1024, 0, s>>>(st, false);
+  launch(dev::k_end, e.G, 1024U, s, early && !recon, st, false);
 }
 uint64_t launches_per_step(b2r_engine const& e, bool recon) {
   return 6U + (recon ? 1U : 0U) + (e.st.tt.n_rt != 0U ? 1U : 0U) + (e.tt->n_unordered != 0U ? 1U : 0U);
 }
 
-// a super-step as its graph (recon: the one with the reconstruction branch)
-// or as single launches
-void run_superstep(b2r_engine& e, cudaStream_t s, bool graph, bool recon) {
-  if (graph) {
-    B2R_CUDA(cudaGraphLaunch(e.graph[recon ? 1 : 0], s));
-  } else {
-    enqueue_superstep(e, s, recon);
+// n super-steps as graphs (recon: the ones with the reconstruction branch),
+// of a whole chunk as far as they go, or as single launches
+void run_supersteps(b2r_engine& e, cudaStream_t s, bool graph, bool recon, uint32_t n) {
+  if (!graph) {
+    for (auto i = 0U; i != n; ++i) enqueue_superstep(e, s, recon, i != 0U);
     B2R_CUDA(cudaGetLastError());
+    return;
   }
+  for (; e.graph_steps > 1U && n >= e.graph_steps; n -= e.graph_steps) B2R_CUDA(cudaGraphLaunch(e.graph[recon ? 3 : 2], s));
+  for (; n != 0U; --n) B2R_CUDA(cudaGraphLaunch(e.graph[recon ? 1 : 0], s));
 }
 
 // admitted slots get their first start labels (and every slot its views) for
@@ -1783,11 +1807,9 @@ struct batch_runner {
       B2R_CUDA(cudaEventRecord(e.ev0, st));
       auto recon = false;
       for (auto const x : slot_q) recon = recon || (x >= 0 && rebuilds_between_groups(runs[static_cast<size_t>(x)].p));
-      for (uint32_t c = 0; c != n_steps; ++c) {
-        run_superstep(e, st, use_graph, recon);
-        launches += launches_per_step(e, recon);
-        ++steps;
-      }
+      run_supersteps(e, st, use_graph, recon, n_steps);
+      launches += n_steps * launches_per_step(e, recon);
+      steps += n_steps;
       B2R_CUDA(cudaEventRecord(e.ev1, st));
       e.d2h_bytes += S * sizeof(b2r_engine::summary_t);
       B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, S * sizeof(b2r_engine::summary_t),
@@ -1936,12 +1958,13 @@ void drop_graphs(b2r_engine& e) {
 
 void capture_graph(b2r_engine& e) {
   drop_graphs(e);
-  for (auto recon = 0; recon != 2; ++recon) {
+  e.graph_steps = e.cfg.profile == 2U ? 1U : e.shape.steps_per_sync;
+  for (auto i = 0U; i != (e.graph_steps > 1U ? 4U : 2U); ++i) {
     cudaGraph_t g = nullptr;
     B2R_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_superstep(e, e.stream, recon != 0);
+    for (auto x = 0U; x != (i < 2U ? 1U : e.graph_steps); ++x) enqueue_superstep(e, e.stream, (i & 1U) != 0U, x != 0U);
     B2R_CUDA(cudaStreamEndCapture(e.stream, &g));
-    B2R_CUDA(cudaGraphInstantiate(&e.graph[recon], g, 0));
+    B2R_CUDA(cudaGraphInstantiate(&e.graph[i], g, 0));
     cudaGraphDestroy(g);
   }
 }
@@ -2165,7 +2188,7 @@ struct serve_state {
         for (auto const* x : slot_item) recon = recon || (x != nullptr && rebuilds_between_groups(x->run.p));
         this->n_steps += n_steps;
         n_launches += n_steps * launches_per_step(e, recon);
-        for (uint32_t c = 0; c != n_steps; ++c) run_superstep(e, st, use_graph, recon);
+        run_supersteps(e, st, use_graph, recon, n_steps);
         B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, e.S * sizeof(b2r_engine::summary_t),
                                  cudaMemcpyDeviceToHost, st));
         in_flight = true;
@@ -3194,7 +3217,7 @@ dev::slot_summary run_slot0(b2r_engine& e) {
   auto* st = e.stream;
   for (uint64_t step = 0;; ++step) {
     if (step > 100000) throw std::runtime_error("super-step cap exceeded");
-    run_superstep(e, st, e.cfg.use_graphs != 0 && e.graph[0] != nullptr, false);
+    run_supersteps(e, st, e.cfg.use_graphs != 0 && e.graph[0] != nullptr, false, 1U);
     B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, sizeof(b2r_engine::summary_t), cudaMemcpyDeviceToHost, st));
     B2R_CUDA(cudaStreamSynchronize(st));
     auto const state = e.h_summary[0].state;

@@ -19,6 +19,16 @@ enum : uint32_t {
 };
 constexpr uint32_t recon_counter(uint32_t par) { return par == 0u ? C_RECON0 : C_RECON1; }
 
+// The first thing every super-step kernel does.  The kernels of a step are
+// launched with programmatic dependencies (enqueue_superstep): the next one
+// may take its place on the SMs from here on, so that its launch does not
+// wait for this one's end, and this one reads and writes nothing before all
+// kernels ahead of it are complete.
+__device__ __forceinline__ void step_begin() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
 __device__ __forceinline__ size_t li(state const& st, uint32_t l, uint32_t s) {
   return static_cast<size_t>(l) * st.S + s;
 }
@@ -251,6 +261,7 @@ __device__ __forceinline__ void sweep(state const& st, uint32_t lane, uint32_t w
 // atomic redundant, and same-address atomics would queue in L2.  A marked
 // real-time run (n_rt != 0) also keeps its queries in the round.
 __global__ void k_mark(state st) {
+  step_begin();
   auto const lane = threadIdx.x & 31u;
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
@@ -407,6 +418,7 @@ __device__ __forceinline__ void dest_slot(state const& st, uint32_t s, uint32_t 
 // reads and X[C_PAR] takes the marks it makes.  The first blocks take the
 // slots, 8 each, the others the lists, so that neither waits for the other.
 __global__ void __launch_bounds__(256) k_routes(state st) {
+  step_begin();
   auto const lane = threadIdx.x & 31u;
   if (blockIdx.x == 0u && threadIdx.x == 0u) st.counters[C_PAR] ^= 1u;
   auto const slot_blocks = (st.S + 7u) / 8u;
@@ -566,6 +578,7 @@ __device__ __forceinline__ void scan_walk_seq(state const& st, uint32_t const* X
 // one trip order at every event (launched only if the timetable has any).
 // A thread per marked (route, group) entry.
 __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ state st) {
+  step_begin();
   auto const& T = st.tt;
   auto const nr = st.counters[C_R];
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
@@ -606,6 +619,7 @@ struct scan_smem {                       // of a warp
 };
 template <int MinBlocks, bool Prof>
 __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
+  step_begin();
   constexpr uint32_t kNone = 0xFFFFFFFFu;
   constexpr uint32_t kCarried = 32u;
   __shared__ scan_smem smem[8];
@@ -849,6 +863,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
 // A lane per pair walked the run one stop at a time, four dependent loads
 // each.
 __global__ void __launch_bounds__(256) k_rt_scan(const __grid_constant__ state st) {
+  step_begin();
   auto const& T = st.tt;
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
   auto const lane = threadIdx.x & 31u;
@@ -1093,6 +1108,7 @@ __device__ __forceinline__ void station_dests_slot(state const& st, uint32_t* X,
 // k_relax leaves out transfers at, and footpaths into, destinations.
 // The first blocks take the slots, 8 each, the others the words.
 __global__ void __launch_bounds__(256) k_reached(state st) {
+  step_begin();
   __shared__ fp_cand cand[8][kMaxFpCand];
   auto const lane = threadIdx.x & 31u;
   auto const par = st.counters[C_PAR];
@@ -1142,6 +1158,7 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
 // pruning bounds differ between the phases, and each keeps its own
 // (tad_phase, timelines; k_reached).
 __global__ void k_relax(state st) {
+  step_begin();
   auto const& T = st.tt;
   auto* X = st.X[st.counters[C_PAR]];
   for_each_pair(
@@ -1542,6 +1559,7 @@ __device__ void next_slot(state const& st, uint32_t* X, slot_t& sl, uint32_t s, 
 // A thread per slot walked destinations x rounds and the journey list one
 // dependent load at a time.
 __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
+  step_begin();
   __shared__ uint32_t run_bits, sweep_bits[kK];
   auto const lane = threadIdx.x & 31u;
   auto const g = blockIdx.x;
