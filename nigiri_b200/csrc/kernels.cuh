@@ -260,11 +260,20 @@ __device__ __forceinline__ void sweep(state const& st, uint32_t lane, uint32_t w
 // gains bits during the kernel, so a read that shows the bits set makes the
 // atomic redundant, and same-address atomics would queue in L2.  A marked
 // real-time run (n_rt != 0) also keeps its queries in the round.
-__global__ void k_mark(state st) {
+// Only queries whose label at the station time_at_dest does not rule out
+// already mark its routes: a trip search from the others ends at its first
+// event (every event is at or after the label, and the search prunes with
+// this station's bound), so a pair marked by none but them reaches nothing.
+// One look at the label here saves one in each of the station's 19 routes,
+// and the pairs that drop out are never scanned.  The round loop's "any
+// route marked" still counts every mark, as do the real-time runs' marks.
+__global__ void __launch_bounds__(256) k_mark(state st) {
   step_begin();
+  __shared__ uint32_t live_bits[8][32];
   auto const lane = threadIdx.x & 31u;
   auto const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto const n_warps = (gridDim.x * blockDim.x) >> 5;
+  auto* live = live_bits[threadIdx.x >> 5];
   auto const par = st.counters[C_PAR];
   auto const* X = st.X[par];
   auto const& T = st.tt;
@@ -284,10 +293,10 @@ __global__ void k_mark(state st) {
     i += step;
     x = i < n ? X[i] : 0u;  // the next pass's word, in flight during this one
     if (__ballot_sync(kFull, w != 0u) == 0u) continue;
-    uint32_t g = 0, rb = 0, cnt = 0;
+    uint32_t g = 0, l = 0, rb = 0, cnt = 0;
     if (w != 0u) {
       g = e % st.G;
-      auto const l = e / st.G;
+      l = e / st.G;
       w &= st.run_mask[g];
       if (w != 0u) {
         rb = __ldg(T.loc_routes_idx + l);
@@ -299,7 +308,47 @@ __global__ void k_mark(state st) {
           for (auto j = 0u; j != m; ++j) atomicOr(&st.RT_R[T.loc_rt[b + j] * st.G + g], w);
         }
         if (any != 0u && (st.any_mask[g] & w) != w) atomicOr(&st.any_mask[g], w);
+        if (cnt == 0u) w = 0u;
       }
+    }
+    // the live queries of each word, its (word, query) pairs spread over the lanes
+    {
+      live[lane] = 0u;
+      auto const bits = static_cast<uint32_t>(__popc(w));
+      auto end = bits;
+      for (auto o = 1u; o < 32u; o <<= 1) {
+        auto const v = __shfl_up_sync(kFull, end, o);
+        if (lane >= o) end += v;
+      }
+      auto const total = __shfl_sync(kFull, end, 31);
+      __syncwarp();
+      for (auto p0 = 0u; p0 < total; p0 += 32u) {
+        auto const p = p0 + lane;
+        uint32_t owner = 0;  // first lane whose prefix end exceeds p
+        for (auto b = 16u; b > 0u; b >>= 1) {
+          if (__shfl_sync(kFull, end, static_cast<int>(owner + b - 1u)) <= p) owner += b;
+        }
+        auto const o_first = __shfl_sync(kFull, end, static_cast<int>(owner)) -
+                             __shfl_sync(kFull, bits, static_cast<int>(owner));
+        auto const o_w = __shfl_sync(kFull, w, static_cast<int>(owner));
+        auto const o_g = __shfl_sync(kFull, g, static_cast<int>(owner));
+        auto const o_l = __shfl_sync(kFull, l, static_cast<int>(owner));
+        if (p < total) {
+          auto const b = nth_bit(o_w, p - o_first);
+          auto const s = o_g * 32u + b;
+          auto const ln = st.lanes[s];
+          auto const at = li(st, o_l, s);
+          auto const prt = dec(st.rt[static_cast<size_t>(ln.k - 1u) * T.n_loc * st.S + at], ln.qtag);
+          auto const lbv = (ln.mode & 8u) ? uint16_t{0} : st.lb[at];
+          if (prt != kKeyInv && lbv != 0xFFFFu && prt + static_cast<int>(lbv) <= ln.tad_k) {
+            atomicOr(&live[owner], 1u << b);
+          }
+        }
+      }
+      __syncwarp();
+      w = live[lane];
+      __syncwarp();
+      if (w == 0u) cnt = 0u;
     }
     auto end = cnt;  // inclusive prefix sum of the route counts
     for (auto o = 1u; o < 32u; o <<= 1) {
