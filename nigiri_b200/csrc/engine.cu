@@ -619,8 +619,8 @@ void launch(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, bool
 
 // One round of every running slot.  recon: some resident query runs several
 // start-time groups, so journeys are rebuilt between them; that kernel runs
-// on stream2 beside the round's, from the swap of the mark arrays (k_routes)
-// to the end of the step.  follows: another super-step is the work before
+// on stream_recon beside the round's, from the end of the marking to the end
+// of the step.  follows: another super-step is the work before
 // this one on the stream.
 // Every kernel after the first is launched with a programmatic dependency on
 // the one before (step_begin in kernels.cuh), which takes its launch off the
@@ -634,8 +634,6 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon, bool follows) 
   auto const list_blocks = static_cast<uint64_t>(e.sms) * 8U;
   auto const early = e.cfg.profile == 0U;
   launch(dev::k_mark, blocks_for(words, 256U, pair_blocks), 256U, s, early && follows, st);
-  launch(dev::k_routes, slot_blocks + blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks), 256U,
-         s, early, st);
   cudaEvent_t rc_a = nullptr, rc_b = nullptr;
   if (recon) {
     auto* s2 = e.stream_recon;
@@ -655,6 +653,8 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon, bool follows) 
     if (e.cfg.profile == 1U) B2R_CUDA(cudaEventRecord(rc_b, s2));
     B2R_CUDA(cudaEventRecord(e.ev_join, s2));
   }
+  launch(dev::k_routes, slot_blocks + blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, 1024U, list_blocks), 256U,
+         s, early, st);
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   if (e.cfg.profile == 2U) {  // timing build: one event pair, captured in the super-step graph
     B2R_CUDA(record_in_graph(e.ev_scan_a, s));
@@ -671,7 +671,7 @@ void enqueue_superstep(b2r_engine& e, cudaStream_t s, bool recon, bool follows) 
   if (e.tt->n_unordered != 0U) launch(dev::k_route_scan_seq, static_cast<unsigned>(list_blocks), 256U, s, early, st);
   {
     auto const block = e.shape.scan_threads;
-    auto const grid = blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, block / dev::kTile,
+    auto const grid = blocks_for(static_cast<uint64_t>(st.tt.n_routes) * e.G, block / 32U,
                                  static_cast<uint64_t>(e.sms) * e.shape.scan_blocks_per_sm);
     if (e.cfg.profile == 1U) {
       launch(dev::k_route_scan<4, true>, grid, block, s, early, st);
@@ -2657,6 +2657,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       st.S = e->S;
       st.G = e->G;
       st.max_j = e->max_j;
+      st.sms = static_cast<uint32_t>(e->sms);
       auto& by = e->bytes;
       auto al = [&](auto*& p, size_t n) {
         using T = std::remove_reference_t<decltype(*p)>;

@@ -250,6 +250,7 @@ struct state {
   uint32_t S;        // slots (multiple of 32)
   uint32_t G;        // slot groups of 32
   uint32_t max_j;    // journeys per slot
+  uint32_t sms;      // multiprocessors
   slot_t* slots;
   lane_t* lanes;
   uint32_t* rt;     // [K][n_loc][S]

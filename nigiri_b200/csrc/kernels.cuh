@@ -13,9 +13,10 @@ namespace b2r::dev {
 
 // C_PAR: which of the two station-mark arrays the next marks go to (k_routes
 // flips it between a step's reads and its writes); C_RECON0 + parity: the
-// journeys listed for reconstruction
+// journeys listed for reconstruction; C_RPAR: the parity of those the step
+// rebuilds
 enum : uint32_t {
-  C_PAR = 0, C_Y = 1, C_R = 2, C_RECON0 = 3, C_ERR = 4, C_F0 = 5, C_F1 = 6, C_RT = 7, C_RECON1 = 8
+  C_PAR = 0, C_Y = 1, C_R = 2, C_RECON0 = 3, C_ERR = 4, C_F0 = 5, C_F1 = 6, C_RT = 7, C_RECON1 = 8, C_RPAR = 9
 };
 constexpr uint32_t recon_counter(uint32_t par) { return par == 0u ? C_RECON0 : C_RECON1; }
 
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(256) k_mark(state st) {
     st.counters[C_R] = 0u;
     st.counters[C_RT] = 0u;
     st.counters[recon_counter(par ^ 1u)] = 0u;
+    st.counters[C_RPAR] = par;  // the list the last k_end filled
   }
   auto const n = T.n_loc * st.G;
   auto const step = n_warps * 32u;
@@ -499,7 +501,8 @@ __global__ void __launch_bounds__(256) k_routes(state st) {
 // one (route, query) pair is a chain of dependent loads as long as the
 // route.
 //
-// Here 8 lanes take one pair, a warp four pairs, 32 stops at a time:
+// Here 8 lanes take one pair, a warp four pairs, 32 stops at a time (32
+// lanes and one pair where there are few, kFewPerSm):
 // * the lanes read the stops' marks, four stops each, and for the marked
 //   boardable ones the label to board from; those that time_at_dest does
 //   not rule out are the searches;
@@ -654,36 +657,39 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
   }
 }
 
-// the parallel scan (above).  Builds with four, five or six blocks of 256
-// threads resident per SM (the launch shape picks one), and with work
-// counters for profiling engines (Prof).  Every loop that shuffles or
-// ballots is uniform over the warp; a tile without work takes part idle.
-constexpr uint32_t kTile = 8;            // lanes of a pair
-constexpr uint32_t kPer = 32u / kTile;   // stops a lane takes of each 32; pairs of a warp
-struct scan_smem {                       // of a warp
+// The parallel scan (above) with kTile lanes per pair.  Every loop that
+// shuffles or ballots is uniform over the warp; a tile without work takes
+// part idle.
+template <uint32_t kTile>
+struct scan_smem {  // of a warp
+  static constexpr uint32_t kPer = 32u / kTile;
   uint4 pair[kPer][4];      // route record (2), lane record, {first stop of the 32, 0, 0, 0}
   uint32_t key[kPer][32];   // per stop: what its search needs (previous label, bound), then the
                             // candidate (order key << 6 | stop), kNone without one
   uint2 trip[kPer][33];     // per stop: the candidate's offset and day; 32: the trip carried in
 };
-template <int MinBlocks, bool Prof>
-__global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
-  step_begin();
+template <uint32_t kTile, bool Prof>
+__device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm, uint32_t nr, scan_ctr& pc) {
+  constexpr uint32_t kPer = 32u / kTile;  // stops a lane takes of each 32; pairs of a warp
+  constexpr uint32_t kTileBits = kTile == 32u ? kFull : (1u << (kTile % 32u)) - 1u;
   constexpr uint32_t kNone = 0xFFFFFFFFu;
   constexpr uint32_t kCarried = 32u;
-  __shared__ scan_smem smem[8];
   auto const& T = st.tt;
   auto const lane = threadIdx.x & 31u;
   auto const tile = lane / kTile, tl = lane % kTile;
-  auto& sm = smem[threadIdx.x >> 5];
   auto const n_tiles = (gridDim.x * blockDim.x) / kTile;
-  auto const nr = st.counters[C_R];
   auto const* X = st.X[st.counters[C_PAR] ^ 1u];
-  auto const tile_bits = [&](bool x) { return (__ballot_sync(kFull, x) >> (tile * kTile)) & ((1u << kTile) - 1u); };
+  auto const tile_bits = [&](bool x) { return (__ballot_sync(kFull, x) >> (tile * kTile)) & kTileBits; };
   auto const tile_shfl = [&](uint32_t x, uint32_t src) {
     return __shfl_sync(kFull, x, static_cast<int>(src), static_cast<int>(kTile));
   };
-  scan_ctr pc{0u, 0u, 0u, 0u, 0u};
+  // With fewer entries than tiles, an entry's queries are shared by 2^split
+  // tiles, each taking the ones in its part of the group: a short frontier
+  // lasts as long as its longest entry, one pair after the other.
+  uint32_t split = 0;
+  while (split < 5u && (nr << (split + 1u)) <= n_tiles) ++split;
+  auto const n_items = nr << split;
+  auto const part_bits = 32u >> split;
   // the tile's entry and pair
   auto w = (blockIdx.x * blockDim.x + threadIdx.x) / kTile;
   uint32_t g = 0, mask = 0, s = 0, sec = 0, i0 = 0;
@@ -699,12 +705,14 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
   while (true) {
     while (!have) {
       if (mask == 0u) {
-        if (w >= nr) break;
-        auto const en = st.rlist[w];
+        if (w >= n_items) break;
+        auto const en = st.rlist[w >> split];
+        mask = en.z & ((split == 0u ? kFull : (1u << part_bits) - 1u) << ((w & ((1u << split) - 1u)) * part_bits));
         w += n_tiles;
+        if (mask == 0u) continue;
         g = en.y;
         R = load_route(T, en.x);
-        mask = (R.flags & kRouteOrder) != 0u ? en.z : 0u;  // else k_route_scan_seq's
+        if ((R.flags & kRouteOrder) == 0u) mask = 0u;  // k_route_scan_seq's
         continue;
       }
       auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
@@ -786,16 +794,25 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       }
       __syncwarp();
       auto const cnt = static_cast<uint32_t>(__popc(m));
-      auto const e1 = __shfl_sync(kFull, cnt, 0);
-      auto const e2 = e1 + __shfl_sync(kFull, cnt, kTile);
-      auto const e3 = e2 + __shfl_sync(kFull, cnt, 2 * kTile);
-      auto const total = e3 + __shfl_sync(kFull, cnt, 3 * kTile);
+      uint32_t ends_at[kPer];  // searches up to each pair's last
+#pragma unroll
+      for (auto x = 0u; x != kPer; ++x) {
+        ends_at[x] = (x == 0u ? 0u : ends_at[x - 1u]) + __shfl_sync(kFull, cnt, static_cast<int>(x * kTile));
+      }
+      auto const total = ends_at[kPer - 1u];
       for (auto q0 = 0u; q0 < total; q0 += 32u) {
         auto const q = q0 + lane;
-        auto const o = (q >= e1 ? 1u : 0u) + (q >= e2 ? 1u : 0u) + (q >= e3 ? 1u : 0u);
+        uint32_t o = 0, first = 0;  // the search's pair and that pair's first search
+#pragma unroll
+        for (auto x = 0u; x + 1u < kPer; ++x) {
+          if (q >= ends_at[x]) {
+            o = x + 1u;
+            first = ends_at[x];
+          }
+        }
         auto const om = __shfl_sync(kFull, m, static_cast<int>(o * kTile));
         if (q < total) {
-          auto const pos = nth_bit(om, q - (o == 0u ? 0u : o == 1u ? e1 : o == 2u ? e2 : e3));
+          auto const pos = nth_bit(om, q - first);
           auto const a = sm.pair[o][0], b = sm.pair[o][1], c = sm.pair[o][2];
           route_rec const oR{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
           auto const oln = *reinterpret_cast<lane_t const*>(&c);
@@ -834,7 +851,7 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       auto run = carry;
 #pragma unroll
       for (auto c = 0u; c != kPer; ++c) {
-        auto const cc = (cuts >> (c * kTile)) & ((1u << kTile) - 1u);
+        auto const cc = (cuts >> (c * kTile)) & kTileBits;
         auto v = ((m >> (c * kTile + tl)) & 1u) != 0u ? sm.key[tile][c * kTile + tl] : kNone;
 #pragma unroll
         for (auto o = 1u; o < kTile; o <<= 1) {
@@ -882,6 +899,28 @@ __global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_cons
       if (ends || i0 >= R.n) have = false;
     }
   }
+}
+
+// Above this many entries per SM the scan takes 8 lanes per pair, else a
+// warp: a step of a warp is about 1,500 instructions for four pairs and 700
+// for one, so with warps to spare one pair ends sooner.
+constexpr uint32_t kFewPerSm = 32;
+
+// Builds with four, five or six blocks of 256 threads resident per SM (the
+// launch shape picks one), and with work counters for profiling engines
+// (Prof).
+template <int MinBlocks, bool Prof>
+__global__ void __launch_bounds__(256, MinBlocks) k_route_scan(const __grid_constant__ state st) {
+  step_begin();
+  __shared__ union {
+    scan_smem<8> few[8];
+    scan_smem<32> one[8];
+  } sm;
+  auto const lane = threadIdx.x & 31u;
+  auto const nr = st.counters[C_R];
+  scan_ctr pc{0u, 0u, 0u, 0u, 0u};
+  if (nr > kFewPerSm * st.sms) scan_tiles<8, Prof>(st, sm.few[threadIdx.x >> 5], nr, pc);
+  else scan_tiles<32, Prof>(st, sm.one[threadIdx.x >> 5], nr, pc);
   if constexpr (Prof) {  // work counters for the roofline (warp-reduced)
     __syncwarp();
     for (auto o = 16; o > 0; o >>= 1) {
@@ -1481,7 +1520,7 @@ __device__ __forceinline__ void reconstruct_one(state const& st, recon_smem<NW>&
 constexpr int kReconWarps = 4;
 __global__ void __launch_bounds__(kReconWarps * 32) k_reconstruct(state st) {
   __shared__ recon_smem<kReconWarps> sm;
-  auto const n = st.counters[recon_counter(st.counters[C_PAR] ^ 1u)];
+  auto const n = st.counters[recon_counter(st.counters[C_RPAR])];
   for (auto i = blockIdx.x; i < n; i += gridDim.x) {
     auto const e = st.recon_list[i];
     reconstruct_one<kReconWarps>(st, sm, e >> 16, e & 0xFFFFu);
