@@ -2646,6 +2646,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
                           (static_cast<uint64_t>(nl) * (4 + b2r::dev::kK) + tt->d.n_routes) / 8 + 256;
       auto by_budget = cfg.hbm_budget / std::max<uint64_t>(1, e->bytes_per_slot);
       auto slots = std::min<uint64_t>(std::max(32U, cfg.max_slots), by_budget);
+      slots = std::min<uint64_t>(slots, 32ULL * b2r::dev::kMaxGroups);
       slots &= ~uint64_t{31};
       if (slots == 0) {
         return b2r::fail(B2R_ERR_OUT_OF_MEMORY, "HBM budget too small for one slot group");
@@ -2684,6 +2685,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.run_mask, G);
       al(st.sweep_k, G * b2r::dev::kK);
       al(st.any_mask, G);
+      al(st.made_mask, G);
       al(st.start_pool, S * e->max_starts);
       al(st.dest_pool, S * e->max_dest);
       al(st.off_pool, S * e->max_off);
@@ -2727,6 +2729,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       B2R_CUDA(cudaMemset(st.run_mask, 0, G * 4));
       B2R_CUDA(cudaMemset(st.sweep_k, 0, G * b2r::dev::kK * 4));
       B2R_CUDA(cudaMemset(st.any_mask, 0, G * 4));
+      B2R_CUDA(cudaMemset(st.made_mask, 0, G * 4));
       B2R_CUDA(cudaMemset(st.Y, 0, static_cast<size_t>(nl) * G * 4));
       B2R_CUDA(cudaMemset(st.R, 0, static_cast<size_t>(tt->d.n_routes) * G * 4));
       B2R_CUDA(cudaMemset(st.D, 0, static_cast<size_t>(nl) * G * 4));

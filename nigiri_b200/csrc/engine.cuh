@@ -25,6 +25,7 @@ constexpr int kKeyInv = 32767;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kMaxLegs = 40;
 constexpr int kMaxTimeline = 128;
+constexpr uint32_t kMaxGroups = 2048;  // slot groups: a slot index has 16 bits (recon_list)
 
 // lrs_stop bits above the position: a ride can end (forward) or begin
 // (backward search) at the pair; the route's event columns are ordered
@@ -271,7 +272,8 @@ struct state {
   uint32_t* counters;  // C_*: list lengths, mark parity, error bits
   uint32_t* run_mask;  // [G]
   uint32_t* sweep_k;   // [G][K] slots to sweep that are at round k
-  uint32_t* any_mask;  // [G]
+  uint32_t* any_mask;  // [G] a route of this round is marked
+  uint32_t* made_mask;  // [G] the round has marked a station
   start_rec* start_pool;
   dest_rec* dest_pool;
   b2r_offset* off_pool;

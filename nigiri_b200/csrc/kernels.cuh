@@ -472,6 +472,9 @@ __global__ void __launch_bounds__(256) k_routes(state st) {
   step_begin();
   auto const lane = threadIdx.x & 31u;
   if (blockIdx.x == 0u && threadIdx.x == 0u) st.counters[C_PAR] ^= 1u;
+  if (blockIdx.x == 0u) {
+    for (auto g = threadIdx.x; g < st.G; g += blockDim.x) st.made_mask[g] = 0u;
+  }
   auto const slot_blocks = (st.S + 7u) / 8u;
   if (blockIdx.x < slot_blocks) {
     auto const s = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -1058,6 +1061,7 @@ __device__ __forceinline__ void dest_label(state const& st, uint32_t* X, slot_t&
   touch(st, ln, k, d, s);
   st.best[li(st, d, s)] = enc(ln.gtag, key);
   atomicOr(&X[d * st.G + (s >> 5)], 1u << (s & 31u));
+  atomicOr(&st.made_mask[s >> 5], 1u << (s & 31u));
   if (key < tad) {
     if (tl_n < kMaxTimeline) {
       st.timeline[(static_cast<size_t>(ph) * st.S + s) * kMaxTimeline + tl_n++] = {pos_hi, pos_lo, key};
@@ -1245,8 +1249,15 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
 // by another one of the round is above a value that is written anyway.  The
 // pruning bounds differ between the phases, and each keeps its own
 // (tad_phase, timelines; k_reached).
-__global__ void k_relax(state st) {
+//
+// Which queries marked a station is gathered per block and written once (a
+// global word per group read and written by every pair doubled the kernel's
+// time at 1,024 slots).
+__global__ void __launch_bounds__(256) k_relax(state st) {
   step_begin();
+  __shared__ uint32_t made_bits[kMaxGroups];
+  for (auto g = threadIdx.x; g < st.G; g += blockDim.x) made_bits[g] = 0u;
+  __syncthreads();
   auto const& T = st.tt;
   auto* X = st.X[st.counters[C_PAR]];
   for_each_pair(
@@ -1265,6 +1276,7 @@ __global__ void k_relax(state st) {
         if (tk == kKeyInv) return;
         auto const stations = (ln.mode & 2u) != 0u;
         auto const& tts = st.slots[s].tts;
+        bool made = false;  // a station marked
         if (!stations || !((st.D[e] >> b) & 1u)) {
           auto const tt = static_cast<int>(T.transfer_time[src]);
           auto const fp = key_add(tk, (ln.mode & 4u) ? tt : static_cast<int>(adjusted<int>(tts, tt)));
@@ -1286,6 +1298,7 @@ __global__ void k_relax(state st) {
               }
               atomicMin(&st.best[li(st, src, s)], enc(ln.gtag, fp));
               atomicOr(&X[e], 1u << b);
+              made = true;
             }
           }
         }
@@ -1328,10 +1341,16 @@ __global__ void k_relax(state st) {
               }
               atomicMin(&st.best[li(st, tgt, s)], enc(ln.gtag, key));
               atomicOr(&X[tgt * st.G + g], 1u << b);
+              made = true;
             }
           }
         }
+        if (made && ((made_bits[g] >> b) & 1u) == 0u) atomicOr(&made_bits[g], 1u << b);
       });
+  __syncthreads();
+  for (auto g = threadIdx.x; g < st.G; g += blockDim.x) {
+    if (made_bits[g] != 0u) atomicOr(&st.made_mask[g], made_bits[g]);
+  }
 }
 
 // ------------------------------------------------- round end / results
@@ -1635,8 +1654,31 @@ __device__ void next_slot(state const& st, uint32_t* X, slot_t& sl, uint32_t s, 
   }
 }
 
+// Round k of a slot whose last round marked no station, without a super-step
+// of its own: all it does is to count, to sweep and to take the destination
+// times (raptor.h:218-226) before it finds nothing marked (raptor.h:243-246),
+// and of the swept labels only the destinations' are read again.
+__device__ __forceinline__ void empty_round(state const& st, slot_t& sl, uint32_t s, uint32_t k, uint32_t lane) {
+  if (!sl.one_to_all) {
+    auto const gtag = tagcode(sl.gen_group), qtag = tagcode(sl.gen_query);
+    int key = kKeyInv;
+    auto const take = [&](uint32_t d) {
+      key = min(key, min(dec(st.best[li(st, d, s)], gtag), dec(st.rt[rti(st, k, d, s)], qtag)));
+    };
+    if (sl.intermodal_dest) {
+      take(B2R_SPECIAL_END);
+    } else {
+      for (auto i = lane; i < sl.n_dest; i += 32u) take(st.dest_pool[sl.dest_off + i].loc);
+    }
+    key = __reduce_min_sync(kFull, key);
+    if (lane >= k && lane < kK && key < sl.tad[lane]) sl.tad[lane] = static_cast<int16_t>(key);
+  }
+  if (lane == 0u) ++sl.n_rounds;
+}
+
 // The end of a super-step, a warp per slot and a block per group of 32
-// slots: the round's end (raptor.h:217), collection when the group's rounds
+// slots: the round's end (raptor.h:217), the next round at once if it would
+// be empty (one step in six), collection when the group's rounds
 // are over, the journeys to rebuild listed (the slot then waits one step in
 // S_RECON), the next start-time group seeded, and the slot's views for the
 // next step (lane record, the group's run mask and, per round, its slots to
@@ -1666,7 +1708,12 @@ __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
       auto const k = static_cast<uint8_t>(sl.k + 1u);
       __syncwarp();
       if (lane == 0u) sl.k = k;
-      if (k >= sl.end_k) state = S_COLLECT;
+      if (k >= sl.end_k) {
+        state = S_COLLECT;
+      } else if (((st.made_mask[g] >> (s & 31u)) & 1u) == 0u) {
+        empty_round(st, sl, s, k, lane);
+        state = S_COLLECT;
+      }
     }
     if (state == S_COLLECT) {
       if (!sl.one_to_all && !collect_slot(st, sl, s, lane)) {
