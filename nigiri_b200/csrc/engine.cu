@@ -256,7 +256,7 @@ struct adm_hdr {
   uint32_t slot;
   uint32_t n_starts, n_dest, n_off;
   uint32_t clear_rt;
-  uint32_t lb_mode;  // 0 zeros, 1 column in payload, 2 solved on the device, 3 from the table,
+  uint32_t lb_mode;  // 0 none (the slot's no_lb), 1 column in payload, 2 solved on the device, 3 from the table,
                      // 4 kept (the column of the query's previous phase)
   uint32_t n_seeds;
   uint32_t flags;
@@ -301,10 +301,8 @@ __global__ void k_admit(dev::state st, adm_hdr const* hdr, uint8_t const* payloa
   auto const* offs = reinterpret_cast<b2r_offset const*>(payload + h.off_off);
   for (auto i = threadIdx.x; i < h.n_off; i += blockDim.x) st.off_pool[s * max_off + i] = offs[i];
   auto const* lbc = reinterpret_cast<uint16_t const*>(payload + h.off_lb);
-  if (h.lb_mode < 2) {
-    for (auto l = threadIdx.x; l < n_loc; l += blockDim.x) {
-      st.lb[static_cast<size_t>(l) * st.S + s] = h.lb_mode ? lbc[l] : uint16_t{0};
-    }
+  if (h.lb_mode == 1) {
+    for (auto l = threadIdx.x; l < n_loc; l += blockDim.x) st.lb[static_cast<size_t>(l) * st.S + s] = lbc[l];
   }
   if (h.clear_rt) {  // query generations wrapped: no stale tag may survive
     for (size_t i = threadIdx.x; i < static_cast<size_t>(dev::kK) * n_loc; i += blockDim.x) {
@@ -735,6 +733,12 @@ int check_capacity(b2r_engine const& e, prepped_query const& p) {
   return B2R_OK;
 }
 
+// whether the query runs without lower bounds: its slot says so and no
+// kernel reads its column
+bool without_lb(b2r_engine const& e, prepped_query const& p) {
+  return p.lb.empty() && (p.one_to_all || (e.lb_mode() != 2 && e.lb_mode() != 3));
+}
+
 // new_gen: a new query generation (raptor::reset_arrivals); otherwise the
 // round times of the slot's previous phase stay in effect
 slot_t make_slot(b2r_engine& e, uint32_t s, prepped_query const& p, bool& clear_rt, bool new_gen = true) {
@@ -776,7 +780,7 @@ slot_t make_slot(b2r_engine& e, uint32_t s, prepped_query const& p, bool& clear_
   // the slot is done and be rebuilt while the next super-steps run
   sl.recon_defer = (p.ontrip && !p.one_to_all && p.recon_mode == 0) ? 1 : 0;
   sl.recon_transfers = p.recon_transfers;
-  sl.no_lb = p.no_lb ? 1 : 0;
+  sl.no_lb = p.no_lb || without_lb(e, p) ? 1 : 0;
   sl.prf = p.prf;
   sl.recon_start = p.recon_start;
   sl.span = p.span;
@@ -955,12 +959,11 @@ void admit(b2r_engine& e, std::vector<adm_req> const& adm, cudaStream_t s) {
     offs.insert(offs.end(), p.dest_offsets.begin(), p.dest_offsets.end());
     h.n_off = static_cast<uint32_t>(offs.size());
     h.off_off = put(offs.data(), offs.size() * sizeof(b2r_offset));
-    h.lb_mode = p.keep_lb          ? 4
-                : !p.lb.empty()      ? 1
-                : p.one_to_all       ? 0
-                : e.lb_mode() == 2 ? 2
-                : e.lb_mode() == 3 ? 3
-                                              : 0;
+    h.lb_mode = p.keep_lb && !without_lb(e, p) ? 4
+                : without_lb(e, p)             ? 0
+                : !p.lb.empty()                ? 1
+                : e.lb_mode() == 2             ? 2
+                                               : 3;
     h.off_lb = put(p.lb.data(), p.lb.size() * sizeof(uint16_t));
     std::vector<uint32_t> seeds;
     for (auto const& [l, d] : p.lb_seeds) {

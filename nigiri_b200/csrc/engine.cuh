@@ -183,7 +183,7 @@ struct slot_t {
   uint8_t recon_mode;        // 0: new journeys of the interval, 1: only the journey
                              // (recon_transfers, recon_start), 2: none
   uint8_t recon_transfers;
-  uint8_t no_lb;             // lower bounds read as 0 (a pong phase)
+  uint8_t no_lb;             // lower bounds read as 0 (a pong phase, a query without bounds)
   uint8_t prf;               // footpath profile (query::prf_idx_)
   int16_t span;              // worst time at destination = group start + dir(span)
   int32_t recon_start;
