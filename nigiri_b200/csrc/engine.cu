@@ -172,7 +172,7 @@ struct b2r_engine {
   std::vector<int64_t> slot_query;  // query index in the current batch, -1 free
   using summary_t = b2r::dev::slot_summary;
   summary_t* d_summary{nullptr};
-  summary_t* h_summary{nullptr};  // pinned
+  summary_t* h_summary{nullptr};  // pinned, [2][S]: the batch loop's chunks in flight by turns
   uint32_t* h_lbcount{nullptr};   // pinned
   uint64_t lb_chunks{0};
   double lb_ms{0};
@@ -195,7 +195,8 @@ struct b2r_engine {
   uint32_t* d_exp_list{nullptr};
 
   b2r_batch_stats last{};
-  cudaEvent_t ev0{nullptr}, ev1{nullptr};
+  cudaEvent_t ev0[2]{nullptr, nullptr}, ev1[2]{nullptr, nullptr};  // a chunk's begin and end
+  cudaEvent_t ev_sum[2]{nullptr, nullptr};                         // its summary is on the host
   // device busy time of a batch: the intervals (ms after ev_base) in which
   // super-step chunks (main stream) and finished-slot work (reconstruction
   // and export kernels, second stream) ran; their union is the batch's
@@ -563,8 +564,8 @@ b2r_engine::~b2r_engine() {
   if (stream_recon != nullptr) cudaStreamDestroy(stream_recon);
   if (ev_fork != nullptr) cudaEventDestroy(ev_fork);
   if (ev_join != nullptr) cudaEventDestroy(ev_join);
-  if (ev0 != nullptr) cudaEventDestroy(ev0);
-  if (ev1 != nullptr) cudaEventDestroy(ev1);
+  for (auto* ev : {ev0[0], ev0[1], ev1[0], ev1[1], ev_sum[0], ev_sum[1]})
+    if (ev != nullptr) cudaEventDestroy(ev);
   if (ev_base != nullptr) cudaEventDestroy(ev_base);
   if (ev_scan_a != nullptr) cudaEventDestroy(ev_scan_a);
   if (ev_scan_b != nullptr) cudaEventDestroy(ev_scan_b);
@@ -1799,7 +1800,8 @@ struct batch_runner {
     std::vector<uint8_t> held(S, 0);   // finished, export held back (below)
     std::vector<uint32_t> held_nj(S, 0), held_list;
     std::vector<b2r_engine::summary_t> sum(S);
-    bool in_flight = false;
+    uint32_t in_flight = 0;                  // chunks launched whose summary has not been read
+    uint32_t n_launched = 0, n_read = 0;     // chunks; their buffers and events by turns
     auto const running = [&]() {
       for (auto x : slot_q)
         if (x >= 0) return true;
@@ -1807,17 +1809,37 @@ struct batch_runner {
     };
     auto const busy = [&]() { return next < runs.size() || running(); };
     auto const launch_chunk = [&](uint32_t n_steps) {
-      B2R_CUDA(cudaEventRecord(e.ev0, st));
+      auto const turn = n_launched++ & 1U;
+      B2R_CUDA(cudaEventRecord(e.ev0[turn], st));
       auto recon = false;
       for (auto const x : slot_q) recon = recon || (x >= 0 && rebuilds_between_groups(runs[static_cast<size_t>(x)].p));
       run_supersteps(e, st, use_graph, recon, n_steps);
       launches += n_steps * launches_per_step(e, recon);
       steps += n_steps;
-      B2R_CUDA(cudaEventRecord(e.ev1, st));
+      B2R_CUDA(cudaEventRecord(e.ev1[turn], st));
       e.d2h_bytes += S * sizeof(b2r_engine::summary_t);
-      B2R_CUDA(cudaMemcpyAsync(e.h_summary, e.d_summary, S * sizeof(b2r_engine::summary_t),
+      B2R_CUDA(cudaMemcpyAsync(e.h_summary + turn * S, e.d_summary, S * sizeof(b2r_engine::summary_t),
                                cudaMemcpyDeviceToHost, st));
-      in_flight = true;
+      B2R_CUDA(cudaEventRecord(e.ev_sum[turn], st));
+      ++in_flight;
+    };
+    // Range queries run for dozens of chunks that the host has nothing to
+    // put between: while no query waits for a slot, one more chunk is
+    // launched before the last one's summary is read, so that the device
+    // does not wait for the host at every chunk (about 20 us each).  What the
+    // host queues after reading a summary then runs behind the chunk in
+    // flight and ahead of the one launched next, as without it.  Not with
+    // pong queries resident, whose next phase the host stages.
+    auto const ahead = [&]() {
+      if (!use_graph || e.cfg.profile != 0U || next < runs.size()) return false;
+      auto ranges = false;
+      for (auto const x : slot_q) {
+        if (x < 0) continue;
+        auto const& p = runs[static_cast<size_t>(x)].p;
+        if (p.pong) return false;
+        ranges = ranges || rebuilds_between_groups(p);
+      }
+      return ranges;
     };
     // every start-time group ends within end_k super-steps; the cap turns a
     // logic error into a reported failure instead of an endless loop
@@ -1841,12 +1863,14 @@ struct batch_runner {
         }
         launch_chunk(chunk);
       }
-      B2R_CUDA(cudaStreamSynchronize(st));
-      in_flight = false;
+      if (in_flight < 2U && ahead()) launch_chunk(chunk);
+      auto const turn = n_read++ & 1U;
+      B2R_CUDA(cudaEventSynchronize(e.ev_sum[turn]));
+      --in_flight;
       {
         float a = 0, b = 0;
-        B2R_CUDA(cudaEventElapsedTime(&a, e.ev_base, e.ev0));
-        B2R_CUDA(cudaEventElapsedTime(&b, e.ev_base, e.ev1));
+        B2R_CUDA(cudaEventElapsedTime(&a, e.ev_base, e.ev0[turn]));
+        B2R_CUDA(cudaEventElapsedTime(&b, e.ev_base, e.ev1[turn]));
         e.busy.emplace_back(a, b);
         if (e.cfg.profile == 2U) {  // one super-step per chunk: its route phase
           B2R_CUDA(cudaEventElapsedTime(&a, e.ev_scan_a, e.ev_scan_b));
@@ -1854,7 +1878,7 @@ struct batch_runner {
           ++e.scan_launches;
         }
       }
-      std::copy(e.h_summary, e.h_summary + S, sum.begin());
+      std::copy(e.h_summary + turn * S, e.h_summary + (turn + 1U) * S, sum.begin());
       for (auto& x : slot_q)
         if (x == kRetiring) x = -1;  // their retirement ran before this summary's chunk ended
       std::vector<uint32_t> done_slots, n_js, n_rows;
@@ -1915,7 +1939,7 @@ struct batch_runner {
       // it instead of leaving the slot idle for a whole chunk
       auto phase_follows = false;
       for (auto const s : done_slots) phase_follows = phase_follows || runs[static_cast<size_t>(slot_q[s])].p.pong;
-      if (!phase_follows && running() && others_run) launch_chunk(chunk);
+      if (in_flight == 0 && !phase_follows && running() && others_run) launch_chunk(chunk);
       if (done_slots.empty()) continue;
       auto const t_exp = std::chrono::steady_clock::now();
       std::vector<exported> ex;
@@ -1980,9 +2004,14 @@ struct preparer {
   void start(b2r_engine& e, b2r_query const* qs, uint32_t n, std::vector<query_run>& runs,
              bool inline_all) {
     auto const hw = std::max(1U, std::thread::hardware_concurrency());
-    auto const n_threads = std::max(1U, std::min<uint32_t>(
-        e.cfg.host_threads != 0 ? e.cfg.host_threads : (hw > 1 ? hw - 1 : 1), n));
     auto const lb_mode = e.lb_mode();
+    // A query's preparation takes a few microseconds, starting a thread some
+    // dozens: 16 queries a thread, unless the lower bounds are a Dijkstra on
+    // the host (about a millisecond)
+    auto dijkstra = lb_mode == 1;
+    for (auto i = 0U; i != n && !dijkstra; ++i) dijkstra = qs[i].prf_idx != 0U;
+    auto const n_threads = std::max(1U, std::min<uint32_t>(
+        e.cfg.host_threads != 0 ? e.cfg.host_threads : (hw > 1 ? hw - 1 : 1), dijkstra ? n : (n + 15U) / 16U));
     auto work = [&e, qs, n, &runs, lb_mode, this]() {
       for (auto i = next++; i < n; i = next++) {
         auto const t0 = std::chrono::steady_clock::now();
@@ -2739,15 +2768,18 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       B2R_CUDA(cudaMemset(st.counters, 0, 16 * 4));
       e->gen_query.assign(S, 0);
       e->slot_query.assign(S, -1);
-      B2R_CUDA(cudaMallocHost(&e->h_summary, S * sizeof(b2r_engine::summary_t)));
+      B2R_CUDA(cudaMallocHost(&e->h_summary, 2 * S * sizeof(b2r_engine::summary_t)));
       B2R_CUDA(cudaMallocHost(&e->h_lbcount, sizeof(uint32_t)));
       B2R_CUDA(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
       B2R_CUDA(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
       B2R_CUDA(cudaStreamCreateWithFlags(&e->stream_recon, cudaStreamNonBlocking));
       B2R_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
       B2R_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
-      B2R_CUDA(cudaEventCreate(&e->ev0));
-      B2R_CUDA(cudaEventCreate(&e->ev1));
+      for (auto i = 0; i != 2; ++i) {
+        B2R_CUDA(cudaEventCreate(&e->ev0[i]));
+        B2R_CUDA(cudaEventCreate(&e->ev1[i]));
+        B2R_CUDA(cudaEventCreateWithFlags(&e->ev_sum[i], cudaEventDisableTiming));
+      }
       B2R_CUDA(cudaEventCreate(&e->ev_base));
       B2R_CUDA(cudaEventCreate(&e->ev_scan_a));
       B2R_CUDA(cudaEventCreate(&e->ev_scan_b));
@@ -2803,7 +2835,7 @@ int b2r_search_batch(b2r_engine* e, const b2r_query* qs, uint32_t n, b2r_result*
       e->prep_ns = 0;
       e->admit_ms = e->export_ms = e->idle_ms = 0;
       b2r::preparer prep;
-      prep.start(*e, qs, n, runs, false);
+      prep.start(*e, qs, n, runs, n == 1U);
       b2r::batch_runner br{*e, runs, e->cfg.use_graphs != 0 && e->graph[0] != nullptr};
       if (e->cfg.profile) B2R_CUDA(cudaMemsetAsync(e->st.prof, 0, 8 * sizeof(unsigned long long), e->stream));
       e->scan_ms = 0;
