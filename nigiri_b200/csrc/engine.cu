@@ -724,7 +724,8 @@ size_t admission_bytes(b2r_engine const& e, prepped_query const& p) {
   return sizeof(slot_t) + p.starts.size() * sizeof(dev::start_rec) +
          (p.dest_dist.size() + p.dest_locs.size()) * sizeof(dev::dest_rec) +
          (p.start_offsets.size() + p.dest_offsets.size()) * sizeof(b2r_offset) +
-         (p.lb.empty() ? 0 : e.tt->d.n_loc * sizeof(uint16_t)) + 64;
+         (p.lb.empty() ? 0 : e.tt->d.n_loc * sizeof(uint16_t)) + p.lb_seeds.size() * 2 * sizeof(uint32_t) +
+         128;  // 16-byte alignment of eight parts
 }
 
 int check_capacity(b2r_engine const& e, prepped_query const& p) {
