@@ -506,12 +506,11 @@ __global__ void __launch_bounds__(256) k_routes(state st) {
 //
 // Here 8 lanes take one pair, a warp four pairs, 32 stops at a time (32
 // lanes and one pair where there are few, kFewPerSm):
-// * the lanes read the stops' marks, four stops each, and for the marked
-//   boardable ones the label to board from; those that time_at_dest does
-//   not rule out are the searches;
-// * the searches of the four pairs are numbered through and the warp's
-//   lanes take 32 of them at once (a search depends only on its stop's
-//   labels; what it needs of its pair lies in shared memory);
+// * the lanes read the stops' marks, four stops each;
+// * the marked boardable stops of the four pairs are numbered through, and
+//   the warp's lanes take 32 of them at once: the label to board from and,
+//   unless time_at_dest rules it out, the search (it depends only on its
+//   stop's labels; what it needs of its pair lies in shared memory);
 // * on a route whose trips keep one order at every event
 //   (b2r_timetable: route_fifo), "switch when at least as good at this
 //   stop" is "keep the best trip so far", whatever stop compares them (on a
@@ -666,16 +665,16 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
 template <uint32_t kTile>
 struct scan_smem {  // of a warp
   static constexpr uint32_t kPer = 32u / kTile;
-  uint4 pair[kPer][4];      // route record (2), lane record, {first stop of the 32, 0, 0, 0}
-  uint32_t key[kPer][32];   // per stop: what its search needs (previous label, bound), then the
-                            // candidate (order key << 6 | stop), kNone without one
+  uint4 pair[kPer][4];      // route record (2), lane record, {first stop of the 32, slot, 0, 0}
+  uint32_t key[kPer][32];   // per stop: its location, then the candidate (order key << 6 | stop),
+                            // kNone without one, kShut where the query cannot go on from
   uint2 trip[kPer][33];     // per stop: the candidate's offset and day; 32: the trip carried in
 };
 template <uint32_t kTile, bool Prof>
 __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm, uint32_t nr, scan_ctr& pc) {
   constexpr uint32_t kPer = 32u / kTile;  // stops a lane takes of each 32; pairs of a warp
   constexpr uint32_t kTileBits = kTile == 32u ? kFull : (1u << (kTile % 32u)) - 1u;
-  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  constexpr uint32_t kNone = 0xFFFFFFFFu, kShut = 0xFFFFFFFEu;
   constexpr uint32_t kCarried = 32u;
   auto const& T = st.tt;
   auto const lane = threadIdx.x & 31u;
@@ -732,9 +731,9 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
     auto const bit = 1u << (s & 31u);
     auto const lb_off = (ln.mode & 8u) != 0u;
     auto const n_blk = have ? min(32u, R.n - i0) : 0u;
-    // the block's stop words, marks and boarding labels
+    // the block's stop words and its marked boardable stops
     uint32_t sw[kPer];
-    bool marked[kPer];
+    uint32_t m = 0, cuts = 0;
 #pragma unroll
     for (auto c = 0u; c != kPer; ++c) {
       auto const p = c * kTile + tl;
@@ -743,41 +742,14 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
 #pragma unroll
     for (auto c = 0u; c != kPer; ++c) {
       auto const p = c * kTile + tl;
-      marked[c] = p < n_blk && i0 + p + 1u != R.n && (fwd ? B2R_STOP_IN(sw[c]) : B2R_STOP_OUT(sw[c])) != 0u &&
-                  (X[B2R_STOP_LOC(sw[c]) * st.G + g] & bit) != 0u;
+      auto const board = p < n_blk && i0 + p + 1u != R.n && (fwd ? B2R_STOP_IN(sw[c]) : B2R_STOP_OUT(sw[c])) != 0u;
+      m |= tile_bits(board && (X[B2R_STOP_LOC(sw[c]) * st.G + g] & bit) != 0u) << (c * kTile);
+      sm.key[tile][p] = B2R_STOP_LOC(sw[c]);
     }
-    uint32_t m = 0, closed = 0, cuts = 0;
-#pragma unroll
-    for (auto c = 0u; c != kPer; ++c) {
-      uint32_t label = kNone;
-      bool shut = false;
-      if (marked[c]) {
-        auto const at = li(st, B2R_STOP_LOC(sw[c]), s);
-        auto const lbv = lb_off ? uint16_t{0} : st.lb[at];
-        auto const prt = dec(st.rt[static_cast<size_t>(ln.k - 1u) * T.n_loc * st.S + at], ln.qtag);
-        // a marked station always carries a best label of its start time
-        // (marks come with best updates), so the boarding rule never meets
-        // an invalid current_best; were it to, the query is failed loudly
-        if (prt != kKeyInv && dec(st.best[at], ln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
-        shut = lbv == 0xFFFFu;
-        // every event of the search is at or after prt: pruned with it
-        if (!shut && prt != kKeyInv && prt + static_cast<int>(lbv) <= ln.tad_k) {
-          label = (static_cast<uint32_t>(static_cast<uint16_t>(prt)) << 16) | lbv;
-        }
-      }
-      sm.key[tile][c * kTile + tl] = label;
-      m |= tile_bits(label != kNone) << (c * kTile);
-      closed |= tile_bits(shut) << (c * kTile);
-    }
-    // raptor.h:1309-1311: the walk ends at the first boardable stop the
-    // query cannot reach, after that stop's arrival
-    auto const ends = closed != 0u;
-    auto const first_closed = static_cast<uint32_t>(__ffs(closed) - 1);
-    if (ends) m &= (1u << first_closed) - 1u;
-    auto const limit = ends ? first_closed + 1u : n_blk;
+    bool ends = false;
     if constexpr (Prof) {
       if (lane == 0u) ++pc.warp_steps;
-      if (tl == 0u) pc.stops += limit;
+      if (tl == 0u) pc.stops += n_blk;
     }
     if (__any_sync(kFull, m != 0u || carry != kNone)) {
       if (__any_sync(kFull, have && (sec & 15u) != 0u)) {
@@ -793,7 +765,7 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
         sm.pair[tile][0] = uint4{R.sb, R.n, R.st, R.t0};
         sm.pair[tile][1] = uint4{R.n_t, R.bf, R.flags, R.filter};
         sm.pair[tile][2] = *reinterpret_cast<uint4 const*>(&ln);
-        sm.pair[tile][3] = uint4{i0, 0u, 0u, 0u};
+        sm.pair[tile][3] = uint4{i0, s, 0u, 0u};
       }
       __syncwarp();
       auto const cnt = static_cast<uint32_t>(__popc(m));
@@ -821,13 +793,20 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
           auto const oln = *reinterpret_cast<lane_t const*>(&c);
           auto const ofwd = oln.fwd != 0;
           auto const i = sm.pair[o][3].x + pos;
-          auto const label = sm.key[o][pos];
-          auto const prt = static_cast<int>(static_cast<int16_t>(label >> 16));
+          auto const at = li(st, sm.key[o][pos], sm.pair[o][3].y);
+          auto const lbv = (oln.mode & 8u) ? uint16_t{0} : st.lb[at];
+          auto const prt = dec(st.rt[static_cast<size_t>(oln.k - 1u) * T.n_loc * st.S + at], oln.qtag);
+          // a marked station always carries a best label of its start time
+          // (marks come with best updates), so the boarding rule never meets
+          // an invalid current_best; were it to, the query is failed loudly
+          if (prt != kKeyInv && dec(st.best[at], oln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
           auto const minutes = static_cast<int>(oln.base) * 1440 + from_key(ofwd, prt);
-          uint32_t nt = 0, v = kNone, n_ev = 0, n_days = 0;
+          uint32_t nt = 0, v = lbv == 0xFFFFu ? kShut : kNone, n_ev = 0, n_days = 0;
           uint16_t nd = 0;
-          if (et_search(T, ofwd, oR, ofwd ? i : oR.n - 1u - i, static_cast<uint16_t>(minutes / 1440), minutes % 1440,
-                        static_cast<int>(label & 0xFFFFu), oln.tad_k, oln.base, nt, nd, n_ev, n_days)) {
+          // every event of the search is at or after prt: pruned with it
+          if (lbv != 0xFFFFu && prt != kKeyInv && prt + static_cast<int>(lbv) <= oln.tad_k &&
+              et_search(T, ofwd, oR, ofwd ? i : oR.n - 1u - i, static_cast<uint16_t>(minutes / 1440), minutes % 1440,
+                        static_cast<int>(lbv), oln.tad_k, oln.base, nt, nd, n_ev, n_days)) {
             uint32_t key;
             if ((oR.flags & 2u) != 0u) {
               auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(oln.base) + 64) * oR.n_t + nt;
@@ -851,11 +830,14 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
       // the trip each stop is reached by: the minimum over the stops before
       // it, from the last cut on
       uint32_t by[kPer];
+      uint32_t closed = 0;  // boardable stops the query cannot reach
       auto run = carry;
 #pragma unroll
       for (auto c = 0u; c != kPer; ++c) {
         auto const cc = (cuts >> (c * kTile)) & kTileBits;
         auto v = ((m >> (c * kTile + tl)) & 1u) != 0u ? sm.key[tile][c * kTile + tl] : kNone;
+        closed |= tile_bits(v == kShut) << (c * kTile);
+        if (v == kShut) v = kNone;
 #pragma unroll
         for (auto o = 1u; o < kTile; o <<= 1) {
           auto const y = __shfl_up_sync(kFull, v, o, kTile);
@@ -866,6 +848,13 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
         by[c] = (cc & ((2u << tl) - 1u)) == 0u ? min(before, run) : before;
         auto const last = tile_shfl(v, kTile - 1u);
         run = cc == 0u ? min(run, last) : last;
+      }
+      // raptor.h:1309-1311: the walk ends at the first boardable stop the
+      // query cannot reach, after that stop's arrival
+      ends = closed != 0u;
+      auto const limit = ends ? static_cast<uint32_t>(__ffs(closed)) : n_blk;
+      if constexpr (Prof) {
+        if (tl == 0u) pc.stops -= n_blk - limit;
       }
       // arrivals (raptor.h:1219-1302)
       uint16_t ev[kPer], lbs[kPer], day[kPer];
