@@ -359,7 +359,7 @@ __global__ void k_admit(dev::state st, adm_hdr const* hdr, uint8_t const* payloa
 // table rows -- every path of length <= kMaxTravelTime only passes
 // locations closer than that, so min(seed distance + row) is the capped
 // multi-source distance.  blockIdx.y = slot group, blockIdx.x = a tile of
-// 128 locations: the tile's values are computed with the threads over
+// 256 locations: the tile's values are computed with the threads over
 // locations (table rows read in order) and written with a warp over the
 // group's slots per location, 64 contiguous bytes of lb.
 struct lb_group {
@@ -369,7 +369,7 @@ struct lb_entry {
   uint32_t lane, n_seeds, fwd, pad;
   uint64_t off_seeds;
 };
-constexpr uint32_t kLbTile = 128;
+constexpr uint32_t kLbTile = 256;
 
 __global__ void k_lb_fill(dev::state st, lb_group const* groups, lb_entry const* entries,
                           uint8_t const* payload) {
@@ -378,31 +378,54 @@ __global__ void k_lb_fill(dev::state st, lb_group const* groups, lb_entry const*
   auto const stride = st.lb_stride;  // table row length, a multiple of 8
   auto const x0 = blockIdx.x * kLbTile;
   // work items (entry, chunk of 8 locations): one 16-byte table load per
-  // seed and chunk, eight running minima
+  // seed and chunk, four seeds' loads in flight, the eight running minima
+  // packed two to a word
   constexpr uint32_t kChunks = kLbTile / 8u;
   for (auto item = threadIdx.x; item < grp.count * kChunks; item += blockDim.x) {
     auto const e = item / kChunks, ch = item % kChunks;
     auto const xc = x0 + ch * 8u;
-    uint32_t best[8];
-    for (auto j = 0u; j != 8u; ++j) best[j] = 0xFFFFu;
+    uint32_t best[4];  // eight minima, two to a word
+    for (auto& x : best) x = 0xFFFFFFFFu;
     if (xc < stride) {  // the chunk lies inside the row (stride % 8 == 0)
       auto const en = entries[grp.first + e];
-      auto const* seeds = reinterpret_cast<uint32_t const*>(payload + en.off_seeds);
-      auto const* tab = en.fwd ? st.lb_table_fwd : st.lb_table_bwd;
-      for (auto i = 0u; i != en.n_seeds; ++i) {
-        auto const m = seeds[2 * i];
-        auto const sd = seeds[2 * i + 1];
-        auto const v = *reinterpret_cast<uint4 const*>(tab + static_cast<size_t>(m) * stride + xc);
-        uint32_t const w[4] = {v.x, v.y, v.z, v.w};
-        for (auto j = 0u; j != 8u; ++j) {
-          auto const d = (w[j >> 1] >> (16u * (j & 1u))) & 0xFFFFu;
-          if (d == 0xFFFFu) continue;
-          auto const c = sd + d;
-          if ((c <= B2R_MAX_TRAVEL_TIME_MIN || xc + j == m) && c < best[j]) best[j] = c;
+      auto const* seeds = reinterpret_cast<uint2 const*>(payload + en.off_seeds);
+      auto const* tab = (en.fwd ? st.lb_table_fwd : st.lb_table_bwd) + xc;
+      constexpr uint32_t kMost = B2R_MAX_TRAVEL_TIME_MIN | (B2R_MAX_TRAVEL_TIME_MIN << 16);
+      for (auto i0 = 0u; i0 < en.n_seeds; i0 += 4u) {
+        uint2 sd[4];
+        uint4 v[4];
+#pragma unroll
+        for (auto x = 0u; x != 4u; ++x) sd[x] = i0 + x < en.n_seeds ? seeds[i0 + x] : uint2{0xFFFFFFFFu, 0u};
+#pragma unroll
+        for (auto x = 0u; x != 4u; ++x) {
+          if (i0 + x < en.n_seeds) v[x] = *reinterpret_cast<uint4 const*>(tab + static_cast<size_t>(sd[x].x) * stride);
+        }
+#pragma unroll
+        for (auto x = 0u; x != 4u; ++x) {
+          if (i0 + x >= en.n_seeds) continue;
+          auto const add = min(sd[x].y, 0xFFFFu) * 0x10001u;
+          uint32_t const w[4] = {v[x].x, v[x].y, v[x].z, v[x].w};
+#pragma unroll
+          for (auto j = 0u; j != 4u; ++j) {
+            // saturating: unreachable (0xFFFF) stays so; beyond the travel
+            // time is unreachable
+            auto const c = __vaddus2(w[j], add);
+            best[j] = __vminu2(best[j], c | __vcmpgtu2(c, kMost));
+          }
+          // a seed farther than the travel time still bounds its own location
+          auto const own = sd[x].x - xc;
+          if (sd[x].y > B2R_MAX_TRAVEL_TIME_MIN && own < 8u) {
+            auto const bits = 16u * (own & 1u);
+            best[own >> 1] = __vminu2(best[own >> 1], (0xFFFFFFFFu & ~(0xFFFFu << bits)) | (min(sd[x].y, 0xFFFFu) << bits));
+          }
         }
       }
     }
-    for (auto j = 0u; j != 8u; ++j) tile[e][ch * 8u + j] = static_cast<uint16_t>(best[j]);
+#pragma unroll
+    for (auto j = 0u; j != 4u; ++j) {
+      tile[e][ch * 8u + 2u * j] = static_cast<uint16_t>(best[j]);
+      tile[e][ch * 8u + 2u * j + 1u] = static_cast<uint16_t>(best[j] >> 16);
+    }
   }
   __syncthreads();
   auto const n_loc = st.tt.n_loc;

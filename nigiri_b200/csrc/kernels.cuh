@@ -895,8 +895,10 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
 
 // Above this many entries per SM the scan takes 8 lanes per pair, else a
 // warp: a step of a warp is about 1,500 instructions for four pairs and 700
-// for one, so with warps to spare one pair ends sooner.
-constexpr uint32_t kFewPerSm = 32;
+// for one, so with warps to spare one pair ends sooner.  12, 32 and 96 took
+// 29.1, 28.9 and 28.7 ms for 96 range queries and 38.1, 37.9 and 37.7 ms for
+// the national mix of 256.
+constexpr uint32_t kFewPerSm = 96;
 
 // Builds with four, five or six blocks of 256 threads resident per SM (the
 // launch shape picks one), and with work counters for profiling engines
