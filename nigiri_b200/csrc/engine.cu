@@ -1650,7 +1650,7 @@ void phase_done(b2r_engine& e, query_run& q, exported& x) {
 
 // ------------------------------------------------------------- the loop
 // Free slots for admission.  Range queries run several start-time groups and
-// so sweep their round times every round (k_sweep); they take slots from the
+// so sweep their round times every round (k_mark); they take slots from the
 // top of the pool, all other queries from the bottom, so that the sweeping
 // slots share slot groups.
 template <typename Free>

@@ -748,7 +748,7 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
     }
     bool ends = false;
     if constexpr (Prof) {
-      if (lane == 0u) ++pc.warp_steps;
+      if (lane == 0u) pc.warp_steps += kPer;  // 32 stops of each of its pairs
       if (tl == 0u) pc.stops += n_blk;
     }
     if (__any_sync(kFull, m != 0u || carry != kNone)) {
@@ -796,10 +796,7 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
           auto const at = li(st, sm.key[o][pos], sm.pair[o][3].y);
           auto const lbv = (oln.mode & 8u) ? uint16_t{0} : st.lb[at];
           auto const prt = dec(st.rt[static_cast<size_t>(oln.k - 1u) * T.n_loc * st.S + at], oln.qtag);
-          // a marked station always carries a best label of its start time
-          // (marks come with best updates), so the boarding rule never meets
-          // an invalid current_best; were it to, the query is failed loudly
-          if (prt != kKeyInv && dec(st.best[at], oln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
+          auto const has_best = dec(st.best[at], oln.gtag) != kKeyInv;
           auto const minutes = static_cast<int>(oln.base) * 1440 + from_key(ofwd, prt);
           uint32_t nt = 0, v = lbv == 0xFFFFu ? kShut : kNone, n_ev = 0, n_days = 0;
           uint16_t nd = 0;
@@ -807,6 +804,10 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
           if (lbv != 0xFFFFu && prt != kKeyInv && prt + static_cast<int>(lbv) <= oln.tad_k &&
               et_search(T, ofwd, oR, ofwd ? i : oR.n - 1u - i, static_cast<uint16_t>(minutes / 1440), minutes % 1440,
                         static_cast<int>(lbv), oln.tad_k, oln.base, nt, nd, n_ev, n_days)) {
+            // a marked station always carries a best label of its start time
+            // (marks come with best updates), so the boarding rule never meets
+            // an invalid current_best; were it to, the query is failed loudly
+            if (!has_best && dec(st.tmp[at], oln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
             uint32_t key;
             if ((oR.flags & 2u) != 0u) {
               auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(oln.base) + 64) * oR.n_t + nt;
