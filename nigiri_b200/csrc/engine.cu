@@ -2736,7 +2736,7 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.R, static_cast<size_t>(tt->d.n_routes) * G);
       al(st.D, static_cast<size_t>(nl) * G);
       al(st.ylist, static_cast<size_t>(nl) * G);
-      al(st.rlist, static_cast<size_t>(tt->d.n_routes) * G);
+      al(st.rlist, static_cast<size_t>(tt->d.n_routes) * G * (32U / b2r::dev::kEntryMarks));
       al(st.counters, 16);
       al(st.run_mask, G);
       al(st.sweep_k, G * b2r::dev::kK);

@@ -25,6 +25,14 @@ constexpr int kKeyInv = 32767;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kMaxLegs = 40;
 constexpr int kMaxTimeline = 128;
+// The most queries of a route scan's entry; a (route, group) word with more is
+// listed as several.  A tile takes an entry's queries one after the other, so
+// where all of a small network's routes are marked by most queries (1,009
+// stops, 1,000 queries: 20 of 32) an entry of a whole word is 20 pairs long,
+// and 21,000 of them on 18,944 resident tiles are one wave and a ninth: 1.94
+// ms for that batch, 1.75 with 8 and 1.57 with 4.  Where words hold one or two
+// marks (40,009 stops) the limit costs nothing.
+constexpr uint32_t kEntryMarks = 4;
 constexpr uint32_t kMaxGroups = 2048;  // slot groups: a slot index has 16 bits (recon_list)
 
 // lrs_stop bits above the position: a ride can end (forward) or begin
@@ -268,7 +276,7 @@ struct state {
   uint32_t* rtlist; // frontier list of (rt transport * G + g)
   uint32_t* D;      // is-destination bits [n_loc][G]
   uint32_t* ylist;  // frontier lists of (loc * G + g)
-  uint4* rlist;     // {route, group, its marks, 0}
+  uint2* rlist;     // {route * G + group, up to kEntryMarks of its marks}
   uint32_t* counters;  // C_*: list lengths, mark parity, error bits
   uint32_t* run_mask;  // [G]
   uint32_t* sweep_k;   // [G][K] slots to sweep that are at round k

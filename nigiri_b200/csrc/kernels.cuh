@@ -382,13 +382,13 @@ __global__ void __launch_bounds__(256) k_mark(state st) {
 }
 
 // The non-zero words of W[0, n) listed in no particular order: emit(at, i,
-// word).  Each thread reads 4 words with one 16-byte load (W comes from
+// word) fills the items(word) places from `at` on.  Each thread reads 4 words with one 16-byte load (W comes from
 // cudaMalloc and i is a multiple of 4), the block scans the counts and
 // reserves its range with one atomicAdd per 4 * blockDim words.
 // Block `block` of `n_blocks`.
-template <typename Emit>
+template <typename Items, typename Emit>
 __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W, uint32_t n, uint32_t counter,
-                                             uint32_t block, uint32_t n_blocks, Emit&& emit) {
+                                             uint32_t block, uint32_t n_blocks, Items&& items, Emit&& emit) {
   __shared__ uint32_t warp_off[32];
   __shared__ uint32_t base;
   auto const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
@@ -405,8 +405,7 @@ __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W,
     } else {
       for (auto j = 0u; j != 4u; ++j) w[j] = i + j < n ? W[i + j] : 0u;
     }
-    auto const cnt = static_cast<uint32_t>(w[0] != 0u) + static_cast<uint32_t>(w[1] != 0u) +
-                     static_cast<uint32_t>(w[2] != 0u) + static_cast<uint32_t>(w[3] != 0u);
+    auto const cnt = items(w[0]) + items(w[1]) + items(w[2]) + items(w[3]);
     auto incl = cnt;  // inclusive scan over the warp
     for (auto d = 1u; d < 32u; d <<= 1) {
       auto const y = __shfl_up_sync(kFull, incl, d);
@@ -427,11 +426,18 @@ __device__ __forceinline__ void list_nonzero(state const& st, uint32_t const* W,
     __syncthreads();
     auto at = base + warp_off[warp] + (incl - cnt);
     for (auto j = 0u; j != 4u; ++j) {
-      if (w[j] != 0u) emit(at++, i + j, w[j]);
+      if (w[j] != 0u) {
+        emit(at, i + j, w[j]);
+        at += items(w[j]);
+      }
     }
     __syncthreads();  // warp_off and base are reused by the next pass
   }
 }
+
+struct one_item {
+  __device__ __forceinline__ uint32_t operator()(uint32_t word) const { return word != 0u ? 1u : 0u; }
+};
 
 // Per slot, a warp: destination times into time_at_dest (raptor.h:224-226;
 // a minimum, so the lanes take the destinations in any order), and a slot
@@ -463,11 +469,12 @@ __device__ __forceinline__ void dest_slot(state const& st, uint32_t s, uint32_t 
   }
 }
 
-// The round's marked (route, group) and (real-time run, group) entries
-// listed, the slots' destination times, and the station-mark arrays swapped:
-// from here to the end of the step X[C_PAR ^ 1] holds the marks the round
-// reads and X[C_PAR] takes the marks it makes.  The first blocks take the
-// slots, 8 each, the others the lists, so that neither waits for the other.
+// The round's marked (route, group) words, in entries of up to kEntryMarks
+// queries, and (real-time run, group) words listed, the slots' destination
+// times, and the station-mark arrays swapped: from here to the end of the
+// step X[C_PAR ^ 1] holds the marks the round reads and X[C_PAR] takes the
+// marks it makes.  The first blocks take the slots, 8 each, the others the
+// lists, so that neither waits for the other.
 __global__ void __launch_bounds__(256) k_routes(state st) {
   step_begin();
   auto const lane = threadIdx.x & 31u;
@@ -482,12 +489,20 @@ __global__ void __launch_bounds__(256) k_routes(state st) {
     return;
   }
   auto const block = blockIdx.x - slot_blocks, n_blocks = gridDim.x - slot_blocks;
-  list_nonzero(st, st.R, st.tt.n_routes * st.G, C_R, block, n_blocks, [&](uint32_t at, uint32_t e, uint32_t marks) {
-    st.rlist[at] = uint4{e / st.G, e % st.G, marks, 0u};
-    st.R[e] = 0u;
-  });
+  list_nonzero(
+      st, st.R, st.tt.n_routes * st.G, C_R, block, n_blocks,
+      [](uint32_t marks) { return (static_cast<uint32_t>(__popc(marks)) + kEntryMarks - 1u) / kEntryMarks; },
+      [&](uint32_t at, uint32_t e, uint32_t marks) {
+        st.R[e] = 0u;
+        while (marks != 0u) {
+          auto rest = marks;  // the marks of a later entry
+          for (auto i = 0u; i != kEntryMarks; ++i) rest &= rest - 1u;
+          st.rlist[at++] = uint2{e, marks ^ rest};
+          marks = rest;
+        }
+      });
   if (st.tt.n_rt != 0u) {
-    list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, C_RT, block, n_blocks,
+    list_nonzero(st, st.RT_R, st.tt.n_rt * st.G, C_RT, block, n_blocks, one_item{},
                  [&](uint32_t at, uint32_t e, uint32_t) { st.rtlist[at] = e; });
   }
 }
@@ -639,10 +654,10 @@ __global__ void __launch_bounds__(256) k_route_scan_seq(const __grid_constant__ 
   scan_ctr pc{0u, 0u, 0u, 0u, 0u};
   for (auto w = blockIdx.x * blockDim.x + threadIdx.x; w < nr; w += gridDim.x * blockDim.x) {
     auto const en = st.rlist[w];
-    auto const R = load_route(T, en.x);
+    auto const R = load_route(T, en.x / st.G);
     if ((R.flags & kRouteOrder) != 0u) continue;  // k_route_scan's
-    auto const g = en.y;
-    for (auto mask = en.z; mask != 0u; mask &= mask - 1u) {
+    auto const g = en.x % st.G;
+    for (auto mask = en.y; mask != 0u; mask &= mask - 1u) {
       auto const b = static_cast<uint32_t>(__ffs(mask) - 1);
       auto const ln = st.lanes[g * 32u + b];
       uint32_t sec = 0u;
@@ -709,11 +724,11 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
       if (mask == 0u) {
         if (w >= n_items) break;
         auto const en = st.rlist[w >> split];
-        mask = en.z & ((split == 0u ? kFull : (1u << part_bits) - 1u) << ((w & ((1u << split) - 1u)) * part_bits));
+        mask = en.y & ((split == 0u ? kFull : (1u << part_bits) - 1u) << ((w & ((1u << split) - 1u)) * part_bits));
         w += n_tiles;
         if (mask == 0u) continue;
-        g = en.y;
-        R = load_route(T, en.x);
+        g = en.x % st.G;
+        R = load_route(T, en.x / st.G);
         if ((R.flags & kRouteOrder) == 0u) mask = 0u;  // k_route_scan_seq's
         continue;
       }
@@ -1225,7 +1240,7 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
       for (auto j = i; j < n; ++j) X[j] = 0u;
     }
   }
-  list_nonzero(st, st.Y, n, C_Y, block, n_blocks, [&](uint32_t at, uint32_t e, uint32_t) { st.ylist[at] = e; });
+  list_nonzero(st, st.Y, n, C_Y, block, n_blocks, one_item{}, [&](uint32_t at, uint32_t e, uint32_t) { st.ylist[at] = e; });
 }
 
 // ------------------------------------------------ transfers and footpaths
