@@ -1260,7 +1260,12 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
 // Which queries marked a station is gathered per block and written once (a
 // global word per group read and written by every pair doubled the kernel's
 // time at 1,024 slots).
-__global__ void __launch_bounds__(256) k_relax(state st) {
+//
+// Four blocks per SM (62 registers): left to itself the compiler took 80, three
+// blocks, for a kernel that waits on gathers (batch of 1,024: 3.64 -> 3.58 ms
+// a pass, 333 filtered queries 2.49 -> 2.44).  48 registers with five blocks took
+// the same, 40 spill.
+__global__ void __launch_bounds__(256, 4) k_relax(state st) {
   step_begin();
   __shared__ uint32_t made_bits[kMaxGroups];
   for (auto g = threadIdx.x; g < st.G; g += blockDim.x) made_bits[g] = 0u;
