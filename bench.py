@@ -696,7 +696,7 @@ def extras_legs(args, h, dtt, qs, B, local, shape):
         "unit": "GB/s", "frac": None, "traffic": traffic,
         "traffic_source": None if traffic is None else cap.get("command"),
         "limiter": "instruction issue and dependent L2 loads, not DRAM (ncu at batch 256: issue "
-                   "active 60%, SM throughput 55%, L2 hit 80%, DRAM throughput 5%, 19 of 32 "
+                   "active 52%, SM throughput 37%, L2 hit 46%, DRAM throughput 10%, 23 of 32 "
                    "threads per instruction)",
         "kernel": "k_route_scan", "launches": tm.route_scan_launches,
         "avg_launch_ms": per_launch_s * 1e3, "algorithmic_bytes_per_launch": per_launch_bytes,
