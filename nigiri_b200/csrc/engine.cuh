@@ -222,7 +222,7 @@ struct __align__(16) lane_t {
   uint16_t base;
   uint8_t fwd;
   uint8_t k;
-  uint8_t run;
+  uint8_t run;   // kLane*; 0: not running
   uint8_t mode;  // bit0 intermodal dest, bit1 has dests, bit2 tts default, bit3 no lower
                  // bounds, bits 4-6 footpath profile, bit7 round times kept for a later
                  // start-time group (the writes set their touched bits)
@@ -230,6 +230,9 @@ struct __align__(16) lane_t {
   uint8_t req;       // required route flags
   uint8_t blast;     // pong bounds: last round (0: none)
 };
+// lane_t::run: the slot runs rounds; this round is the start-time group's last
+// one, whose labels are not searched on from
+constexpr uint32_t kLaneRun = 1u, kLaneLast = 2u;
 
 struct start_rec {
   int32_t time_at_start;

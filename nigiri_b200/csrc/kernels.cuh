@@ -141,7 +141,7 @@ __device__ __forceinline__ void update_tad(slot_t& sl, uint32_t k, int key) {  /
 __device__ __forceinline__ lane_t lane_of(slot_t const& sl) {
   lane_t ln{};
   if (sl.state != S_RUN) return ln;
-  ln.run = 1;
+  ln.run = static_cast<uint8_t>(kLaneRun | (sl.k + 1u >= sl.end_k ? kLaneLast : 0u));
   ln.fwd = sl.fwd;
   ln.k = sl.k;
   ln.base = sl.base;
@@ -1067,8 +1067,10 @@ __device__ __forceinline__ void dest_label(state const& st, uint32_t* X, slot_t&
   rtw = enc(ln.qtag, key);
   touch(st, ln, k, d, s);
   st.best[li(st, d, s)] = enc(ln.gtag, key);
-  atomicOr(&X[d * st.G + (s >> 5)], 1u << (s & 31u));
-  atomicOr(&st.made_mask[s >> 5], 1u << (s & 31u));
+  if ((ln.run & kLaneLast) == 0u) {
+    atomicOr(&X[d * st.G + (s >> 5)], 1u << (s & 31u));
+    atomicOr(&st.made_mask[s >> 5], 1u << (s & 31u));
+  }
   if (key < tad) {
     if (tl_n < kMaxTimeline) {
       st.timeline[(static_cast<size_t>(ph) * st.S + s) * kMaxTimeline + tl_n++] = {pos_hi, pos_lo, key};
@@ -1257,6 +1259,10 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
 // pruning bounds differ between the phases, and each keeps its own
 // (tad_phase, timelines; k_reached).
 //
+// A start-time group's last round marks nothing: no round of the group would
+// read the marks, and left in place they would be the next search's of the
+// slot, which starts from its own stations alone (raptor.h:179-188).
+//
 // Which queries marked a station is gathered per block and written once (a
 // global word per group read and written by every pair doubled the kernel's
 // time at 1,024 slots).
@@ -1288,6 +1294,7 @@ __global__ void __launch_bounds__(256, 4) k_relax(state st) {
         if (tk == kKeyInv) return;
         auto const stations = (ln.mode & 2u) != 0u;
         auto const& tts = st.slots[s].tts;
+        auto const marks = (ln.run & kLaneLast) == 0u;
         bool made = false;  // a station marked
         if (!stations || !((st.D[e] >> b) & 1u)) {
           auto const tt = static_cast<int>(T.transfer_time[src]);
@@ -1309,8 +1316,10 @@ __global__ void __launch_bounds__(256, 4) k_relax(state st) {
                 touch(st, ln, ln.k, src, s);
               }
               atomicMin(&st.best[li(st, src, s)], enc(ln.gtag, fp));
-              atomicOr(&X[e], 1u << b);
-              made = true;
+              if (marks) {
+                atomicOr(&X[e], 1u << b);
+                made = true;
+              }
             }
           }
         }
@@ -1352,8 +1361,10 @@ __global__ void __launch_bounds__(256, 4) k_relax(state st) {
                 touch(st, ln, ln.k, tgt, s);
               }
               atomicMin(&st.best[li(st, tgt, s)], enc(ln.gtag, key));
-              atomicOr(&X[tgt * st.G + g], 1u << b);
-              made = true;
+              if (marks) {
+                atomicOr(&X[tgt * st.G + g], 1u << b);
+                made = true;
+              }
             }
           }
         }
