@@ -41,7 +41,9 @@ enum b2r_status {
   B2R_ERR_OUT_OF_MEMORY = -3, /* HBM budget or device allocation exhausted */
   B2R_ERR_CAPACITY = -4,      /* a per-query fixed-size buffer overflowed */
   B2R_ERR_NOT_READY = -5,     /* b2r_poll: ticket still running */
-  B2R_ERR_DEVICE_STATUS = -6, /* a kernel wrote an error status word */
+  B2R_ERR_DEVICE_STATUS = -6, /* a kernel failed the query: a fixed-size
+                                 buffer of its round is too small (more
+                                 than 64 footpaths into destinations) */
   B2R_ERR_UNSUPPORTED = -7,
   B2R_ERR_INTERNAL = -8
 };
@@ -368,7 +370,8 @@ uint32_t b2r_engine_slots(const b2r_engine* e);
 
 /* Batched search: runs n queries (any mix of kinds and directions) through
  * the resident slot pool with continuous admission and blocks until all are
- * done.  out[i] receives query i's result. */
+ * done.  out[i] receives query i's result.  Returns B2R_ERR_DEVICE_STATUS if
+ * any out[i].status is that; the other results stand. */
 int b2r_search_batch(b2r_engine* e, const b2r_query* qs, uint32_t n,
                      b2r_result* out);
 

@@ -15,6 +15,7 @@ B2R_OK = 0
 B2R_ERR_INVALID_ARGUMENT = -1
 B2R_ERR_CAPACITY = -4
 B2R_ERR_NOT_READY = -5
+B2R_ERR_DEVICE_STATUS = -6
 B2R_K = 16
 B2R_MAX_TRANSFERS = 14
 # limits of b2r_one_to_all_noalloc's fixed scratch array

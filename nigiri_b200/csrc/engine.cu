@@ -2071,6 +2071,18 @@ void fill_out(b2r_engine& e, std::vector<query_run>& runs, b2r_result* out) {
   }
 }
 
+// what a call returns whose queries have run: B2R_ERR_DEVICE_STATUS if a
+// kernel failed one of them (fail_slot), so that callers who do not look at
+// every result notice
+int device_status(std::vector<query_run> const& runs) {
+  for (auto const& r : runs) {
+    if (r.status == B2R_ERR_DEVICE_STATUS) {
+      return fail(B2R_ERR_DEVICE_STATUS, "a kernel failed a query of the call: too many destination labels in one round");
+    }
+  }
+  return B2R_OK;
+}
+
 // ------------------------------------------------------------- serving
 // Continuous batching: submitted queries are prepared on a host pool and
 // admitted into free slots at super-step boundaries while the queries
@@ -2752,7 +2764,6 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
       al(st.timeline, 2U * S * b2r::dev::kMaxTimeline);
       al(st.timeline_n, 2U * S);
       al(st.tad_phase, 2U * S);
-      al(st.status_word, 4);
       al(e->d_summary, S);
       st.summary = e->d_summary;
       al(st.prof, 8);
@@ -2916,17 +2927,8 @@ int b2r_search_batch(b2r_engine* e, const b2r_query* qs, uint32_t n, b2r_result*
         e->last.recon_max_journey_us = static_cast<double>(c[6]) / 1e3;
         e->last.recon_journeys = c[7];
       }
-      uint32_t err = 0;
-      B2R_CUDA(cudaMemcpy(&err, e->st.counters + b2r::dev::C_ERR, 4, cudaMemcpyDeviceToHost));
-      if (err != 0) {
-        B2R_CUDA(cudaMemset(e->st.counters + b2r::dev::C_ERR, 0, 4));
-        for (auto& r : runs) {
-          r.status = B2R_ERR_DEVICE_STATUS;
-          r.res.view.status = B2R_ERR_DEVICE_STATUS;
-        }
-      }
       b2r::fill_out(*e, runs, out);
-      return err != 0 ? b2r::fail(B2R_ERR_DEVICE_STATUS, "device status word set") : B2R_OK;
+      return b2r::device_status(runs);
     } catch (b2r::cuda_error const& ex) {
       return b2r::fail(B2R_ERR_CUDA, ex.what());
     }
@@ -2951,7 +2953,7 @@ int b2r_search_plain(b2r_engine* e, const b2r_query* q, b2r_result* out) {
       e->last.kernel_launches = br.launches + e->aux_launches;
       e->last.super_steps = br.steps;
       b2r::fill_out(*e, runs, out);
-      return B2R_OK;
+      return b2r::device_status(runs);
     } catch (b2r::cuda_error const& ex) {
       return b2r::fail(B2R_ERR_CUDA, ex.what());
     }

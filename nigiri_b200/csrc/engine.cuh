@@ -47,7 +47,8 @@ enum : uint8_t {
   S_COLLECT = 3,   // rounds of the current group finished
   S_DONE = 4,      // phase finished, host reads results
   S_ERROR = 5,
-  S_RECON = 6      // journeys of the finished group being rebuilt, next group follows
+  S_RECON = 6      // waits one step: journeys of the finished group being rebuilt, next group
+                   // follows; or, with slot_t::error set, the marks of an unfinished round cleared
 };
 
 // ------------------------------------------------------- timetable image
@@ -208,7 +209,7 @@ struct slot_t {
   uint32_t next_start;   // index of the next start label (group cursor)
   int32_t cur_start_time;
   uint32_t n_journeys;
-  int32_t error;
+  int32_t error;  // 0, or why the query fails (fail_slot, S_ERROR)
   int16_t tad[kK];  // time_at_dest_ keys
   uint64_t n_rounds, n_groups_run;
 };
@@ -280,7 +281,7 @@ struct state {
   uint32_t* D;      // is-destination bits [n_loc][G]
   uint32_t* ylist;  // frontier lists of (loc * G + g)
   uint2* rlist;     // {route * G + group, up to kEntryMarks of its marks}
-  uint32_t* counters;  // C_*: list lengths, mark parity, error bits
+  uint32_t* counters;  // C_*: list lengths, mark parity
   uint32_t* run_mask;  // [G]
   uint32_t* sweep_k;   // [G][K] slots to sweep that are at round k
   uint32_t* any_mask;  // [G] a route of this round is marked
@@ -295,7 +296,6 @@ struct state {
   tl_entry* timeline;     // [2][S][kMaxTimeline]: transfers, footpaths
   uint32_t* timeline_n;   // [2][S]
   int16_t* tad_phase;     // [2][S] tad[k] at the start of the phase
-  uint32_t* status_word;  // [0] device error flags
   unsigned long long* prof;  // route-scan work counters (profiling engines)
   uint32_t profile;
   // lower bounds computed on the device: tagged distances, frontier bits

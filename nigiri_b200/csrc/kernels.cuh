@@ -16,9 +16,15 @@ namespace b2r::dev {
 // journeys listed for reconstruction; C_RPAR: the parity of those the step
 // rebuilds
 enum : uint32_t {
-  C_PAR = 0, C_Y = 1, C_R = 2, C_RECON0 = 3, C_ERR = 4, C_F0 = 5, C_F1 = 6, C_RT = 7, C_RECON1 = 8, C_RPAR = 9
+  C_PAR = 0, C_Y = 1, C_R = 2, C_RECON0 = 3, C_F0 = 5, C_F1 = 6, C_RT = 7, C_RECON1 = 8, C_RPAR = 9
 };
 constexpr uint32_t recon_counter(uint32_t par) { return par == 0u ? C_RECON0 : C_RECON1; }
+
+// The round kernels' way to fail a query (a buffer of theirs is too small for
+// it): the slot ends at the end of the step (k_end), its neighbours go on.
+__device__ __forceinline__ void fail_slot(state const& st, uint32_t s) {
+  st.slots[s].error = B2R_ERR_DEVICE_STATUS;
+}
 
 // The first thing every super-step kernel does.  The kernels of a step are
 // launched with programmatic dependencies (enqueue_superstep): the next one
@@ -822,7 +828,7 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
             // a marked station always carries a best label of its start time
             // (marks come with best updates), so the boarding rule never meets
             // an invalid current_best; were it to, the query is failed loudly
-            if (!has_best && dec(st.tmp[at], oln.gtag) == kKeyInv) atomicOr(&st.counters[C_ERR], 4u);
+            if (!has_best && dec(st.tmp[at], oln.gtag) == kKeyInv) fail_slot(st, sm.pair[o][3].y);
             uint32_t key;
             if ((oR.flags & 2u) != 0u) {
               auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(oln.base) + 64) * oR.n_t + nt;
@@ -1075,7 +1081,7 @@ __device__ __forceinline__ void dest_label(state const& st, uint32_t* X, slot_t&
     if (tl_n < kMaxTimeline) {
       st.timeline[(static_cast<size_t>(ph) * st.S + s) * kMaxTimeline + tl_n++] = {pos_hi, pos_lo, key};
     } else {
-      atomicOr(&st.counters[C_ERR], 1u);
+      fail_slot(st, s);
     }
   }
   update_tad(sl, k, key);
@@ -1178,7 +1184,7 @@ __device__ __forceinline__ void station_dests_slot(state const& st, uint32_t* X,
       auto const m = __ballot_sync(kFull, has);
       auto const at = nc + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
       if (has && at < kMaxFpCand) c[at] = cd;
-      if (has && at >= kMaxFpCand) atomicOr(&st.counters[C_ERR], 2u);
+      if (has && at >= kMaxFpCand) fail_slot(st, s);
       nc = min(nc + static_cast<uint32_t>(__popc(m)), kMaxFpCand);
     }
   }
@@ -1703,7 +1709,8 @@ __device__ __forceinline__ void empty_round(state const& st, slot_t& sl, uint32_
 // slots: the round's end (raptor.h:217), the next round at once if it would
 // be empty (one step in six), collection when the group's rounds
 // are over, the journeys to rebuild listed (the slot then waits one step in
-// S_RECON), the next start-time group seeded, and the slot's views for the
+// S_RECON; so does a failed one, whose round left marks that that step
+// clears), the next start-time group seeded, and the slot's views for the
 // next step (lane record, the group's run mask and, per round, its slots to
 // sweep) and for the host
 // (summary).  seed_only: admitted slots are seeded and the views renewed,
@@ -1727,31 +1734,36 @@ __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
   if (seed_only) {
     if (state == S_START) next_slot(st, st.X[par], sl, s, lane, false);
   } else {
-    if (state == S_RUN) {
-      auto const k = static_cast<uint8_t>(sl.k + 1u);
-      __syncwarp();
-      if (lane == 0u) sl.k = k;
-      if (k >= sl.end_k) {
-        state = S_COLLECT;
-      } else if (((st.made_mask[g] >> (s & 31u)) & 1u) == 0u) {
-        empty_round(st, sl, s, k, lane);
-        state = S_COLLECT;
+    auto const failed = sl.error != 0;
+    if (state == S_START || (state == S_RECON && !failed)) {
+      next_slot(st, st.X[par], sl, s, lane, state == S_RECON);
+    } else if (state == S_RECON) {
+      if (lane == 0u) sl.state = S_ERROR;
+    } else {
+      if (state == S_RUN) {
+        auto const k = static_cast<uint8_t>(sl.k + 1u);
+        __syncwarp();
+        if (lane == 0u) sl.k = k;
+        if (failed) {
+          state = S_RECON;
+        } else if (k >= sl.end_k) {
+          state = S_COLLECT;
+        } else if (((st.made_mask[g] >> (s & 31u)) & 1u) == 0u) {
+          empty_round(st, sl, s, k, lane);
+          state = S_COLLECT;
+        }
       }
-    }
-    if (state == S_COLLECT) {
-      if (!sl.one_to_all && !collect_slot(st, sl, s, lane)) {
-        state = S_ERROR;
-        if (lane == 0u) sl.error = B2R_ERR_CAPACITY;
-      } else if (!sl.one_to_all && !sl.recon_defer && list_recon(st, sl, s, lane, par)) {
-        state = S_RECON;  // else rebuilt when the slot is done (k_reconstruct_done), or nothing to rebuild
-      } else {
-        next_slot(st, st.X[par], sl, s, lane, true);
+      if (state == S_COLLECT) {
+        if (!sl.one_to_all && !collect_slot(st, sl, s, lane)) {
+          state = S_ERROR;
+          if (lane == 0u) sl.error = B2R_ERR_CAPACITY;
+        } else if (!sl.one_to_all && !sl.recon_defer && list_recon(st, sl, s, lane, par)) {
+          state = S_RECON;  // else rebuilt when the slot is done (k_reconstruct_done), or nothing to rebuild
+        } else {
+          next_slot(st, st.X[par], sl, s, lane, true);
+        }
       }
       if ((state == S_ERROR || state == S_RECON) && lane == 0u) sl.state = state;
-    } else if (state == S_RECON) {
-      next_slot(st, st.X[par], sl, s, lane, true);
-    } else if (state == S_START) {
-      next_slot(st, st.X[par], sl, s, lane, false);
     }
   }
   __syncwarp();
