@@ -12,6 +12,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -1061,6 +1062,26 @@ void retire(b2r_engine& e, std::vector<uint32_t> const& slots, cudaStream_t s) {
   B2R_CUDA(cudaGetLastError());
 }
 
+// Every slot empty and no station marked, after a loop ended with an error
+// while searches were running: left in place, their marks and destination
+// bits would be those of the next queries of the slots.  Errors of its own
+// are not reported (the caller has one to report; a device error stays until
+// the context's end).
+void abandon_searches(b2r_engine& e) noexcept {
+  cudaStreamSynchronize(e.stream);
+  cudaStreamSynchronize(e.stream2);
+  try {
+    std::vector<uint32_t> all(e.S);
+    std::iota(all.begin(), all.end(), 0U);
+    retire(e, all, e.stream);
+    auto const words = static_cast<size_t>(e.tt->d.n_loc) * e.G;
+    for (auto* x : e.st.X) B2R_CUDA(cudaMemsetAsync(x, 0, words * sizeof(uint32_t), e.stream));
+    seed(e, e.stream);  // the views of the slots
+    B2R_CUDA(cudaStreamSynchronize(e.stream));
+  } catch (std::exception const&) {
+  }
+}
+
 // a page-locked row buffer back into the pool (at most 512 buffers and
 // 4 GiB; beyond that it is freed)
 void give_rows(b2r_engine& e, row_buf&& r) {
@@ -1749,12 +1770,15 @@ struct batch_runner {
   void run(uint32_t chunk) {
     auto const S = e.S;
     auto* st = e.stream;
-    // row copies into result buffers may still be in flight when an error
-    // unwinds the batch: they end before those buffers can be freed
-    struct drain {
-      cudaStream_t s;
-      ~drain() { cudaStreamSynchronize(s); }
-    } drain2{e.stream2};
+    // when an error unwinds the batch, its searches end and row copies into
+    // result buffers land before those buffers can be freed
+    struct unwind {
+      b2r_engine& e;
+      bool finished{false};
+      ~unwind() {
+        if (!finished) abandon_searches(e);
+      }
+    } guard{e};
     e.busy.clear();
     B2R_CUDA(cudaEventRecord(e.ev_base, st));
     e.base_recorded = true;
@@ -1996,6 +2020,7 @@ struct batch_runner {
     }
     B2R_CUDA(cudaStreamSynchronize(st));
     B2R_CUDA(cudaStreamSynchronize(e.stream2));  // one-to-all rows still on their way
+    guard.finished = true;
     busy_ms = busy_union_ms(e.busy);
   }
 };
@@ -2331,6 +2356,7 @@ struct serve_state {
         cv_done.notify_all();
       }
     } catch (std::exception const& ex) {
+      abandon_searches(e);  // the engine may run batches once the loop is stopped
       std::lock_guard<std::mutex> lock{mu};
       failed_status = B2R_ERR_CUDA;
       failed_msg = ex.what();
