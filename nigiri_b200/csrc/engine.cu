@@ -2731,13 +2731,20 @@ int b2r_engine_create(b2r_timetable* tt, const b2r_engine_config* cfg_in, b2r_en
         }
       }
       auto const nl = tt->d.n_loc;
-      e->bytes_per_slot = static_cast<uint64_t>(nl) * (b2r::dev::kK * (4 + 2) + 4 + 4 + 2 + 4) +
-                          static_cast<uint64_t>(e->max_j) *
-                              (sizeof(b2r::dev::journey_rec) + b2r::dev::kMaxLegs * sizeof(b2r_leg)) +
-                          e->max_starts * sizeof(b2r::dev::start_rec) +
-                          e->max_dest * sizeof(b2r::dev::dest_rec) + e->max_off * sizeof(b2r_offset) +
-                          b2r::dev::kMaxTimeline * sizeof(b2r::dev::tl_entry) +
-                          (static_cast<uint64_t>(nl) * (4 + b2r::dev::kK) + tt->d.n_routes) / 8 + 256;
+      {
+        // the arrays below, by what they are sized by: a slot, its journeys,
+        // its labels of a location, a mark word of 32 slots
+        using namespace b2r::dev;
+        auto const per_slot = sizeof(slot_t) + sizeof(lane_t) + sizeof(slot_summary) + sizeof(uint32_t) +
+                              e->max_starts * sizeof(start_rec) + e->max_dest * sizeof(dest_rec) +
+                              e->max_off * sizeof(b2r_offset) +
+                              2U * (kMaxTimeline * sizeof(tl_entry) + sizeof(uint32_t) + sizeof(int16_t));
+        auto const per_journey = sizeof(journey_rec) + kMaxLegs * sizeof(b2r_leg) + sizeof(uint32_t) + 1U;
+        auto const per_label = kK * (sizeof(uint32_t) + sizeof(int16_t)) + 3U * sizeof(uint32_t) + sizeof(uint16_t);
+        auto const words = static_cast<uint64_t>(nl) * (kK + 9U) +
+                           static_cast<uint64_t>(tt->d.n_routes) * (1U + 2U * (32U / kEntryMarks)) + kK + 4U;
+        e->bytes_per_slot = per_slot + e->max_j * per_journey + nl * per_label + (words * sizeof(uint32_t) + 31U) / 32U;
+      }
       auto by_budget = cfg.hbm_budget / std::max<uint64_t>(1, e->bytes_per_slot);
       auto slots = std::min<uint64_t>(std::max(32U, cfg.max_slots), by_budget);
       slots = std::min<uint64_t>(slots, 32ULL * b2r::dev::kMaxGroups);
