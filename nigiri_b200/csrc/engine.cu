@@ -2052,15 +2052,7 @@ struct preparer {
   std::atomic<uint32_t> next{0};
   void start(b2r_engine& e, b2r_query const* qs, uint32_t n, std::vector<query_run>& runs,
              bool inline_all) {
-    auto const hw = std::max(1U, std::thread::hardware_concurrency());
     auto const lb_mode = e.lb_mode();
-    // A query's preparation takes a few microseconds, starting a thread some
-    // dozens: 16 queries a thread, unless the lower bounds are a Dijkstra on
-    // the host (about a millisecond)
-    auto dijkstra = lb_mode == 1;
-    for (auto i = 0U; i != n && !dijkstra; ++i) dijkstra = qs[i].prf_idx != 0U;
-    auto const n_threads = std::max(1U, std::min<uint32_t>(
-        e.cfg.host_threads != 0 ? e.cfg.host_threads : (hw > 1 ? hw - 1 : 1), dijkstra ? n : (n + 15U) / 16U));
     auto work = [&e, qs, n, &runs, lb_mode, this]() {
       for (auto i = next++; i < n; i = next++) {
         auto const t0 = std::chrono::steady_clock::now();
@@ -2074,7 +2066,24 @@ struct preparer {
       work();
       return;
     }
+    auto const n_threads = threads(e, qs, n);
     for (auto t = 0U; t < n_threads; ++t) pool.emplace_back(work);
+  }
+  // As many threads as the caller asked for, else one for about 50 us of
+  // preparation (starting one takes some dozens): 16 queries of one start
+  // time (1 to 4 us each, national ones too); windows by their start stops
+  // (8 to 20 us for one, 50 to 110 for 6, 400 to 1,200 for 64); a query whose
+  // lower bounds are a Dijkstra on the host has one of its own (about a
+  // millisecond).
+  static uint32_t threads(b2r_engine const& e, b2r_query const* qs, uint32_t n) {
+    if (e.cfg.host_threads != 0) return std::max(1U, std::min(e.cfg.host_threads, n));
+    uint64_t parts = 0;  // sixteenths of a thread
+    for (auto i = 0U; i != n; ++i) {
+      auto const window = qs[i].is_interval != 0 && qs[i].algorithm != B2R_ALGO_PONG;
+      parts += e.lb_mode() == 1 || qs[i].prf_idx != 0U ? 16U : window ? std::clamp(4U * qs[i].n_start, 4U, 16U) : 1U;
+    }
+    auto const hw = std::max(2U, std::thread::hardware_concurrency());
+    return static_cast<uint32_t>(std::clamp<uint64_t>((parts + 15U) / 16U, 1U, hw - 1U));
   }
   void join() {
     for (auto& t : pool) t.join();
