@@ -253,7 +253,9 @@ struct tl_entry {  // time_at_dest timeline of one phase
 
 // what the host reads of every slot after a super-step chunk
 struct slot_summary {
-  uint8_t state, pad[3];
+  uint8_t state;
+  uint8_t starts_left;  // start labels whose group has not begun (255: that many or more)
+  uint8_t pad[2];
   uint32_t n_journeys;
 };
 

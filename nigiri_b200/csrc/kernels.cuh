@@ -1768,7 +1768,7 @@ __global__ void __launch_bounds__(1024, 1) k_end(state st, bool seed_only) {
   }
   __syncwarp();
   if (lane == 0u) {
-    st.summary[s] = {sl.state, {0, 0, 0}, sl.n_journeys};
+    st.summary[s] = {sl.state, static_cast<uint8_t>(min(255u, sl.n_starts - sl.next_start)), {0, 0}, sl.n_journeys};
     st.lanes[s] = lane_of(sl);
     if (sl.state == S_RUN) {
       atomicOr(&run_bits, 1u << (s & 31u));
