@@ -2650,14 +2650,11 @@ int b2r_timetable_upload(const b2r_timetable_desc* d, int device, b2r_timetable*
       dd.route_tr_to = up(d->route_transport_to, nr);
       dd.route_st_from = up(d->route_stop_time_from, nr);
       dd.st = up(d->route_stop_times, d->n_route_stop_times);
-      dd.route_bf = up(d->route_traffic_days, nr);
       dd.transport_bf = up(d->transport_traffic_days, ntr);
       dd.transport_route = up(d->transport_route, ntr);
       dd.bf = up(d->bitfields, 8ull * d->n_bitfields);
       dd.loc_routes_idx = up(d->location_routes_index, nl + 1);
       dd.loc_routes = up(d->location_routes, d->location_routes_index[nl]);
-      dd.route_sorted = up(sorted.data(), nr);
-      dd.route_fifo = up(fifo.data(), nr);
       dd.route_filter = up(rfilter.data(), nr);
       dd.route_sec = up(rsec.data(), rsec.size());
       t->routes.resize(nr);

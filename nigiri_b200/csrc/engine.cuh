@@ -53,23 +53,28 @@ enum : uint8_t {
 
 // ------------------------------------------------------- timetable image
 // what a scan of a route needs before its stops and events, in two 16-byte
-// loads (the same values as the arrays of dtt)
+// loads (sb, st, t0 and filter as in the arrays of dtt)
 struct __align__(16) route_rec {
   uint32_t sb;      // route_stop_idx
   uint32_t n;       // stops
   uint32_t st;      // route_st_from
   uint32_t t0;      // route_tr_from
   uint32_t n_t;     // transports
-  uint32_t bf;      // route_bf
+  uint32_t bf;      // traffic days
   uint32_t flags;   // kRoute*
   uint32_t filter;  // route_filter
 };
-// flags: bits 0-1 route_fifo, route_sorted, and whether every transport's
-// traffic days are the route's
-constexpr uint32_t kRouteOrder = 3u, kRouteSorted = 4u, kRouteOneDays = 8u;
+// flags: kRouteOrder bit 0: the route's trips (transport, service day) compare
+// the same way at every event of the route, equal at all or strictly ordered
+// at all; bit 1 (kRouteOffsetOrder): and (service day, transport offset) orders
+// them as their times do (columns ordered by minute, every first departure on
+// its service day, fewer than 16384 transports).  kRouteSorted: every event
+// column is ordered by minutes after midnight.  kRouteOneDays: every
+// transport's traffic days are the route's.
+constexpr uint32_t kRouteOrder = 3u, kRouteOffsetOrder = 2u, kRouteSorted = 4u, kRouteOneDays = 8u;
 
 struct dtt {
-  uint32_t n_loc, n_routes, n_transports, n_groups_unused;
+  uint32_t n_loc, n_routes, n_transports;
   int32_t internal_from_days;
   uint8_t const* transfer_time;
   uint32_t const* parent;
@@ -92,19 +97,11 @@ struct dtt {
   uint32_t const* route_tr_to;
   uint32_t const* route_st_from;
   uint16_t const* st;  // route_stop_times (packed delta)
-  uint32_t const* route_bf;
   uint32_t const* transport_bf;
   uint32_t const* transport_route;
   uint64_t const* bf;
   uint32_t const* loc_routes_idx;
   uint32_t const* loc_routes;
-  uint8_t const* route_sorted;  // 1: every event column is ordered by mam
-  // bit 0: the route's trips (transport, service day) compare the same way
-  // at every event of the route, equal at all or strictly ordered at all;
-  // bit 1: and (service day, transport offset) orders them as their times
-  // do (columns ordered by minute, every first departure on its service day,
-  // fewer than 16384 transports)
-  uint8_t const* route_fifo;
   route_rec const* routes;
   // lower-bound graphs (build_lb_graph.h), packed footpath words
   uint32_t const* lbg_fwd_idx;

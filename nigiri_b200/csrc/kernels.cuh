@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256) k_routes(state st) {
 //   unless time_at_dest rules it out, the search (it depends only on its
 //   stop's labels; what it needs of its pair lies in shared memory);
 // * on a route whose trips keep one order at every event
-//   (b2r_timetable: route_fifo), "switch when at least as good at this
+//   (kRouteOrder), "switch when at least as good at this
 //   stop" is "keep the best trip so far", whatever stop compares them (on a
 //   tie both are the same trip or equal at every event), so a prefix
 //   minimum over the stops gives the trip each stop is reached by;
@@ -719,8 +719,8 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
   route_rec R{};
   lane_t ln{};
   bool have = false;
-  // The trips' order key, below 2^21, smaller is better: with route_fifo
-  // bit 1 (service day - base + 64) * n_t + transport offset (the service
+  // The trips' order key, below 2^21, smaller is better: with
+  // kRouteOffsetOrder (service day - base + 64) * n_t + transport offset (the service
   // day lies within 64 days of the base day, n_t < 2^14), else the time at
   // the route's first departure event (|t| < 2^20 minutes) + 2^20; both
   // mirrored backward, where later is better.
@@ -830,7 +830,7 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
             // an invalid current_best; were it to, the query is failed loudly
             if (!has_best && dec(st.tmp[at], oln.gtag) == kKeyInv) fail_slot(st, sm.pair[o][3].y);
             uint32_t key;
-            if ((oR.flags & 2u) != 0u) {
+            if ((oR.flags & kRouteOffsetOrder) != 0u) {
               auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(oln.base) + 64) * oR.n_t + nt;
               key = ofwd ? x : (1u << 21) - 1u - x;
             } else {

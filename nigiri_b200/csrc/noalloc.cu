@@ -256,7 +256,7 @@ __device__ void walk_route(dtt const& T, params const& P, arrays const& a, dev::
 
 // update_route (raptor.h:1177-1349), a warp per marked route, the lanes over
 // its stops: every marked boardable stop searches its earliest trip, and on
-// a route whose trips keep one order at every event (route_fifo) the trip a
+// a route whose trips keep one order at every event (kRouteOrder) the trip a
 // stop is reached by is the prefix minimum of the candidates before it, from
 // the last section on that lacks a required flag.
 __device__ void scan_routes(dtt const& T, params const& P, arrays const& a, uint32_t k, uint32_t lane, uint32_t i,
@@ -298,7 +298,7 @@ __device__ void scan_routes(dtt const& T, params const& P, arrays const& a, uint
           if (prt <= P.tad && prt != kInv &&
               dev::et_search(T, fwd, R, si, static_cast<uint16_t>(minutes / 1440), minutes % 1440, 0, P.tad, P.base, nt,
                              nd, n_ev, n_days)) {
-            if ((R.flags & 2u) != 0u) {  // the order key of the batched scan
+            if ((R.flags & dev::kRouteOffsetOrder) != 0u) {  // the order key of the batched scan
               auto const x = static_cast<uint32_t>(static_cast<int>(nd) - static_cast<int>(P.base) + 64) * R.n_t + nt;
               key = fwd ? x : (1u << 21) - 1u - x;
             } else {
