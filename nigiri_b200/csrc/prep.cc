@@ -214,7 +214,7 @@ void lower_bounds(view const& v, prepped_query const& p, std::vector<uint16_t>& 
   };
   for (auto const& [l, dd] : seed) {
     v.metas(p.dest_mode, l, [&](uint32_t m) {
-      push(m, dd);
+      if (dd < kBuckets) push(m, dd);  // farther than the travel time: bounds itself, nothing around it
       dist[m] = std::min(dd, dist[m]);
     });
   }
