@@ -30,9 +30,13 @@ constexpr int kMaxTimeline = 128;
 // where all of a small network's routes are marked by most queries (1,009
 // stops, 1,000 queries: 20 of 32) an entry of a whole word is 20 pairs long,
 // and 21,000 of them on 18,944 resident tiles are one wave and a ninth: 1.94
-// ms for that batch, 1.75 with 8 and 1.57 with 4.  Where words hold one or two
-// marks (40,009 stops) the limit costs nothing.
+// ms on the device for that batch.  Fewer marks an entry are faster throughout
+// (8, 4, 2, 1: 1.77, 1.59, 1.50, 1.44 ms for that batch; 3.78, 3.77, 3.69,
+// 3.42 for 1,024 queries on 40,009 stops; 43.5, 43.3, 42.2, 39.5 for the
+// national 256) and take more room: 8 bytes an entry, 32 / kEntryMarks entries
+// a word, 64 bytes per (route, group) with 4.
 constexpr uint32_t kEntryMarks = 4;
+static_assert(32u % kEntryMarks == 0u);  // the list's room (rlist)
 constexpr uint32_t kMaxGroups = 2048;  // slot groups: a slot index has 16 bits (recon_list)
 
 // lrs_stop bits above the position: a ride can end (forward) or begin

@@ -917,9 +917,12 @@ __device__ __forceinline__ void scan_tiles(state const& st, scan_smem<kTile>& sm
 
 // Above this many entries per SM the scan takes 8 lanes per pair, else a
 // warp: a step of a warp is about 1,500 instructions for four pairs and 700
-// for one, so with warps to spare one pair ends sooner.  12, 32 and 96 took
-// 29.1, 28.9 and 28.7 ms for 96 range queries and 38.1, 37.9 and 37.7 ms for
-// the national mix of 256.
+// for one, so with warps to spare one pair ends sooner.  Device time with 0
+// (never a warp), 48, 96, 192, 384 and no limit (always a warp): 32.1, 31.4,
+// 31.3, 31.2, 31.3, 31.3 ms for 96 range queries; 3.70, 3.79, 3.77, 3.79,
+// 3.91, 4.50 for 1,024 on 40,009 stops; 1.57, 1.60, 1.59, 1.59, 1.68, 1.84 for
+// 1,000 on 1,009 stops.  The same run repeats within 0.5%: the line lies
+// anywhere between 48 and 192.
 constexpr uint32_t kFewPerSm = 96;
 
 // Builds with four, five or six blocks of 256 threads resident per SM (the
@@ -1274,9 +1277,10 @@ __global__ void __launch_bounds__(256) k_reached(state st) {
 // time at 1,024 slots).
 //
 // Four blocks per SM (62 registers): left to itself the compiler took 80, three
-// blocks, for a kernel that waits on gathers (batch of 1,024: 3.64 -> 3.58 ms
-// a pass, 333 filtered queries 2.49 -> 2.44).  48 registers with five blocks took
-// the same, 40 spill.
+// blocks, for a kernel that waits on gathers (device time of 1,024 queries 3.87
+// -> 3.77 ms, of the national 256 44.0 -> 43.3, 333 filtered ones 2.68 -> 2.65;
+// runs repeat within 0.5%).  48 registers with five blocks took the same, 40
+// spill.
 __global__ void __launch_bounds__(256, 4) k_relax(state st) {
   step_begin();
   __shared__ uint32_t made_bits[kMaxGroups];
