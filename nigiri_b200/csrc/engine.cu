@@ -1807,33 +1807,31 @@ struct batch_runner {
       pending.clear();
       slot_picker pick{S, [&](uint32_t s) { return slot_q[s] == -1; }};
       while (next < runs.size()) {
-        while (next < runs.size()) {
-          auto& q = runs[next];
-          if (!q.ready.load(std::memory_order_acquire)) break;
-          if (q.p.status != B2R_OK || q.p.empty_result) {
-            q.status = q.p.status;
-            q.res.view.status = q.p.status;
-            q.res.view.interval_from = q.p.iv_from;
-            q.res.view.interval_to = q.p.iv_to;
-            q.finished = true;
-            ++next;
-            continue;
-          }
-          if (auto const c = check_capacity(e, q.p); c != B2R_OK) {
-            q.status = c;
-            q.res.view.status = c;
-            q.finished = true;
-            ++next;
-            continue;
-          }
-          break;
+        auto& q = runs[next];
+        // looked at once: a query that gets ready after this is taken up by
+        // the next admission, refusals and capacity checked
+        if (!q.ready.load(std::memory_order_acquire)) break;
+        if (q.p.status != B2R_OK || q.p.empty_result) {
+          q.status = q.p.status;
+          q.res.view.status = q.p.status;
+          q.res.view.interval_from = q.p.iv_from;
+          q.res.view.interval_to = q.p.iv_to;
+          q.finished = true;
+          ++next;
+          continue;
         }
-        if (next >= runs.size() || !runs[next].ready.load(std::memory_order_acquire)) break;
-        auto const s = pick.take(sweeps(runs[next].p));
+        if (auto const c = check_capacity(e, q.p); c != B2R_OK) {
+          q.status = c;
+          q.res.view.status = c;
+          q.finished = true;
+          ++next;
+          continue;
+        }
+        auto const s = pick.take(sweeps(q.p));
         if (s < 0) break;
         slot_q[s] = static_cast<int64_t>(next);
-        starts_left[s] = runs[next].p.starts.size();
-        adm.push_back({static_cast<uint32_t>(s), &runs[next].p});
+        starts_left[s] = q.p.starts.size();
+        adm.push_back({static_cast<uint32_t>(s), &q.p});
         ++next;
       }
       auto const t0 = std::chrono::steady_clock::now();
