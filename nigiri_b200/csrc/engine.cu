@@ -1722,6 +1722,7 @@ void rearm(b2r_engine& e, uint32_t s, query_run& q, cudaStream_t st) {
   cur.early_term = 0;
   cur.next_start = 0;
   cur.n_starts = static_cast<uint32_t>(q.p.starts.size());
+  cur.n_journeys = static_cast<uint32_t>(q.keep.size());  // the slot is written behind k_set_journeys
   if (cur.n_starts > e.max_starts) throw std::runtime_error("start capacity exceeded");
   std::vector<dev::start_rec> starts(q.p.starts.size());
   for (auto j = 0U; j != starts.size(); ++j) {
