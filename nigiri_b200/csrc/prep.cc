@@ -700,11 +700,12 @@ void prepare(host_view const& hv, b2r_query const& q, int lb_mode, prepped_query
   }
 
   // add_start_labels, search.h:220-225, 401-411
+  p.use_start_footpaths = q.use_start_footpaths != 0;
   if (p.iv_to - p.iv_from != 0) {
-    collect_starts(v, p, true, 0, p.iv_from, p.iv_to, q.use_start_footpaths != 0, true, p.starts);
+    collect_starts(v, p, true, 0, p.iv_from, p.iv_to, p.use_start_footpaths, true, p.starts);
   } else {
-    collect_starts(v, p, !p.ontrip, q.start_time, q.interval_from, q.interval_to,
-                   q.use_start_footpaths != 0, true, p.starts);
+    collect_starts(v, p, !p.ontrip, q.start_time, q.interval_from, q.interval_to, p.use_start_footpaths, true,
+                   p.starts);
   }
   sort_starts(p.fwd, p.starts);
 }
@@ -712,7 +713,7 @@ void prepare(host_view const& hv, b2r_query const& q, int lb_mode, prepped_query
 void add_interval_starts(host_view const& hv, prepped_query const& p, int32_t from, int32_t to,
                          bool add_ontrip, std::vector<start_label>& starts) {
   view const v{hv.d, hv.rt};
-  collect_starts(v, p, true, 0, from, to, false, add_ontrip, starts);
+  collect_starts(v, p, true, 0, from, to, p.use_start_footpaths, add_ontrip, starts);
   sort_starts(p.fwd, starts);
 }
 

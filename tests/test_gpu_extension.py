@@ -43,7 +43,7 @@ def answer(r):
 
 
 @pytest.mark.parametrize("seed", range(6))
-@pytest.mark.parametrize("footpaths", [0])
+@pytest.mark.parametrize("footpaths", [0, 1])
 def test_extended_windows_match_oracle(city, footpaths, seed):
     h, tt, eng = city
     qs = queries(h, 160, footpaths, seed)
@@ -58,7 +58,7 @@ def test_extended_windows_match_oracle(city, footpaths, seed):
     assert phases > 0  # windows wider than their first extension
 
 
-@pytest.mark.parametrize("footpaths", [0])
+@pytest.mark.parametrize("footpaths", [0, 1])
 def test_extended_windows_step_driven(city, tmp_path, footpaths):
     h, tt, _ = city
     run = helper(str(tmp_path)).algo_search
