@@ -1174,12 +1174,20 @@ __device__ __forceinline__ void station_dests_slot(state const& st, uint32_t* X,
           auto const tk = dec(st.tmp[li(st, src, s)], ln.gtag);
           if (tk != kKeyInv) {
             auto const o0 = oidx[src], o1 = oidx[src + 1];
+            // the footpath in the source's own list: among several between
+            // the two, the one of this duration
+            auto at = o1;
             for (auto y = o0; y != o1; ++y) {
               if (B2R_FP_TARGET(odat[y]) != d) continue;
-              auto const dur = adjusted<int>(sl.tts, static_cast<int>(B2R_FP_DURATION(odat[y])));
-              cd = {src, y - o0, d, key_add(tk, dur)};
-              has = true;
+              if (at == o1) at = y;
+              if (B2R_FP_DURATION(odat[y]) != B2R_FP_DURATION(idat[x])) continue;
+              at = y;
               break;
+            }
+            if (at != o1) {
+              auto const dur = adjusted<int>(sl.tts, static_cast<int>(B2R_FP_DURATION(odat[at])));
+              cd = {src, at - o0, d, key_add(tk, dur)};
+              has = true;
             }
           }
         }
