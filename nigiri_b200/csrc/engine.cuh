@@ -232,8 +232,8 @@ struct __align__(16) lane_t {
   uint8_t req;       // required route flags
   uint8_t blast;     // pong bounds: last round (0: none)
 };
-// lane_t::run: the slot runs rounds; this round is the start-time group's last
-// one, whose labels are not searched on from
+// lane_t::run: the slot runs rounds; the one it is in is the last of its
+// start-time group, whose labels are not searched on from
 constexpr uint32_t kLaneRun = 1u, kLaneLast = 2u;
 
 struct start_rec {
